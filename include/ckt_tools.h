@@ -57,6 +57,15 @@ int ckt_check_recip_quotient(uint64_t seed, uint64_t count, int32_t divisor, int
 int ckt_check_wide_quotient(uint64_t seed, uint64_t count, int32_t divisor,
                             unsigned long long *counts, void *stream);
 
+/* The split quotient by a divisor that EXACT mode's check accepts, against
+ * __fdiv_rn: `count` pseudo-random divisors (ranges as above), 24 dividends
+ * each, those that come nearest to a rounding boundary among them.  Adds to
+ * counts[0] the mismatches, to counts[1] the divisors accepted, to counts[2]
+ * those accepted with a moved second part, to counts[3] the divisors drawn
+ * (device memory, 4 x uint64). */
+int ckt_check_split_quotient(uint64_t seed, uint64_t count, int32_t divisor,
+                             unsigned long long *counts, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

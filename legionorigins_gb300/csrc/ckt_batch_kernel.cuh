@@ -170,13 +170,22 @@ __device__ __forceinline__ void dc_contrib_block(const RoundCircuit &rc, uint32_
 // scattered by the CNC tiles then summed contiguously.
 // Tiles of two wires per thread run both wires in one paired stepper
 // (cnc_wire_pair), which needs more registers: two blocks of 256 per SM.
+// EXACT tiles of one wire too: with a third block its 80 registers spill the
+// free steps' loop (16 circuits, block 256, schedule 2: 9.29 -> 9.01 ms with
+// two blocks).
 template <uint32_t BLOCK, int WPT, int DCS, int MODE>
-__global__ void __launch_bounds__(BLOCK, (WPT == 2 ? 512 : 768) / BLOCK)
+__global__ void __launch_bounds__(BLOCK,
+                                  (WPT == 2 || MODE == CKT_MODE_EXACT ? 512 : 768) / BLOCK)
     round_kernel(const BatchItem *__restrict__ items, uint32_t num_items,
                  const RoundCircuit *__restrict__ circ, BatchSync sync, float dt,
                  uint64_t timeout_ns) {
   __shared__ uint32_t s_item, s_go;
-  __shared__ float sval[DCS == 1 ? 1 : kDcChunk];
+  // The CNC tiles' saved states and the DC tiles' staged contributions are
+  // never in use at the same time.
+  constexpr int kSave = MODE == CKT_MODE_EXACT ? kSavedState * WPT * (int)BLOCK : WPT;
+  constexpr int kStage = DCS == 1 ? 1 : (int)kDcChunk;
+  __shared__ __align__(8) float sbuf[kSave > kStage ? kSave : kStage];
+  float *sval = sbuf;
   __shared__ uint32_t smask[DCS == 0 ? kDcChunk / 32 : 1];
   while (true) {
     if (threadIdx.x == 0) {
@@ -211,8 +220,10 @@ __global__ void __launch_bounds__(BLOCK, (WPT == 2 ? 512 : 768) / BLOCK)
           const bool has_b = tb < item.count;
           const uint32_t w = item.begin + ta, wb = item.begin + (has_b ? tb : ta);
           float2 i0, i9;
-          cnc_wire_pair<MODE, CKT_INIT_KERNEL>((int64_t)w, (int64_t)wb, has_b, wa, volts,
-                                               rc.steps, dt, &i0, &i9);
+          cnc_wire_pair<MODE, CKT_INIT_KERNEL, (int)BLOCK>(
+              (int64_t)w, (int64_t)wb, has_b, wa, volts, rc.steps, dt,
+              reinterpret_cast<float2 *>(sbuf) + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0), &i0,
+              &i9);
           if (DCS == 2) {
             rc.contrib[rc.slot_in[w]] = __fmul_rn(-dt, i0.x);
             rc.contrib[rc.slot_out[w]] = __fmul_rn(dt, i9.x);
@@ -229,7 +240,9 @@ __global__ void __launch_bounds__(BLOCK, (WPT == 2 ? 512 : 768) / BLOCK)
           if (t < item.count) {
             const uint32_t w = item.begin + t;
             float i0, i9;
-            cnc_wire<MODE, CKT_INIT_KERNEL>((int64_t)w, wa, volts, rc.steps, dt, &i0, &i9);
+            cnc_wire<MODE, CKT_INIT_KERNEL, (int)BLOCK>(
+                (int64_t)w, wa, volts, rc.steps, dt,
+                sbuf + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0), &i0, &i9);
             if (DCS == 2) {
               rc.contrib[rc.slot_in[w]] = __fmul_rn(-dt, i0);
               rc.contrib[rc.slot_out[w]] = __fmul_rn(dt, i9);

@@ -53,6 +53,26 @@
 //    guarantees.  Zeros and infinities are a times RN(1/b), exact for them.
 //    Dividends whose quotient may be subnormal (subnormal_quot) are left to
 //    the divide routine.
+//
+//  * A checked divisor (check_split), one multiply and one FMA, as for dt:
+//        q = RN(a*y + RN(a*yl)).
+//    Scale a = A 2^-23 and b = B 2^-23 to 24-bit integers A, B in [2^23, 2^24)
+//    (only signs and exponents change).  For A < B the quotient lies in
+//    (1/2, 1) and the distance of a/b from the rounding boundary
+//    (2m+1)/2^25 is |r| / (2^48 b) with r = 2^25 A - (2m+1) B; for A >= B it
+//    is |r| / (2^47 b) with r = 2^24 A - (2m+1) B.  The sum rounded at the
+//    end is off a/b by at most a |1/b - y - yl| + ulp(a yl) / 2 < 2^-49 + 2^-49
+//    (|yl| <= 2^-25, so ulp(yl) <= 2^-49 and ulp(a yl) <= 2^-48).  b < 2, so
+//    only A < B with |r| = 1 can be rounded to the wrong side; r is even for
+//    even B, so only odd B, and A = +-2^-25 mod B: one dividend per divisor
+//    (the other is below 2^23), which check_split finds by a modular inverse
+//    and tries (Brisebarre, Muller and Raina's method, cited above, bounds and
+//    tries the candidates the same way).  1.27% of all divisors fail there;
+//    moving yl by one ulp up or down cures 95% of those.  The moved sum is off
+//    by less than 2.5 2^-48, so its candidates are A < B with |r| in {1, 3}
+//    and A >= B with |r| = 1, all tried.  A divisor that stays unchecked
+//    (0.06%) keeps the corrected quotient.  The bound needs RN(a*yl) normal:
+//    |a| >= kSplitLo (|yl| is 0 or at least 2^-48 / |b|, and |b| <= 2^30).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -136,6 +156,103 @@ __device__ __forceinline__ float2 recip_quot2(float2 a, const Recip2 &k) {
   const float2 q0 = __ffma2_rn(a, k.y, __fmul2_rn(a, k.yl));
   const float2 r = __ffma2_rn(q0, k.nb, a);
   return __ffma2_rn(r, k.y, q0);
+}
+
+// a / b for a divisor check_split accepted, kSplitLo <= |a| < infinity or NaN.
+// Divisors below kSplitMin are left out: a * yl could overflow beside a
+// finite a, to an infinity of the wrong sign that nothing would show.
+constexpr float kSplitLo = 0x1p-48f, kSplitMin = 0x1p-20f;
+__device__ __forceinline__ float split_quot(float a, const Recip &k) {
+  return __fmaf_rn(a, k.y, __fmul_rn(a, k.yl));
+}
+__device__ __forceinline__ float2 split_quot2(float2 a, const Recip2 &k) {
+  return __ffma2_rn(a, k.y, __fmul2_rn(a, k.yl));
+}
+
+// b's significand in [1, 2) and the parts of its reciprocal: a power of two
+// and a sign away from b's own, exact.
+struct SplitBase {
+  Recip n;
+  uint32_t B, A1;  // the significand as an integer, 2^-25 mod B (odd B)
+};
+__device__ __forceinline__ SplitBase split_base(const Recip &k) {
+  SplitBase s;
+  const uint32_t bits = __float_as_uint(-k.nb);
+  const float scale = __uint_as_float(bits & 0xff800000u);
+  s.n.nb = -__uint_as_float(0x3f800000u | (bits & 0x7fffffu));
+  s.n.y = __fmul_rn(k.y, scale);
+  s.n.yl = __fmul_rn(k.yl, scale);
+  const uint32_t B = (bits & 0x7fffffu) | 0x800000u;
+  uint32_t x = (3u * B) ^ 2u;  // B^-1 mod 2^5, then by Newton mod 2^10, 2^20, 2^32
+  x *= 2u - B * x;
+  x *= 2u - B * x;
+  x *= 2u - B * x;
+  const uint32_t t = (0u - x) & 0x1ffffffu;  // -B^-1 mod 2^25
+  s.B = B;
+  s.A1 = (uint32_t)((1ull + (uint64_t)B * t) >> 25);
+  return s;
+}
+// True when the split quotient with yl rounds a = A 2^-23 like the corrected
+// one; A outside [2^23, 2^24) is no candidate.
+__device__ __forceinline__ bool split_right_at(uint32_t A, const Recip &n, float yl) {
+  const float a = __fmul_rn(__uint2float_rn(A), 0x1p-23f);
+  const bool right = __fmaf_rn(a, n.y, __fmul_rn(a, yl)) == recip_quot(a, n);
+  return (A - 0x800000u >= 0x800000u) | right;
+}
+// Whether split_quot is RN(a/b) for every dividend of its range, k as
+// make_recip gives it.  (A1 and B - A1 add up to B < 2^24: only the larger
+// can be a significand.)
+__device__ __forceinline__ bool split_as_made(const Recip &k) {
+  const SplitBase s = split_base(k);
+  return !(s.B & 1u) | split_right_at(max(s.A1, s.B - s.A1), s.n, s.n.yl);
+}
+// How many ulps (-1 or 1) yl must move for that; 0: neither helps.  (The
+// corrected quotient stays exact with the moved yl: its q0 is still within
+// an ulp.)
+__device__ __forceinline__ int split_move(const Recip &k) {
+  const SplitBase s = split_base(k);
+  const uint32_t B = s.B, A1 = s.A1;
+  const uint32_t A2 = 2u * A1 >= B ? 2u * A1 - B : 2u * A1;  // 2^-24 mod B
+  const uint32_t A3 = A1 + A2 >= B ? A1 + A2 - B : A1 + A2;  // 3 2^-25 mod B
+#pragma unroll 1
+  for (int d = -1; d <= 1; d += 2) {
+    const float yl = __int_as_float(__float_as_int(s.n.yl) + d);
+    if (split_right_at(max(A1, B - A1), s.n, yl) && split_right_at(max(A3, B - A3), s.n, yl) &&
+        split_right_at(B + A2, s.n, yl) && split_right_at(2u * B - A2, s.n, yl))
+      return d;
+  }
+  return 0;
+}
+// Checks N divisors, moving their yl where that makes the split quotient
+// right; returns the mask of those it is right for.  The moves are rare
+// (1.27% of divisors) and come last, one divisor of each lane at a time,
+// whichever it is.
+template <int N>
+__device__ __forceinline__ uint32_t check_split(const float (&nb)[N], const float (&y)[N],
+                                                float (&yl)[N]) {
+  uint32_t fail = 0, right = 0;
+#pragma unroll
+  for (int d = 0; d < N; d++) {
+    const Recip k = {nb[d], y[d], yl[d]};
+    if (fabsf(nb[d]) < kSplitMin) continue;
+    if (split_as_made(k)) right |= 1u << d;
+    else fail |= 1u << d;
+  }
+#pragma unroll 1
+  while (fail) {
+    const uint32_t bit = fail & (0u - fail);
+    Recip k = {nb[0], y[0], yl[0]};
+#pragma unroll
+    for (int d = 1; d < N; d++)
+      if (bit == 1u << d) k = {nb[d], y[d], yl[d]};
+    const int move = split_move(k);
+    if (move) right |= bit;
+#pragma unroll
+    for (int d = 0; d < N; d++)
+      if (bit == 1u << d) yl[d] = __int_as_float(__float_as_int(yl[d]) + move);
+    fail ^= bit;
+  }
+  return right;
 }
 
 // True for a nonzero |a| below tiny (NaN: false).

@@ -160,6 +160,23 @@ struct DualFast {
   }
 };
 
+// min(m, |a|, |b|); a NaN argument is ignored.
+__device__ __forceinline__ float min_abs(float m, float a, float b) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(fabsf(a)), "f"(fabsf(b)));
+  return r;
+}
+// i, v: the least |I0| and |V0| of a wire (NaN ones apart).  See exact_steps.
+__device__ __forceinline__ bool sound_wire(float i, float v, float L, float C, float dt) {
+  return (i >= 0x1p-50f) & (v >= 0x1p-50f) & (fabsf(L) >= 0x1p-43f) & (fabsf(C) >= 0x1p-20f) &
+         (__fmul_rn(v, fabsf(C)) >= __fmul_rn(0x1p-22f, dt));
+}
+// Which wires' values are NaN: bit 0 the first (or only) wire, bit 1 the second.
+__device__ __forceinline__ uint32_t nan_bits(float a) { return a != a ? 1u : 0u; }
+__device__ __forceinline__ uint32_t nan_bits(float2 a) {
+  return (a.x != a.x ? 1u : 0u) | (a.y != a.y ? 2u : 0u);
+}
+
 // EXACT, two wires per thread: the reference's operations in the reference's
 // order, each rounded as IEEE fp32 rounds it, with the 29 divisions of a
 // wire-step done as correctly rounded quotients by precomputed reciprocals
@@ -178,6 +195,7 @@ struct DualFast {
 // split reciprocal (2 operations); otherwise they are corrected quotients too.
 template <bool DTF>
 struct DualExact {
+  static constexpr bool kFree = DTF;  // has free steps (exact_steps)
   float2 L, dt2, neg1;
   Recip2 kR, kC, kdt;
   float dt;
@@ -289,72 +307,288 @@ struct DualExact {
       }
     }
   }
-  // step() for a state whose 10 currents and 9 wire voltages are all NaN,
-  // in both wires.  Such a state stays NaN -- every new current and voltage
-  // depends on a NaN of the previous step -- so every dividend is NaN, every
-  // guard of step() lets it pass and step() takes exactly these operations:
-  // the same arithmetic without the compares and the branches.
-  __device__ __forceinline__ void step_all_nan(float2 (&ni)[10], float2 (&nv)[11],
-                                               const float2 (&nI0)[10],
-                                               const float2 (&V0)[9]) const {
-    float2 a2[10];
+  // Which divisors take the split quotient in both wires (check_split):
+  // bit 0 R, bit 1 C.
+  __device__ __forceinline__ uint32_t check() {
+    const float nb[4] = {kR.nb.x, kR.nb.y, kC.nb.x, kC.nb.y};
+    const float y[4] = {kR.y.x, kR.y.y, kC.y.x, kC.y.y};
+    float yl[4] = {kR.yl.x, kR.yl.y, kC.yl.x, kC.yl.y};
+    const uint32_t right = check_split(nb, y, yl);
+    kR.yl = make_float2(yl[0], yl[1]);
+    kC.yl = make_float2(yl[2], yl[3]);
+    return ((right & 3u) == 3u ? 1u : 0u) | (right >= 12u ? 2u : 0u);
+  }
+  // step() without guards and branches.  SPLIT bit 0 (1): the quotients by R
+  // (C) are split quotients (2 operations), otherwise corrected ones (4).
+  // LOW: low collects the least |dividend| of
+  // R and C (NaN ones apart).  exact_steps says when the result is step()'s.
+  template <uint32_t SPLIT, bool LOW>
+  __device__ __forceinline__ void step_free(float2 (&ni)[10], float2 (&nv)[11],
+                                            const float2 (&nI0)[10], const float2 (&V0)[9],
+                                            float &low) const {
 #pragma unroll
     for (int k = 0; k < 10; k++) {
       const float2 a1 = __fmul2_rn(L, __fadd2_rn(ni[k], nI0[k]));
-      a2[k] = __ffma2_rn(dt_div(a1), neg1, __ffma2_rn(nv[k], neg1, nv[k + 1]));
+      const float2 a2 = __ffma2_rn(dt_div(a1), neg1, __ffma2_rn(nv[k], neg1, nv[k + 1]));
+      if (LOW) low = min_abs(low, a2.x, a2.y);
+      ni[k] = SPLIT & 1u ? split_quot2(a2, kR) : recip_quot2(a2, kR);
     }
 #pragma unroll
-    for (int k = 0; k < 10; k++) ni[k] = recip_quot2(a2[k], kR);
-    float2 a3[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) a3[k] = __fmul2_rn(dt2, __ffma2_rn(ni[k + 1], neg1, ni[k]));
-#pragma unroll
-    for (int k = 0; k < 9; k++) nv[k + 1] = __fadd2_rn(V0[k], recip_quot2(a3[k], kC));
+    for (int k = 0; k < 9; k++) {
+      const float2 a3 = __fmul2_rn(dt2, __ffma2_rn(ni[k + 1], neg1, ni[k]));
+      if (LOW) low = min_abs(low, a3.x, a3.y);
+      nv[k + 1] = __fadd2_rn(V0[k], SPLIT & 2u ? split_quot2(a3, kC) : recip_quot2(a3, kC));
+    }
   }
-  static __device__ __forceinline__ bool first_nan(const float2 (&ni)[10]) {
-    return ni[0].x != ni[0].x;
+  // The loop's constants keep every dividend's tininess from mattering
+  // (exact_steps).
+  __device__ __forceinline__ bool sound(const float2 (&nI0)[10], const float2 (&V0)[9]) const {
+    float ix = fabsf(nI0[0].x), iy = fabsf(nI0[0].y), vx = fabsf(V0[0].x), vy = fabsf(V0[0].y);
+#pragma unroll
+    for (int k = 1; k < 10; k++) {
+      ix = fminf(ix, fabsf(nI0[k].x));
+      iy = fminf(iy, fabsf(nI0[k].y));
+    }
+#pragma unroll
+    for (int k = 1; k < 9; k++) {
+      vx = fminf(vx, fabsf(V0[k].x));
+      vy = fminf(vy, fabsf(V0[k].y));
+    }
+    return sound_wire(ix, vx, L.x, kC.nb.x, dt) & sound_wire(iy, vy, L.y, kC.nb.y, dt);
   }
-  static __device__ __forceinline__ bool all_nan(const float2 (&ni)[10], const float2 (&nv)[11]) {
-    bool nan = true;
+  // step() for a state whose 10 currents and 9 wire voltages are all NaN,
+  // in both wires.  Such a state stays NaN -- every new current and voltage
+  // depends on a NaN of the previous step -- so every dividend is NaN and any
+  // form of quotient gives step()'s NaN: the split quotients, no compares.
+  __device__ __forceinline__ void step_all_nan(float2 (&ni)[10], float2 (&nv)[11],
+                                               const float2 (&nI0)[10],
+                                               const float2 (&V0)[9]) const {
 #pragma unroll
-    for (int k = 0; k < 10; k++) nan &= (ni[k].x != ni[k].x) & (ni[k].y != ni[k].y);
+    for (int k = 0; k < 10; k++) {
+      const float2 a1 = __fmul2_rn(L, __fadd2_rn(ni[k], nI0[k]));
+      ni[k] = split_quot2(__ffma2_rn(dt_div(a1), neg1, __ffma2_rn(nv[k], neg1, nv[k + 1])), kR);
+    }
 #pragma unroll
-    for (int k = 1; k < 10; k++) nan &= (nv[k].x != nv[k].x) & (nv[k].y != nv[k].y);
+    for (int k = 0; k < 9; k++)
+      nv[k + 1] = __fadd2_rn(
+          V0[k], split_quot2(__fmul2_rn(dt2, __ffma2_rn(ni[k + 1], neg1, ni[k])), kC));
+  }
+  static constexpr uint32_t kWires = 3u;  // nan_bits of both wires
+  // NaN where any of a wire's currents or voltages is NaN (or infinities
+  // cancel).
+  static __device__ __forceinline__ float2 state_sum(const float2 (&ni)[10],
+                                                     const float2 (&nv)[11]) {
+    float2 s = ni[9], t = nv[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) s = __fadd2_rn(s, ni[k]);
+#pragma unroll
+    for (int k = 1; k < 9; k++) t = __fadd2_rn(t, nv[k]);
+    return __fadd2_rn(s, t);
+  }
+  static __device__ __forceinline__ float least_current(const float2 (&ni)[10]) {
+    float m = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int k = 0; k < 10; k++) m = min_abs(m, ni[k].x, ni[k].y);
+    return m;
+  }
+  // The wires whose 10 currents and 9 wire voltages are all NaN.
+  static __device__ __forceinline__ uint32_t all_nan(const float2 (&ni)[10],
+                                                     const float2 (&nv)[11]) {
+    uint32_t nan = nan_bits(ni[0]);
+    if (nan) {
+#pragma unroll
+      for (int k = 1; k < 10; k++) nan &= nan_bits(ni[k]) & nan_bits(nv[k]);
+    }
     return nan;
   }
 };
 
-// The inner loop of DualExact: step() in blocks of kNanCheckSteps; at each
-// block boundary, once the states of all the warp's wires have become all
-// NaN (as the reference's recurrence does within ~10-30 steps at the
-// benchmark's inductances, and stays), the remaining steps run with
-// step_all_nan -- every operation of every step still computed, the same
-// bits.
-constexpr int kNanCheckSteps = 16;
-template <typename Stepper, typename F>
-__device__ __forceinline__ void exact_steps(const Stepper &pk, int steps, F (&ni)[10], F (&nv)[11],
-                                            const F (&nI0)[10], const F (&V0)[9]) {
-  int j = 0;
-#pragma unroll 1
-  while (j < steps) {
-    // The full test only once the first current is NaN (one compare on a
-    // finite state); the switch only when every thread of the warp can take
-    // it, so that a warp never runs the two loops one after the other.
-    const bool mine = Stepper::first_nan(ni) && Stepper::all_nan(ni, nv);
-    if (__all_sync(__activemask(), mine)) break;
-    const int n = min(kNanCheckSteps, steps - j);
-#pragma unroll 1
-    for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
-    j += n;
+// The inner loop of DualExact and SoloExact.  The steps run in blocks; at a
+// block's start, once the states of all the warp's wires have become all NaN
+// (as the reference's recurrence does within ~10-30 steps at the benchmark's
+// inductances, and stays), the remaining steps run with step_all_nan -- every
+// operation of every step still computed, the same bits.
+//
+// A block runs without guards (step_free) and is checked as a whole at its
+// end; if the check fails in any lane the warp returns to the state saved in
+// shared memory and runs the block with step().  What could be wrong in a
+// free block, and why its check finds it:
+//  * Huge and infinite dividends.  A finite dividend gives the correctly
+//    rounded quotient or (the corrected quotient's q0 overflowing) NaN; an
+//    infinite one gives its infinity or NaN.  A NaN in place of a number does
+//    not get lost: a NaN current makes its own next value NaN, a NaN voltage
+//    the currents beside it.  So a wire's state that holds no NaN at the end
+//    was right throughout; one that was all NaN at the start stays so.
+//  * Tiny dividends and zeros.  Both quotients are right for |a| >= 2^-77 |b|
+//    (split: RN(a yl) is normal, |yl| >= 2^-48 / |b|; corrected: the remainder
+//    is representable, |b| >= 2^-20).  Below that the true quotient and the
+//    computed one are both at most 2^-76 -- the wrong bits, or a zero of the
+//    wrong sign, of something that small.  A block of LOW steps fails when it
+//    met a dividend below kSplitLo (corrected: kCLo).  Steps without LOW need
+//    sound constants (sound_wire), with which such a quotient never matters:
+//      - by C: V0 + q = V0 when |V0| >= 2^-50;
+//      - by R, in the wire's next step: i - I0 = -I0 when |I0| >= 2^-50;
+//      - by R, in the same step's i_k - i_k+1: if the neighbour is at least
+//        2^-50 the difference is the neighbour either way; otherwise the
+//        difference is at most 2^-49 and, divided by C, at most
+//        2^-48 dt/|C|, which V0 absorbs when |V0| >= 2^-22 dt/|C|;
+//      - by R, as the loop's result: the last block fails when a current's
+//        magnitude is below 2^-75;
+//      - a1 / dt is right: i - I0 is 0 or at least half an ulp of I0, 2^-75,
+//        so with |L| >= 2^-43 a1 is 0 or at least 2^-118 = kDtTiny.
+//    (With LOW a1 needs no check either, see dt_outside.)
+// A failed block costs its own steps once more: the first blocks are short,
+// and after a failure the next blocks run guarded, 1, 2, 4 and 8 of them as
+// failures repeat (a loop's first steps from zero currents, a blow-up, a
+// wire in equilibrium with zero differences).
+//
+// Why: the guards' 58 compares and two branches per paired step held the loop
+// at 75% of the FP32 pipe, and the corrected quotients are 76 of its 163
+// operations.  A free step has 125 operations and nothing else.  The 19
+// three-input minima of LOW are not free beside it: FMAs of three register
+// pairs keep the register ports busy.  1,048,576 wires, 1000 steps, GB300:
+// guarded 5.88 ms, free with LOW 4.64 ms, without 3.83 ms, all NaN 3.59 ms
+// (4.80 ms with corrected quotients); the 125 operations at the pipe's full
+// rate take 3.25 ms.  124,867 wires: 1.10 -> 0.64 ms.
+constexpr int kGuardedRun = 16;  // steps of a guarded block
+constexpr int kFirstRun = 8, kMostRun = 32;  // steps of a free block
+// Values per thread in shared memory: the state at a block's start (10
+// currents, 9 voltages), the two node voltages and yl of R and C.
+constexpr int kSavedState = 23;
+// Checking the divisors costs about as much as 5 steps; below this many steps
+// the loop runs guarded.
+constexpr int kFreeSteps = 16;
+
+template <int STRIDE, typename F>
+__device__ __forceinline__ void save_state(F *save, const F (&ni)[10], const F (&nv)[11]) {
+#pragma unroll
+  for (int k = 0; k < 10; k++) save[k * STRIDE] = ni[k];
+#pragma unroll
+  for (int k = 0; k < 9; k++) save[(10 + k) * STRIDE] = nv[k + 1];
+}
+template <int STRIDE, typename F>
+__device__ __forceinline__ void load_state(const F *save, F (&ni)[10], F (&nv)[11]) {
+#pragma unroll
+  for (int k = 0; k < 10; k++) ni[k] = save[k * STRIDE];
+#pragma unroll
+  for (int k = 0; k < 9; k++) nv[k + 1] = save[(10 + k) * STRIDE];
+}
+
+// ni, nv: the state before the first step, and after the last.  wires: the
+// thread's wires in global memory (SoloWire, DualWires), unchanged until the
+// loop is done: their constants are loaded again for each stretch of blocks
+// rather than kept over a guarded one.
+template <int STRIDE, typename Stepper, typename Wires, typename F>
+__device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&ni)[10],
+                                            F (&nv)[11], F *save) {
+  const uint32_t lanes = __activemask();
+  uint32_t split = 0;
+  bool sound = false;
+  int j = 0, run = kFirstRun, guarded = 0, penalty = 1;
+  save_state<STRIDE>(save, ni, nv);
+  save[19 * STRIDE] = nv[0];
+  save[20 * STRIDE] = nv[10];
+  if (Stepper::kFree && steps >= kFreeSteps) {
+    Stepper pk = wires.template stepper<Stepper>();
+    const uint32_t checked = pk.check();
+    split = (__all_sync(lanes, checked & 1u) ? 1u : 0u) | (__all_sync(lanes, checked & 2u) ? 2u : 0u);
+    F nI0[10], V0[9];
+    wires.load(nI0, V0);
+    sound = __all_sync(lanes, pk.sound(nI0, V0));
+    save[21 * STRIDE] = pk.kR.yl;
+    save[22 * STRIDE] = pk.kC.yl;
+  } else {
+    guarded = steps;  // no free block
   }
 #pragma unroll 1
-  for (; j < steps; j++) pk.step_all_nan(ni, nv, nI0, V0);
+  while (j < steps) {
+    load_state<STRIDE>(save, ni, nv);
+    uint32_t nan = Stepper::all_nan(ni, nv);
+    // the switch only when every thread of the warp can take it, so that a
+    // warp never runs the two loops one after the other
+    if (__all_sync(lanes, nan == Stepper::kWires)) break;
+    if (Stepper::kFree && guarded == 0) {
+      bool right = true;
+      if (sound) {
+        Stepper pk = wires.template stepper<Stepper>();
+        pk.kR.yl = save[21 * STRIDE];
+        pk.kC.yl = save[22 * STRIDE];
+        F nI0[10], V0[9];
+        wires.load(nI0, V0);
+        nv[0] = save[19 * STRIDE];
+        nv[10] = save[20 * STRIDE];
+        bool all_nan = false;
+        float none = 0.0f;
+#pragma unroll 1
+        while (!all_nan && j < steps) {
+          const int n = min(run, steps - j);
+          // one loop per pair of quotient forms: a warp with one unchecked
+          // divisor (8% of paired warps) keeps the other's split quotients
+          if (split == 3u) {
+#pragma unroll 1
+            for (int i = 0; i < n; i++) pk.template step_free<3, false>(ni, nv, nI0, V0, none);
+          } else if (split == 2u) {
+#pragma unroll 1
+            for (int i = 0; i < n; i++) pk.template step_free<2, false>(ni, nv, nI0, V0, none);
+          } else if (split == 1u) {
+#pragma unroll 1
+            for (int i = 0; i < n; i++) pk.template step_free<1, false>(ni, nv, nI0, V0, none);
+          } else {
+#pragma unroll 1
+            for (int i = 0; i < n; i++) pk.template step_free<0, false>(ni, nv, nI0, V0, none);
+          }
+          right = (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
+          if (j + n == steps) right &= Stepper::least_current(ni) >= 0x1p-75f;
+          right = __all_sync(lanes, right);
+          if (!right) break;
+          j += n;
+          if (run == kMostRun) penalty = 1;
+          run = min(2 * run, kMostRun);
+          save_state<STRIDE>(save, ni, nv);
+          nan = Stepper::all_nan(ni, nv);
+          all_nan = __all_sync(lanes, nan == Stepper::kWires);
+        }
+      } else {
+        const int n = min(run, steps - j);
+        right = wires.template low<Stepper, STRIDE>(n, split == 3u, nan, save);
+        right = __all_sync(lanes, right);
+        if (right) {
+          j += n;
+          if (run == kMostRun) penalty = 1;
+          run = min(2 * run, kMostRun);
+        } else {
+          save_state<STRIDE>(save, ni, nv);
+        }
+      }
+      if (right) continue;
+      guarded = penalty;
+      penalty = min(2 * penalty, 8);
+      run = kFirstRun;
+    }
+    const int n = min(kGuardedRun, steps - j);
+    wires.template guarded<Stepper, STRIDE>(n, save);
+    j += n;
+    guarded--;
+  }
+  if (j < steps) {
+    const Stepper pk = wires.template stepper<Stepper>();
+    F nI0[10], V0[9];
+    wires.load(nI0, V0);
+    load_state<STRIDE>(save, ni, nv);
+    nv[0] = save[19 * STRIDE];
+    nv[10] = save[20 * STRIDE];
+#pragma unroll 1
+    for (; j < steps; j++) pk.step_all_nan(ni, nv, nI0, V0);
+  } else {
+    load_state<STRIDE>(save, ni, nv);
+  }
 }
 
 // EXACT, one wire per thread: DualExact's arithmetic and guards on scalar
 // instructions (the batched kernel's one-wire tiles).  Bit-identical to it.
 template <bool DTF>
 struct SoloExact {
+  static constexpr bool kFree = DTF;
   float L, dt;
   Recip kR, kC, kdt;
   __device__ __forceinline__ SoloExact(float l, float r, float c, float d) {
@@ -431,34 +665,81 @@ struct SoloExact {
       }
     }
   }
-  // step() for a state whose 10 currents and 9 wire voltages are all NaN:
-  // the same operations without the compares and the branches (see
-  // DualExact::step_all_nan).
-  __device__ __forceinline__ void step_all_nan(float (&ni)[10], float (&nv)[11],
-                                               const float (&I0)[10],
-                                               const float (&V0)[9]) const {
-    float a2[10];
+  // As in DualExact.
+  __device__ __forceinline__ uint32_t check() {
+    const float nb[2] = {kR.nb, kC.nb}, y[2] = {kR.y, kC.y};
+    float yl[2] = {kR.yl, kC.yl};
+    const uint32_t right = check_split(nb, y, yl);
+    kR.yl = yl[0];
+    kC.yl = yl[1];
+    return right;
+  }
+  template <uint32_t SPLIT, bool LOW>
+  __device__ __forceinline__ void step_free(float (&ni)[10], float (&nv)[11],
+                                            const float (&I0)[10], const float (&V0)[9],
+                                            float &low) const {
+    float a[10];
 #pragma unroll
     for (int k = 0; k < 10; k++) {
       const float a1 = __fmul_rn(L, __fsub_rn(ni[k], I0[k]));
-      const float q1 = DTF ? dt_quot(a1) : recip_quot(a1, kdt);
-      a2[k] = __fsub_rn(__fsub_rn(nv[k + 1], nv[k]), q1);
+      a[k] = __fsub_rn(__fsub_rn(nv[k + 1], nv[k]), dt_quot(a1));
+      ni[k] = SPLIT & 1u ? split_quot(a[k], kR) : recip_quot(a[k], kR);
     }
 #pragma unroll
-    for (int k = 0; k < 10; k++) ni[k] = recip_quot(a2[k], kR);
-    float a3[9];
+    for (int k = 0; k < 10; k += 2)
+      if (LOW) low = min_abs(low, a[k], a[k + 1]);
 #pragma unroll
-    for (int k = 0; k < 9; k++) a3[k] = __fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1]));
+    for (int k = 0; k < 9; k++) {
+      a[k] = __fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1]));
+      nv[k + 1] = __fadd_rn(V0[k], SPLIT & 2u ? split_quot(a[k], kC) : recip_quot(a[k], kC));
+    }
 #pragma unroll
-    for (int k = 0; k < 9; k++) nv[k + 1] = __fadd_rn(V0[k], recip_quot(a3[k], kC));
+    for (int k = 0; k < 8; k += 2)
+      if (LOW) low = min_abs(low, a[k], a[k + 1]);
+    if (LOW) low = fminf(low, fabsf(a[8]));
   }
-  static __device__ __forceinline__ bool first_nan(const float (&ni)[10]) { return ni[0] != ni[0]; }
-  static __device__ __forceinline__ bool all_nan(const float (&ni)[10], const float (&nv)[11]) {
-    bool nan = true;
+  __device__ __forceinline__ bool sound(const float (&I0)[10], const float (&V0)[9]) const {
+    float i = fabsf(I0[0]), v = fabsf(V0[0]);
 #pragma unroll
-    for (int k = 0; k < 10; k++) nan &= ni[k] != ni[k];
+    for (int k = 1; k < 10; k++) i = fminf(i, fabsf(I0[k]));
 #pragma unroll
-    for (int k = 1; k < 10; k++) nan &= nv[k] != nv[k];
+    for (int k = 1; k < 9; k++) v = fminf(v, fabsf(V0[k]));
+    return sound_wire(i, v, L, kC.nb, dt);
+  }
+  __device__ __forceinline__ void step_all_nan(float (&ni)[10], float (&nv)[11],
+                                               const float (&I0)[10],
+                                               const float (&V0)[9]) const {
+#pragma unroll
+    for (int k = 0; k < 10; k++) {
+      const float a1 = __fmul_rn(L, __fsub_rn(ni[k], I0[k]));
+      const float q1 = DTF ? dt_quot(a1) : split_quot(a1, kdt);
+      ni[k] = split_quot(__fsub_rn(__fsub_rn(nv[k + 1], nv[k]), q1), kR);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      nv[k + 1] = __fadd_rn(V0[k], split_quot(__fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1])), kC));
+  }
+  static constexpr uint32_t kWires = 1u;
+  static __device__ __forceinline__ float state_sum(const float (&ni)[10], const float (&nv)[11]) {
+    float s = ni[9], t = nv[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) s = __fadd_rn(s, ni[k]);
+#pragma unroll
+    for (int k = 1; k < 9; k++) t = __fadd_rn(t, nv[k]);
+    return __fadd_rn(s, t);
+  }
+  static __device__ __forceinline__ float least_current(const float (&ni)[10]) {
+    float m = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int k = 0; k < 10; k += 2) m = min_abs(m, ni[k], ni[k + 1]);
+    return m;
+  }
+  static __device__ __forceinline__ uint32_t all_nan(const float (&ni)[10], const float (&nv)[11]) {
+    uint32_t nan = nan_bits(ni[0]);
+    if (nan) {
+#pragma unroll
+      for (int k = 1; k < 10; k++) nan &= nan_bits(ni[k]) & nan_bits(nv[k]);
+    }
     return nan;
   }
 };
@@ -483,11 +764,102 @@ struct NodeVolts {
   const float *pvt, *shr, *ghost;
 };
 
+// The wires of a thread, as exact_steps takes them.
+struct WireSource {
+  const float *L, *R, *C, *cur, *vol;
+  int64_t S;
+  float dt;
+};
+// n guarded steps on the state in `save`.  Out of line, as the LOW steps
+// below: they are rare, and their registers (all dividends of a phase at
+// once) would spill the free steps' loop.
+template <typename Stepper, int STRIDE, typename Wires, typename F>
+__device__ __noinline__ void guarded_steps(const Wires wires, int n, F *save) {
+  const Stepper pk = wires.template stepper<Stepper>();
+  F nI0[10], V0[9], ni[10], nv[11];
+  wires.load(nI0, V0);
+  load_state<STRIDE>(save, ni, nv);
+  nv[0] = save[19 * STRIDE];
+  nv[10] = save[20 * STRIDE];
+#pragma unroll 1
+  for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
+  save_state<STRIDE>(save, ni, nv);
+}
+// n free steps with LOW on the state in `save`; whether they were right.
+template <typename Stepper, int STRIDE, typename Wires, typename F>
+__device__ __noinline__ bool low_steps(const Wires wires, int n, bool split, uint32_t nan,
+                                       F *save) {
+  Stepper pk = wires.template stepper<Stepper>();
+  pk.kR.yl = save[21 * STRIDE];
+  pk.kC.yl = save[22 * STRIDE];
+  F nI0[10], V0[9], ni[10], nv[11];
+  wires.load(nI0, V0);
+  load_state<STRIDE>(save, ni, nv);
+  nv[0] = save[19 * STRIDE];
+  nv[10] = save[20 * STRIDE];
+  float low = __int_as_float(0x7f800000);
+  if (split) {
+#pragma unroll 1
+    for (int i = 0; i < n; i++) pk.template step_free<3, true>(ni, nv, nI0, V0, low);
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < n; i++) pk.template step_free<0, true>(ni, nv, nI0, V0, low);
+  }
+  save_state<STRIDE>(save, ni, nv);
+  return low >= (split ? kSplitLo : kCLo) &&
+         (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
+}
+struct SoloWire : WireSource {
+  int64_t w;
+  template <typename Stepper>
+  __device__ __forceinline__ Stepper stepper() const {
+    return Stepper(L[w], R[w], C[w], dt);
+  }
+  __device__ __forceinline__ void load(float (&I0)[10], float (&V0)[9]) const {
+#pragma unroll
+    for (int k = 0; k < 10; k++) I0[k] = cur[k * S + w];
+#pragma unroll
+    for (int k = 0; k < 9; k++) V0[k] = vol[k * S + w];
+  }
+  template <typename Stepper, int STRIDE>
+  __device__ __forceinline__ void guarded(int n, float *save) const {
+    guarded_steps<Stepper, STRIDE>(*this, n, save);
+  }
+  template <typename Stepper, int STRIDE>
+  __device__ __forceinline__ bool low(int n, bool split, uint32_t nan, float *save) const {
+    return low_steps<Stepper, STRIDE>(*this, n, split, nan, save);
+  }
+};
+struct DualWires : WireSource {
+  int64_t wa, wb;
+  template <typename Stepper>
+  __device__ __forceinline__ Stepper stepper() const {
+    return Stepper(make_float2(L[wa], L[wb]), make_float2(R[wa], R[wb]),
+                   make_float2(C[wa], C[wb]), dt);
+  }
+  __device__ __forceinline__ void load(float2 (&nI0)[10], float2 (&V0)[9]) const {
+#pragma unroll
+    for (int k = 0; k < 10; k++) nI0[k] = make_float2(-cur[k * S + wa], -cur[k * S + wb]);
+#pragma unroll
+    for (int k = 0; k < 9; k++) V0[k] = make_float2(vol[k * S + wa], vol[k * S + wb]);
+  }
+  template <typename Stepper, int STRIDE>
+  __device__ __forceinline__ void guarded(int n, float2 *save) const {
+    guarded_steps<Stepper, STRIDE>(*this, n, save);
+  }
+  template <typename Stepper, int STRIDE>
+  __device__ __forceinline__ bool low(int n, bool split, uint32_t nan, float2 *save) const {
+    return low_steps<Stepper, STRIDE>(*this, n, split, nan, save);
+  }
+};
+
 // One wire's whole inner loop: load, S steps in registers, store.
-template <int MODE, int INIT>
+// save: this thread's column of kSavedState rows of STRIDE floats in shared
+// memory (EXACT).
+template <int MODE, int INIT, int STRIDE = 1>
 __device__ __forceinline__ void cnc_wire(int64_t w, const WireArrays &a, const NodeVolts &nv_in,
-                                         int steps, float dt, float *i0_out = nullptr,
-                                         float *i9_out = nullptr) {
+                                         int steps, float dt, float *save = nullptr,
+                                         float *i0_out = nullptr, float *i9_out = nullptr) {
   const int64_t S = a.S;
   float I0[10], V0[9], ni[10], nv[11];
 #pragma unroll
@@ -563,12 +935,12 @@ __device__ __forceinline__ void cnc_wire(int64_t w, const WireArrays &a, const N
     }
   } else if (MODE == CKT_MODE_EXACT && __float_as_uint(dt) == kDtBits &&
              SoloExact<true>::eligible(a.R[w], a.C[w], dt)) {
-    const SoloExact<true> ws(a.L[w], a.R[w], a.C[w], dt);
-    exact_steps(ws, steps, ni, nv, I0, V0);
+    const SoloWire ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, w};
+    exact_steps<STRIDE, SoloExact<true>>(ws, steps, ni, nv, save);
   } else if (MODE == CKT_MODE_EXACT && __float_as_uint(dt) != kDtBits &&
              SoloExact<false>::eligible(a.R[w], a.C[w], dt)) {
-    const SoloExact<false> ws(a.L[w], a.R[w], a.C[w], dt);
-    exact_steps(ws, steps, ni, nv, I0, V0);
+    const SoloWire ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, w};
+    exact_steps<STRIDE, SoloExact<false>>(ws, steps, ni, nv, save);
   } else {
     static_assert(MODE == CKT_MODE_EXACT || MODE == CKT_MODE_EXACT_DIVIDE, "unknown mode");
     const DivideStep ws(a.L[w], a.R[w], a.C[w], dt);
@@ -593,10 +965,13 @@ __device__ __forceinline__ void cnc_wire(int64_t w, const WireArrays &a, const N
 // block handles wires base + t and base + t + 256, so each field's loads and
 // stores stay one contiguous line per warp.  Without a partner wire the
 // thread runs its wire in both lanes and stores one.
-template <int MODE, int INIT>
+// save: this thread's column of kSavedState rows of STRIDE float2 in shared
+// memory (EXACT).
+template <int MODE, int INIT, int STRIDE>
 __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b,
                                               const WireArrays &a, const NodeVolts &nvin,
-                                              int steps, float dt, float2 *i0_out = nullptr,
+                                              int steps, float dt, float2 *save,
+                                              float2 *i0_out = nullptr,
                                               float2 *i9_out = nullptr) {
   static_assert(MODE == CKT_MODE_FAST || MODE == CKT_MODE_EXACT, "paired modes: FAST, EXACT");
   const int64_t S = a.S;
@@ -607,10 +982,10 @@ __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b
       !(dt_fixed ? DualExact<true>::eligible(R2, C2, dt) : DualExact<false>::eligible(R2, C2, dt))) {
     // a divisor outside the corrected quotients' range: the divide routine
     float ia0, ia9, ib0, ib9;
-    cnc_wire<CKT_MODE_EXACT_DIVIDE, INIT>(wa, a, nvin, steps, dt, &ia0, &ia9);
+    cnc_wire<CKT_MODE_EXACT_DIVIDE, INIT>(wa, a, nvin, steps, dt, nullptr, &ia0, &ia9);
     ib0 = ia0;
     ib9 = ia9;
-    if (has_b) cnc_wire<CKT_MODE_EXACT_DIVIDE, INIT>(wb, a, nvin, steps, dt, &ib0, &ib9);
+    if (has_b) cnc_wire<CKT_MODE_EXACT_DIVIDE, INIT>(wb, a, nvin, steps, dt, nullptr, &ib0, &ib9);
     if (i0_out) *i0_out = make_float2(ia0, ib0);
     if (i9_out) *i9_out = make_float2(ia9, ib9);
     return;
@@ -655,11 +1030,11 @@ __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b
       for (int k = 0; k < 10; k++) ni[k] = make_float2(-nI0[k].x, -nI0[k].y);  // no step: I0
     }
   } else if (dt_fixed) {
-    const DualExact<true> pk(L2, R2, C2, dt);
-    exact_steps(pk, steps, ni, nv, nI0, V0);
+    const DualWires ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, wa, wb};
+    exact_steps<STRIDE, DualExact<true>>(ws, steps, ni, nv, save);
   } else {
-    const DualExact<false> pk(L2, R2, C2, dt);
-    exact_steps(pk, steps, ni, nv, nI0, V0);
+    const DualWires ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, wa, wb};
+    exact_steps<STRIDE, DualExact<false>>(ws, steps, ni, nv, save);
   }
 #pragma unroll
   for (int k = 0; k < 10; k++) a.cur[k * S + wa] = ni[k].x;
@@ -681,20 +1056,26 @@ template <int MODE, int INIT>
 __global__ void __launch_bounds__(kPairBlock, 2)
     cnc_pair_kernel(uint32_t first_wire, uint32_t num_wires, WireArrays a, NodeVolts v, int steps,
                     float dt) {
+  __shared__ float2 save[MODE == CKT_MODE_EXACT ? kSavedState * kPairBlock : 1];
   const uint32_t ta = blockIdx.x * (2 * kPairBlock) + threadIdx.x, tb = ta + kPairBlock;
   if (ta >= num_wires) return;
   const bool has_b = tb < num_wires;
-  cnc_wire_pair<MODE, INIT>((int64_t)first_wire + ta, (int64_t)first_wire + (has_b ? tb : ta),
-                            has_b, a, v, steps, dt);
+  cnc_wire_pair<MODE, INIT, kPairBlock>((int64_t)first_wire + ta,
+                                        (int64_t)first_wire + (has_b ? tb : ta), has_b, a, v,
+                                        steps, dt,
+                                        save + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0));
 }
 
 template <int MODE, int INIT>
 __global__ void __launch_bounds__(256)
     cnc_kernel(uint32_t first_wire, uint32_t num_wires, WireArrays a, NodeVolts v, int steps,
                float dt) {
+  // EXACT launches have one-warp blocks
+  __shared__ float save[MODE == CKT_MODE_EXACT ? kSavedState * 32 : 1];
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= num_wires) return;
-  cnc_wire<MODE, INIT>((int64_t)first_wire + t, a, v, steps, dt);
+  cnc_wire<MODE, INIT, 32>((int64_t)first_wire + t, a, v, steps, dt,
+                           save + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0));
 }
 
 // ---------------------------------------------------------------------------

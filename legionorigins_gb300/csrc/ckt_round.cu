@@ -83,7 +83,11 @@ int round_blocks_per_sm(const ckt_batch_config &c, int *out) {
       &a, reinterpret_cast<const void *>(round_kernel_for(CKT_MODE_FAST, c)), c.block, 0));
   CKT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &b, reinterpret_cast<const void *>(round_kernel_for(CKT_MODE_EXACT, c)), c.block, 0));
-  *out = std::max(1, std::min(a, b));
+  // The modes' kernels of one configuration may differ (EXACT's one-wire tiles
+  // use more registers).  The grid is the larger: a block that is not resident
+  // yet holds no ticket, so nothing waits for it, and it finds none left when
+  // it starts.
+  *out = std::max(1, std::max(a, b));
   return CKT_OK;
 }
 

@@ -33,7 +33,7 @@ void build_round_table(std::vector<RoundCircuit> &circuits, const ckt_batch_conf
 // The kernel for (mode, launch shape), or null.
 BatchKernelFn round_kernel_for(int mode, const ckt_batch_config &cfg);
 
-// Resident blocks per SM of the round kernel for this shape (both modes).
+// Most resident blocks per SM of the round kernel for this shape, over the modes.
 int round_blocks_per_sm(const ckt_batch_config &cfg, int *out);
 
 // One round: clears the sync words (ticket, error, done counters of C

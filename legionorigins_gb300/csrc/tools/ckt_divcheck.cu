@@ -191,9 +191,74 @@ __global__ void __launch_bounds__(256)
   warp_add(counts + 2, drawn);
 }
 
+// The split quotient by a checked divisor (check_split) against the divide
+// routine: dividends that come nearest to a rounding boundary (the residues
+// r 2^-25 mod B and r 2^-24 mod B, r odd and small, above and below B) and
+// random ones, at any exponent the quotient is used for.
+__global__ void __launch_bounds__(256)
+    split_quotient_check_kernel(uint64_t seed, uint64_t count, int32_t divisor,
+                                unsigned long long *counts) {
+  const int e0 = divisor == 0 ? -8 : -30, e1 = -e0 - 1;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t rounds = (count + stride - 1) / stride;
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t bad = 0, checked = 0, moved = 0, drawn = 0;
+  for (uint64_t r = 0; r < rounds; r++) {
+    const uint64_t i = r * stride + t;
+    if (i >= count) continue;
+    const uint64_t h1 = mix64(seed * 0x9e3779b97f4a7c15ull + 2 * i + 1);
+    const uint64_t h2 = mix64(h1 ^ 0x632be59bd9b4e019ull);
+    const float b = rand_float(h1, e0, e1);
+    const Recip made = make_recip(b);
+    const float nb[1] = {made.nb}, y[1] = {made.y};
+    float yl[1] = {made.yl};
+    drawn++;
+    if (!check_split(nb, y, yl)) continue;
+    checked++;
+    moved += yl[0] != made.yl;
+    const Recip k = {made.nb, made.y, yl[0]};
+    const uint32_t B = (__float_as_uint(b) & 0x7fffffu) | 0x800000u;
+    uint64_t A1 = 1;  // 2^-25 mod B for odd B, by halving
+    for (int q = 0; q < 25; q++) A1 = (A1 & 1u) ? (A1 + B) / 2 : A1 / 2;
+    for (uint32_t d = 0; d < 24; d++) {
+      const uint32_t odd = 2u * (d % 6u) + 1u;
+      uint32_t A = (uint32_t)((odd * A1 * (d < 12 ? 1u : 2u)) % B);
+      if (d % 12u >= 6u) A = B - A;
+      if (d >= 12) A += B;
+      if (A < 0x800000u || A > 0xffffffu)
+        A = 0x800000u | ((uint32_t)(mix64(h2 + d) >> 11) & 0x7fffffu);
+      // 2^-77 |b| <= |a| < 2^127
+      const int lo = (int)((__float_as_uint(b) >> 23) & 0xffu) - 127 - 76;
+      const int e = lo + (int)((uint32_t)(mix64(h2 ^ d) >> 40) % (uint32_t)(127 - lo));
+      const float a = ((h2 >> d) & 1u ? -1.0f : 1.0f) *
+                      __uint_as_float((uint32_t)(e + 127) << 23 | (A & 0x7fffffu));
+      bad += !same_float(split_quot(a, k), __fdiv_rn(a, b));
+    }
+  }
+  warp_add(counts + 0, bad);
+  warp_add(counts + 1, checked);
+  warp_add(counts + 2, moved);
+  warp_add(counts + 3, drawn);
+}
+
 }  // namespace ckt
 
 using namespace ckt;
+
+extern "C" int ckt_check_split_quotient(uint64_t seed, uint64_t count, int32_t divisor,
+                                        unsigned long long *counts, void *stream) {
+  CKT_REQUIRE(counts != nullptr, "counts is NULL");
+  CKT_REQUIRE(divisor == 0 || divisor == 1, "divisor must be 0 (R) or 1 (C), got %d", divisor);
+  if (count == 0) return CKT_OK;
+  int dev = 0, sms = 0;
+  CKT_CUDA(cudaGetDevice(&dev));
+  CKT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const uint64_t want = (count + 255) / 256;
+  const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)sms * 8);
+  split_quotient_check_kernel<<<grid, 256, 0, as_stream(stream)>>>(seed, count, divisor, counts);
+  CKT_CHECK_LAUNCH();
+  return CKT_OK;
+}
 
 extern "C" int ckt_check_dt_quotient(uint64_t begin, uint64_t count, unsigned long long *counts,
                                      void *stream) {

@@ -843,3 +843,44 @@ void ocl_wide_quotient_check(uint64_t seed, uint64_t n, int divisor, uint64_t *b
   *outside = nout;
   *drawn = nd;
 }
+
+/* The check of a divisor for the split quotient (see ckt_oracle.h). */
+static int sq_right_at(uint32_t A, float m, float y, float yl)
+{
+  if (A < (1u << 23) || A >= (1u << 24)) return 1;
+  const float a = ldexpf((float)A, -23);
+  return fmaf(a, y, a * yl) == a / m;
+}
+
+int ocl_split_divisor(float b, float *y, float *yl)
+{
+  *y = 1.0f / b;
+  *yl = fmaf(-b, *y, 1.0f) / b;
+  const uint32_t bits = wq_u(b), B = (bits & 0x7fffffu) | 0x800000u;
+  if (!(B & 1u)) return 1;
+  const float m = ldexpf((float)B, -23), my = 1.0f / m, myl = fmaf(-m, my, 1.0f) / m;
+  uint64_t A1 = 1; /* 2^-25 mod B, by halving */
+  for (int i = 0; i < 25; i++) A1 = (A1 & 1u) ? (A1 + B) / 2 : A1 / 2;
+  if (sq_right_at((uint32_t)A1, m, my, myl) && sq_right_at(B - (uint32_t)A1, m, my, myl)) return 1;
+  const uint32_t A2 = (uint32_t)(2 * A1 % B), A3 = (uint32_t)(3 * A1 % B);
+  for (int d = -1; d <= 1; d += 2) {
+    const float t = wq_bits(wq_u(myl) + (uint32_t)d);
+    if (sq_right_at((uint32_t)A1, m, my, t) && sq_right_at(B - (uint32_t)A1, m, my, t) &&
+        sq_right_at(A3, m, my, t) && sq_right_at(B - A3, m, my, t) && sq_right_at(B + A2, m, my, t) &&
+        sq_right_at(2 * B - A2, m, my, t)) {
+      *yl = wq_bits(wq_u(*yl) + (uint32_t)d);
+      return 2;
+    }
+  }
+  return 0;
+}
+
+uint64_t ocl_split_divisor_sweep(float b, float y, float yl, int exponent)
+{
+  uint64_t bad = 0;
+  for (uint32_t A = 1u << 23; A < 1u << 24; A++) {
+    const float a = ldexpf((float)A, exponent - 23);
+    bad += fmaf(a, y, a * yl) != a / b;
+  }
+  return bad;
+}

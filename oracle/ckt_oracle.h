@@ -20,7 +20,7 @@
  *                       reduction-instance fold/apply order of
  *                       runtime/lowlevel.h:475-492 (pieces applied ascending)
  *   ocl_uv_f32/_f64     apps/circuit/circuit.cc:445-460, :1290-1307
- *   ocl_split_quotient_check, ocl_wide_quotient_check
+ *   ocl_split_quotient_check, ocl_wide_quotient_check, ocl_split_divisor(_sweep)
  *                       the division by dt of apps/circuit/circuit.cc:391-393
  *                       as the GPU's EXACT mode forms it (split reciprocal),
  *                       against IEEE division, over ranges of dividends
@@ -165,6 +165,14 @@ void ocl_split_quotient_check(uint64_t lo, uint64_t hi, float dt, float zh, floa
  * dividend class (see the definition). */
 void ocl_wide_quotient_check(uint64_t seed, uint64_t n, int divisor, uint64_t *bad,
                              uint64_t *outside, uint64_t *drawn);
+
+/* The split quotient by b, fma(a, y, a * yl): sets y and yl and returns 1
+ * when it equals a / b for every dividend clear of underflow and overflow
+ * with y = RN(1/b), yl = RN(1/b - y), 2 when it does with yl one ulp off
+ * (as set), 0 when neither does.  b normal, 1/b and the parts normal. */
+int ocl_split_divisor(float b, float *y, float *yl);
+/* Mismatches of it among the 2^23 dividends of one binade. */
+uint64_t ocl_split_divisor_sweep(float b, float y, float yl, int exponent);
 
 #ifdef __cplusplus
 }

@@ -122,6 +122,10 @@ def lib():
         L.ocl_split_quotient_check.restype = None
         L.ocl_wide_quotient_check.argtypes = [u64, u64, i32, P, P, P]
         L.ocl_wide_quotient_check.restype = None
+        L.ocl_split_divisor.argtypes = [f32, P, P]
+        L.ocl_split_divisor.restype = i32
+        L.ocl_split_divisor_sweep.argtypes = [f32, f32, f32, i32]
+        L.ocl_split_divisor_sweep.restype = u64
         _lib = L
     return _lib
 
@@ -393,3 +397,14 @@ def wide_quotient_check(seed: int, n: int, divisor: int):
     lib().ocl_wide_quotient_check(seed, n, divisor, ctypes.byref(bad), ctypes.byref(out),
                                   ctypes.byref(drawn))
     return bad.value, out.value, drawn.value
+
+
+def split_divisor(b: float):
+    """(verdict, y, yl) of the split quotient by b; see ocl_split_divisor."""
+    y, yl = ctypes.c_float(), ctypes.c_float()
+    v = lib().ocl_split_divisor(b, ctypes.byref(y), ctypes.byref(yl))
+    return v, y.value, yl.value
+
+
+def split_divisor_sweep(b: float, y: float, yl: float, exponent: int) -> int:
+    return lib().ocl_split_divisor_sweep(b, y, yl, exponent)
