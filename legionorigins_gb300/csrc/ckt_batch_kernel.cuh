@@ -166,6 +166,24 @@ __device__ __forceinline__ void dc_contrib_block(const RoundCircuit &rc, uint32_
   }
 }
 
+// A CNC tile of a circuit with few steps (EXACT), out of line for the sake of
+// the other tiles' registers.
+template <int MODE>
+__device__ __noinline__ float4 few_steps_pair(int64_t wa, int64_t wb, bool has_b,
+                                              const WireArrays a, const NodeVolts v, int steps,
+                                              float dt) {
+  float2 i0, i9;
+  cnc_wire_pair<MODE, CKT_INIT_KERNEL, 0>(wa, wb, has_b, a, v, steps, dt, nullptr, &i0, &i9);
+  return make_float4(i0.x, i0.y, i9.x, i9.y);
+}
+template <int MODE>
+__device__ __noinline__ float2 few_steps(int64_t w, const WireArrays a, const NodeVolts v,
+                                         int steps, float dt) {
+  float i0, i9;
+  cnc_wire<MODE, CKT_INIT_KERNEL, 0>(w, a, v, steps, dt, nullptr, &i0, &i9);
+  return make_float2(i0, i9);
+}
+
 // DCS: 0 = staged block gather, 1 = one thread per node, 2 = contributions
 // scattered by the CNC tiles then summed contiguously.
 // Tiles of two wires per thread run both wires in one paired stepper
@@ -220,10 +238,17 @@ __global__ void __launch_bounds__(BLOCK,
           const bool has_b = tb < item.count;
           const uint32_t w = item.begin + ta, wb = item.begin + (has_b ? tb : ta);
           float2 i0, i9;
-          cnc_wire_pair<MODE, CKT_INIT_KERNEL, (int)BLOCK>(
-              (int64_t)w, (int64_t)wb, has_b, wa, volts, rc.steps, dt,
-              reinterpret_cast<float2 *>(sbuf) + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0), &i0,
-              &i9);
+          if (MODE == CKT_MODE_EXACT && rc.steps < kFreeSteps) {
+            const float4 r = few_steps_pair<MODE>((int64_t)w, (int64_t)wb, has_b, wa, volts,
+                                                  rc.steps, dt);
+            i0 = make_float2(r.x, r.y);
+            i9 = make_float2(r.z, r.w);
+          } else {
+            cnc_wire_pair<MODE, CKT_INIT_KERNEL, MODE == CKT_MODE_EXACT ? (int)BLOCK : 0>(
+                (int64_t)w, (int64_t)wb, has_b, wa, volts, rc.steps, dt,
+                reinterpret_cast<float2 *>(sbuf) + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0),
+                &i0, &i9);
+          }
           if (DCS == 2) {
             rc.contrib[rc.slot_in[w]] = __fmul_rn(-dt, i0.x);
             rc.contrib[rc.slot_out[w]] = __fmul_rn(dt, i9.x);
@@ -240,9 +265,15 @@ __global__ void __launch_bounds__(BLOCK,
           if (t < item.count) {
             const uint32_t w = item.begin + t;
             float i0, i9;
-            cnc_wire<MODE, CKT_INIT_KERNEL, (int)BLOCK>(
-                (int64_t)w, wa, volts, rc.steps, dt,
-                sbuf + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0), &i0, &i9);
+            if (MODE == CKT_MODE_EXACT && rc.steps < kFreeSteps) {
+              const float2 r = few_steps<MODE>((int64_t)w, wa, volts, rc.steps, dt);
+              i0 = r.x;
+              i9 = r.y;
+            } else {
+              cnc_wire<MODE, CKT_INIT_KERNEL, MODE == CKT_MODE_EXACT ? (int)BLOCK : 0>(
+                  (int64_t)w, wa, volts, rc.steps, dt,
+                  sbuf + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0), &i0, &i9);
+            }
             if (DCS == 2) {
               rc.contrib[rc.slot_in[w]] = __fmul_rn(-dt, i0);
               rc.contrib[rc.slot_out[w]] = __fmul_rn(dt, i9);

@@ -195,7 +195,6 @@ __device__ __forceinline__ uint32_t nan_bits(float2 a) {
 // split reciprocal (2 operations); otherwise they are corrected quotients too.
 template <bool DTF>
 struct DualExact {
-  static constexpr bool kFree = DTF;  // has free steps (exact_steps)
   float2 L, dt2, neg1;
   Recip2 kR, kC, kdt;
   float dt;
@@ -455,9 +454,12 @@ constexpr int kFirstRun = 8, kMostRun = 32;  // steps of a free block
 // Values per thread in shared memory: the state at a block's start (10
 // currents, 9 voltages), the two node voltages and yl of R and C.
 constexpr int kSavedState = 23;
-// Checking the divisors costs about as much as 5 steps; below this many steps
-// the loop runs guarded.
-constexpr int kFreeSteps = 16;
+// Launches of fewer steps run guarded throughout: checking the divisors costs
+// about as much as 5 steps, the blocks that fail from the generated state
+// (zeros, overflow) 20.  1,000,000 wires: 16 steps 104 us guarded, 102 us free
+// from finite values, 107 and 208 us from the generated state; 32 steps 192
+// and 153, 164 and 143 us.
+constexpr int kFreeSteps = 32;
 
 template <int STRIDE, typename F>
 __device__ __forceinline__ void save_state(F *save, const F (&ni)[10], const F (&nv)[11]) {
@@ -482,13 +484,13 @@ template <int STRIDE, typename Stepper, typename Wires, typename F>
 __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&ni)[10],
                                             F (&nv)[11], F *save) {
   const uint32_t lanes = __activemask();
-  uint32_t split = 0;
-  bool sound = false;
+  uint32_t split;
+  bool sound;
   int j = 0, run = kFirstRun, guarded = 0, penalty = 1;
   save_state<STRIDE>(save, ni, nv);
   save[19 * STRIDE] = nv[0];
   save[20 * STRIDE] = nv[10];
-  if (Stepper::kFree && steps >= kFreeSteps) {
+  {
     Stepper pk = wires.template stepper<Stepper>();
     const uint32_t checked = pk.check();
     split = (__all_sync(lanes, checked & 1u) ? 1u : 0u) | (__all_sync(lanes, checked & 2u) ? 2u : 0u);
@@ -497,8 +499,6 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
     sound = __all_sync(lanes, pk.sound(nI0, V0));
     save[21 * STRIDE] = pk.kR.yl;
     save[22 * STRIDE] = pk.kC.yl;
-  } else {
-    guarded = steps;  // no free block
   }
 #pragma unroll 1
   while (j < steps) {
@@ -507,7 +507,7 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
     // the switch only when every thread of the warp can take it, so that a
     // warp never runs the two loops one after the other
     if (__all_sync(lanes, nan == Stepper::kWires)) break;
-    if (Stepper::kFree && guarded == 0) {
+    if (guarded == 0) {
       bool right = true;
       if (sound) {
         Stepper pk = wires.template stepper<Stepper>();
@@ -584,11 +584,29 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
   }
 }
 
+// The same loop with guarded steps only: few steps, or a general dt.
+template <typename Stepper, typename F>
+__device__ __forceinline__ void exact_steps_guarded(const Stepper &pk, int steps, F (&ni)[10],
+                                                    F (&nv)[11], const F (&nI0)[10],
+                                                    const F (&V0)[9]) {
+  const uint32_t lanes = __activemask();
+  int j = 0;
+#pragma unroll 1
+  while (j < steps) {
+    if (__all_sync(lanes, Stepper::all_nan(ni, nv) == Stepper::kWires)) break;
+    const int n = min(kGuardedRun, steps - j);
+#pragma unroll 1
+    for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
+    j += n;
+  }
+#pragma unroll 1
+  for (; j < steps; j++) pk.step_all_nan(ni, nv, nI0, V0);
+}
+
 // EXACT, one wire per thread: DualExact's arithmetic and guards on scalar
 // instructions (the batched kernel's one-wire tiles).  Bit-identical to it.
 template <bool DTF>
 struct SoloExact {
-  static constexpr bool kFree = DTF;
   float L, dt;
   Recip kR, kC, kdt;
   __device__ __forceinline__ SoloExact(float l, float r, float c, float d) {
@@ -854,9 +872,9 @@ struct DualWires : WireSource {
 };
 
 // One wire's whole inner loop: load, S steps in registers, store.
-// save: this thread's column of kSavedState rows of STRIDE floats in shared
-// memory (EXACT).
-template <int MODE, int INIT, int STRIDE = 1>
+// EXACT: save is this thread's column of kSavedState rows of STRIDE floats in
+// shared memory, and dt (float)1e-6; STRIDE 0: guarded steps, any dt.
+template <int MODE, int INIT, int STRIDE = 0>
 __device__ __forceinline__ void cnc_wire(int64_t w, const WireArrays &a, const NodeVolts &nv_in,
                                          int steps, float dt, float *save = nullptr,
                                          float *i0_out = nullptr, float *i9_out = nullptr) {
@@ -933,14 +951,19 @@ __device__ __forceinline__ void cnc_wire(int64_t w, const WireArrays &a, const N
 #pragma unroll
       for (int k = 0; k < 10; k++) ni[k] = d[k];
     }
-  } else if (MODE == CKT_MODE_EXACT && __float_as_uint(dt) == kDtBits &&
+  } else if (MODE == CKT_MODE_EXACT && (STRIDE || __float_as_uint(dt) == kDtBits) &&
              SoloExact<true>::eligible(a.R[w], a.C[w], dt)) {
-    const SoloWire ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, w};
-    exact_steps<STRIDE, SoloExact<true>>(ws, steps, ni, nv, save);
-  } else if (MODE == CKT_MODE_EXACT && __float_as_uint(dt) != kDtBits &&
+    if constexpr (STRIDE > 0) {
+      const SoloWire ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, w};
+      exact_steps<STRIDE, SoloExact<true>>(ws, steps, ni, nv, save);
+    } else {
+      const SoloExact<true> ws(a.L[w], a.R[w], a.C[w], dt);
+      exact_steps_guarded(ws, steps, ni, nv, I0, V0);
+    }
+  } else if (MODE == CKT_MODE_EXACT && !STRIDE && __float_as_uint(dt) != kDtBits &&
              SoloExact<false>::eligible(a.R[w], a.C[w], dt)) {
-    const SoloWire ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, w};
-    exact_steps<STRIDE, SoloExact<false>>(ws, steps, ni, nv, save);
+    const SoloExact<false> ws(a.L[w], a.R[w], a.C[w], dt);
+    exact_steps_guarded(ws, steps, ni, nv, I0, V0);
   } else {
     static_assert(MODE == CKT_MODE_EXACT || MODE == CKT_MODE_EXACT_DIVIDE, "unknown mode");
     const DivideStep ws(a.L[w], a.R[w], a.C[w], dt);
@@ -962,11 +985,10 @@ __device__ __forceinline__ void cnc_wire(int64_t w, const WireArrays &a, const N
 }
 
 // Two wires per thread (FAST: DualFast, EXACT: DualExact): thread t of a
-// block handles wires base + t and base + t + 256, so each field's loads and
-// stores stay one contiguous line per warp.  Without a partner wire the
+// block handles wires base + t and base + t + block size, so each field's
+// loads and stores stay one contiguous line per warp.  Without a partner wire the
 // thread runs its wire in both lanes and stores one.
-// save: this thread's column of kSavedState rows of STRIDE float2 in shared
-// memory (EXACT).
+// save, STRIDE: as cnc_wire's, of float2.
 template <int MODE, int INIT, int STRIDE>
 __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b,
                                               const WireArrays &a, const NodeVolts &nvin,
@@ -977,7 +999,7 @@ __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b
   const int64_t S = a.S;
   const float2 L2 = make_float2(a.L[wa], a.L[wb]), R2 = make_float2(a.R[wa], a.R[wb]),
                C2 = make_float2(a.C[wa], a.C[wb]);
-  const bool dt_fixed = __float_as_uint(dt) == kDtBits;
+  const bool dt_fixed = STRIDE || __float_as_uint(dt) == kDtBits;
   if (MODE == CKT_MODE_EXACT &&
       !(dt_fixed ? DualExact<true>::eligible(R2, C2, dt) : DualExact<false>::eligible(R2, C2, dt))) {
     // a divisor outside the corrected quotients' range: the divide routine
@@ -1029,12 +1051,15 @@ __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b
 #pragma unroll
       for (int k = 0; k < 10; k++) ni[k] = make_float2(-nI0[k].x, -nI0[k].y);  // no step: I0
     }
-  } else if (dt_fixed) {
+  } else if constexpr (STRIDE > 0) {
     const DualWires ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, wa, wb};
     exact_steps<STRIDE, DualExact<true>>(ws, steps, ni, nv, save);
+  } else if (dt_fixed) {
+    const DualExact<true> pk(L2, R2, C2, dt);
+    exact_steps_guarded(pk, steps, ni, nv, nI0, V0);
   } else {
-    const DualWires ws = {{a.L, a.R, a.C, a.cur, a.vol, S, dt}, wa, wb};
-    exact_steps<STRIDE, DualExact<false>>(ws, steps, ni, nv, save);
+    const DualExact<false> pk(L2, R2, C2, dt);
+    exact_steps_guarded(pk, steps, ni, nv, nI0, V0);
   }
 #pragma unroll
   for (int k = 0; k < 10; k++) a.cur[k * S + wa] = ni[k].x;
@@ -1050,32 +1075,236 @@ __device__ __forceinline__ void cnc_wire_pair(int64_t wa, int64_t wb, bool has_b
   if (i9_out) *i9_out = ni[9];
 }
 
-constexpr int kPairBlock = 256;  // threads; a block covers 2 * kPairBlock wires
-
-template <int MODE, int INIT>
-__global__ void __launch_bounds__(kPairBlock, 2)
+// A block of BLOCK threads covers 2 * BLOCK wires.  FREE (EXACT): at least
+// kFreeSteps steps of (float)1e-6.
+template <int MODE, int INIT, bool FREE, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
     cnc_pair_kernel(uint32_t first_wire, uint32_t num_wires, WireArrays a, NodeVolts v, int steps,
                     float dt) {
-  __shared__ float2 save[MODE == CKT_MODE_EXACT ? kSavedState * kPairBlock : 1];
-  const uint32_t ta = blockIdx.x * (2 * kPairBlock) + threadIdx.x, tb = ta + kPairBlock;
+  __shared__ float2 save[FREE ? kSavedState * BLOCK : 1];
+  const uint32_t ta = blockIdx.x * (2 * BLOCK) + threadIdx.x, tb = ta + BLOCK;
   if (ta >= num_wires) return;
   const bool has_b = tb < num_wires;
-  cnc_wire_pair<MODE, INIT, kPairBlock>((int64_t)first_wire + ta,
-                                        (int64_t)first_wire + (has_b ? tb : ta), has_b, a, v,
-                                        steps, dt,
-                                        save + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0));
+  cnc_wire_pair<MODE, INIT, FREE ? BLOCK : 0>(
+      (int64_t)first_wire + ta, (int64_t)first_wire + (has_b ? tb : ta), has_b, a, v, steps, dt,
+      save + (FREE ? threadIdx.x : 0));
 }
 
-template <int MODE, int INIT>
+// FREE: as above, in one-warp blocks.
+template <int MODE, int INIT, bool FREE>
 __global__ void __launch_bounds__(256)
     cnc_kernel(uint32_t first_wire, uint32_t num_wires, WireArrays a, NodeVolts v, int steps,
                float dt) {
-  // EXACT launches have one-warp blocks
-  __shared__ float save[MODE == CKT_MODE_EXACT ? kSavedState * 32 : 1];
+  __shared__ float save[FREE ? kSavedState * 32 : 1];
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= num_wires) return;
-  cnc_wire<MODE, INIT, 32>((int64_t)first_wire + t, a, v, steps, dt,
-                           save + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0));
+  cnc_wire<MODE, INIT, FREE ? 32 : 0>((int64_t)first_wire + t, a, v, steps, dt,
+                                      save + (FREE ? threadIdx.x : 0));
+}
+
+// ---------------------------------------------------------------------------
+// calc_new_currents, EXACT, small launches: five lanes per wire.  Lane g of a
+// wire holds segments 2g and 2g+1 -- their currents and the voltages v_2g,
+// v_2g+1, v_2g+2 around them, the outer two of which its neighbours compute
+// too, so that one exchange of currents per step (two shuffles, in flight
+// together) is all the lanes tell each other.  A warp takes six wires; lanes
+// 30 and 31 idle.
+//
+// Why: with about one warp per scheduler a step takes as long as that warp
+// needs to issue it and its chain of dependent operations.  One wire per
+// thread issues 125 operations one after another; here 13 paired ones and 5
+// single ones, and the chain of 13 operations and a shuffle shows.
+//
+// The arithmetic, the blocks of free steps and their checks are
+// exact_steps'; the rollback state stays in registers.
+// ---------------------------------------------------------------------------
+constexpr int kLanesPerWire = 5;
+constexpr uint32_t kLaneWires = 6;  // per warp
+
+// What a lane carries from step to step.  The signs let every difference of
+// a free step be a paired addition; negation is exact.
+struct LaneState {
+  float2 x;  // -i_2g, i_2g+1
+  float2 e;  // v_2g, v_2g+2
+  float nb;  // -v_2g+1
+};
+
+// RN(a / b) for every dividend and divisor: the corrected quotient where it
+// is right, the divide routine elsewhere.
+__device__ __forceinline__ float any_quot(float a, const Recip &k, bool eligible, float lo,
+                                          float hi) {
+  return eligible && !outside(a, lo, hi) ? recip_quot(a, k) : div_rn(a, -k.nb);
+}
+
+struct LaneWire {
+  Recip2 R, E;  // R twice; C of v_2g and v_2g+2, 1 / infinity where the wire ends there
+  Recip C;
+  float L, dt;
+  float2 nX0, Ve;  // starting currents I_2g, -I_2g+1; starting voltages of v_2g, v_2g+2
+  float nVb;       // minus that of v_2g+1
+  int left, right;  // lanes of the neighbours (the lane itself at the wire's ends)
+  bool first, last, okR, okC;  // okR, okC: eligible divisors (divisor_ok)
+
+  // SPLIT, LOW: as DualExact::step_free.  The voltages at the wire's ends
+  // stay: V + a * 0.
+  template <uint32_t SPLIT, bool LOW>
+  __device__ __forceinline__ void step_free(LaneState &s, float &low) const {
+    const float2 neg1 = make_float2(-1.0f, -1.0f);
+    const float2 a1 = __fmul2_rn(make_float2(L, L), __fadd2_rn(s.x, nX0));
+    const float2 a2 =
+        __ffma2_rn(dt_quot2(a1), neg1, __fadd2_rn(s.e, make_float2(s.nb, s.nb)));
+    s.x = SPLIT & 1u ? split_quot2(a2, R) : recip_quot2(a2, R);
+    const float l = __shfl_sync(0xffffffffu, s.x.y, left);
+    const float r = __shfl_sync(0xffffffffu, s.x.x, right);
+    const float a3 = __fmul_rn(dt, __fadd_rn(s.x.x, s.x.y));
+    s.nb = __fadd_rn(nVb, SPLIT & 2u ? split_quot(a3, C) : recip_quot(a3, C));
+    const float2 ae = __fmul2_rn(make_float2(dt, dt), __fadd2_rn(make_float2(l, r), s.x));
+    s.e = __fadd2_rn(Ve, SPLIT & 2u ? split_quot2(ae, E) : recip_quot2(ae, E));
+    if (LOW) {
+      low = min_abs(low, a2.x, a2.y);
+      low = min_abs(low, a3, first ? 1.0f : ae.x);
+      low = fminf(low, last ? 1.0f : fabsf(ae.y));
+    }
+  }
+  // The reference's step for every state and divisor.
+  __device__ __forceinline__ float dt_div(float a) const {
+    return tiny_nonzero(a, kDtTiny) ? __fdiv_rn(a, dt) : dt_quot(a);
+  }
+  __device__ __forceinline__ void step(LaneState &s) const {
+    const Recip r = {R.nb.x, R.y.x, R.yl.x};
+    const float va = s.e.x, vb = -s.nb, vc = s.e.y;
+    const float q0 = dt_div(__fmul_rn(L, __fsub_rn(-s.x.x, nX0.x)));
+    const float q1 = dt_div(__fmul_rn(L, __fsub_rn(s.x.y, -nX0.y)));
+    const float i0 = any_quot(__fsub_rn(__fsub_rn(vb, va), q0), r, okR, kRLo, kRHi);
+    const float i1 = any_quot(__fsub_rn(__fsub_rn(vc, vb), q1), r, okR, kRLo, kRHi);
+    const float l = __shfl_sync(0xffffffffu, i1, left), n = __shfl_sync(0xffffffffu, i0, right);
+    const float da = __fmul_rn(dt, __fsub_rn(l, i0)), dc = __fmul_rn(dt, __fsub_rn(i1, n));
+    const float db = __fmul_rn(dt, __fsub_rn(i0, i1));
+    s.x = make_float2(-i0, i1);
+    s.nb = -__fadd_rn(-nVb, any_quot(db, C, okC, kCLo, kCHi));
+    if (!first) s.e.x = __fadd_rn(Ve.x, any_quot(da, C, okC, kCLo, kCHi));
+    if (!last) s.e.y = __fadd_rn(Ve.y, any_quot(dc, C, okC, kCLo, kCHi));
+  }
+  template <uint32_t SPLIT, bool LOW>
+  __device__ __forceinline__ void steps_free(LaneState &s, int n, float &low) const {
+#pragma unroll 4
+    for (int i = 0; i < n; i++) step_free<SPLIT, LOW>(s, low);
+  }
+};
+
+template <int INIT>
+__global__ void __launch_bounds__(32)
+    cnc_lanes_kernel(uint32_t first_wire, uint32_t num_wires, WireArrays a, NodeVolts v, int steps,
+                     float dt) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x, g = lane % kLanesPerWire, slot = lane / kLanesPerWire;
+  const uint32_t t = blockIdx.x * kLaneWires + slot;
+  // lanes without a wire of their own run along on another
+  const bool mine = slot < kLaneWires && t < num_wires;
+  const int64_t w = (int64_t)first_wire + min(t, num_wires - 1u), S = a.S;
+  const uint32_t wire_lanes = 0x1fu << (slot * kLanesPerWire);
+
+  auto start_voltage = [&](uint32_t k) -> float {  // v_k before the first step
+    if (k == 10) return pick_instance(a.out_loc[w], v.pvt, v.shr, v.ghost)[a.out_ptr[w]];
+    if (INIT == CKT_INIT_CPU_TASK) return k < 9 ? a.vol[k * S + w] : 0.0f;
+    return k ? a.vol[(k - 1) * S + w]
+             : pick_instance(a.in_loc[w], v.pvt, v.shr, v.ghost)[a.in_ptr[w]];
+  };
+  const float r = a.R[w], c = a.C[w];
+  const float I0 = a.cur[2 * g * S + w], I1 = a.cur[(2 * g + 1) * S + w];
+  LaneState s = {make_float2(-I0, I1), make_float2(start_voltage(2 * g), start_voltage(2 * g + 2)),
+                 -start_voltage(2 * g + 1)};
+  LaneWire x;
+  x.R = make_recip2(r, r);
+  x.C = make_recip(c);
+  x.L = a.L[w];
+  x.dt = dt;
+  x.nX0 = make_float2(I0, -I1);
+  x.first = g == 0;
+  x.last = g == kLanesPerWire - 1;
+  x.Ve = make_float2(x.first ? s.e.x : a.vol[(2 * g - 1) * S + w],
+                     x.last ? s.e.y : a.vol[(2 * g + 1) * S + w]);
+  x.nVb = -a.vol[2 * g * S + w];
+  x.left = (int)lane - (x.first ? 0 : 1);
+  x.right = (int)lane + (x.last || lane == 31u ? 0 : 1);
+  x.okR = divisor_ok(r, kRMin, kRMax);
+  x.okC = divisor_ok(c, kCMin, kCMax);
+
+  int guarded = __all_sync(kAll, x.okR && x.okC) ? 0 : steps;
+  uint32_t split = 0;
+  bool sound = false;
+  if (guarded == 0) {
+    const float nb[2] = {x.R.nb.x, x.C.nb}, y[2] = {x.R.y.x, x.C.y};
+    float yl[2] = {x.R.yl.x, x.C.yl};
+    const uint32_t checked = check_split(nb, y, yl);
+    x.R.yl = make_float2(yl[0], yl[0]);
+    x.C.yl = yl[1];
+    split = (__all_sync(kAll, checked & 1u) ? 1u : 0u) | (__all_sync(kAll, checked & 2u) ? 2u : 0u);
+    sound = __all_sync(kAll, sound_wire(fminf(fabsf(I0), fabsf(I1)),
+                                        min_abs(fabsf(x.nVb), x.first ? 1.0f : x.Ve.x,
+                                                x.last ? 1.0f : x.Ve.y),
+                                        x.L, c, dt));
+  }
+  x.E.nb = make_float2(x.C.nb, x.C.nb);
+  x.E.y = make_float2(x.first ? 0.0f : x.C.y, x.last ? 0.0f : x.C.y);
+  x.E.yl = make_float2(x.first ? 0.0f : x.C.yl, x.last ? 0.0f : x.C.yl);
+
+  int j = 0, run = kFirstRun, penalty = 1;
+#pragma unroll 1
+  while (j < steps) {
+    // which lanes' state is all NaN (each answers for what it computes)
+    const uint32_t nan = __ballot_sync(
+        kAll, (s.x.x != s.x.x && s.x.y != s.x.y && s.nb != s.nb && (x.first || s.e.x != s.e.x) &&
+               (x.last || s.e.y != s.e.y)) ||
+                  !mine);
+    float low = __int_as_float(0x7f800000);
+    if (nan == kAll) {  // stays so: any form of quotient gives NaN, nothing to check
+      x.steps_free<3, false>(s, steps - j, low);
+      break;
+    }
+    if (guarded == 0) {
+      const LaneState start = s;
+      const int n = min(run, steps - j);
+      bool right = true;
+      if (sound) {
+        if (split == 3u) x.steps_free<3, false>(s, n, low);
+        else if (split == 2u) x.steps_free<2, false>(s, n, low);
+        else if (split == 1u) x.steps_free<1, false>(s, n, low);
+        else x.steps_free<0, false>(s, n, low);
+        if (j + n == steps) right = fminf(fabsf(s.x.x), fabsf(s.x.y)) >= 0x1p-75f;
+      } else if (split == 3u) {
+        x.steps_free<3, true>(s, n, low);
+        right = low >= kSplitLo;
+      } else {
+        x.steps_free<0, true>(s, n, low);
+        right = low >= kCLo;
+      }
+      const float sum = __fadd_rn(__fadd_rn(s.x.x, s.x.y), __fadd_rn(__fadd_rn(s.e.x, s.e.y), s.nb));
+      right &= sum == sum;
+      right |= !mine || (nan & wire_lanes) == wire_lanes;
+      if (__all_sync(kAll, right)) {
+        j += n;
+        if (run == kMostRun) penalty = 1;
+        run = min(2 * run, kMostRun);
+        continue;
+      }
+      s = start;
+      run = kFirstRun;
+      guarded = penalty;
+      penalty = min(2 * penalty, 8);
+    }
+    const int n = min(kGuardedRun, steps - j);
+#pragma unroll 1
+    for (int i = 0; i < n; i++) x.step(s);
+    j += n;
+    guarded--;
+  }
+  if (mine) {
+    a.cur[2 * g * S + w] = -s.x.x;
+    a.cur[(2 * g + 1) * S + w] = s.x.y;
+    a.vol[2 * g * S + w] = -s.nb;
+    if (!x.last) a.vol[(2 * g + 1) * S + w] = s.e.y;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -77,20 +77,52 @@ static void launch_cnc_t(uint32_t first, uint32_t n, const ckt_wires &w, const f
                          const float *vs, const float *vg, const ckt_params *p, cudaStream_t s) {
   const WireArrays a = wire_arrays(w);
   const NodeVolts v = {vp, vs, vg};
-  // EXACT with at most three warps per SM scheduler: one wire per thread in
-  // one-warp blocks, spread over every SM, runs each step several times
-  // faster than the paired kernel on the few SMs its blocks would occupy
-  // (same bits: the scalar and paired steppers round every operation alike).
-  const int sms = M == CKT_MODE_EXACT ? device_sms() : 0;
-  if (M == CKT_MODE_EXACT && sms > 0 && n <= 384u * (uint32_t)sms) {
-    cnc_kernel<M, I><<<grid_for(n, 32), 32, 0, s>>>(first, n, a, v, p->steps, p->dt);
+  // The paired kernel fills the GPU best, but its blocks leave SMs idle or
+  // unevenly filled when there are few, and a step then takes as long as its
+  // slowest warp.  Same bits in every form (each rounds every operation
+  // alike).  us per 1000 steps on a GB300, finite values:
+  //   EXACT  wires       1024  4096  8000  16000  64000  124867  200000  300000
+  //     five lanes/wire    63    76    95    139
+  //     one thread/wire    92   110   112    111    315     518     789    1136
+  //     paired, 128       207   207   209    206    391     628     874    1157
+  //   FAST   wires            4096  16000  48000  64000  160000  500000  4194304
+  //     one thread/wire         47     48    105    135     276     760
+  //     paired, 128             72     72    126    127     287     715     5525
+  //     paired, 256            123    123    125    125     339     763     5510
+  const uint32_t sms = (uint32_t)device_sms();
+  uint32_t dt_bits;
+  memcpy(&dt_bits, &p->dt, sizeof(dt_bits));
+  if constexpr (M == CKT_MODE_EXACT) {
+    if (dt_bits == kDtBits && p->steps >= kFreeSteps) {
+      if (n <= 48u * sms)  // at most two warps per scheduler
+        cnc_lanes_kernel<I><<<grid_for(n, kLaneWires), 32, 0, s>>>(first, n, a, v, p->steps,
+                                                                  p->dt);
+      else if (n <= 1440u * sms)
+        cnc_kernel<M, I, true><<<grid_for(n, 32), 32, 0, s>>>(first, n, a, v, p->steps, p->dt);
+      else
+        cnc_pair_kernel<M, I, true, 128><<<grid_for(n, 256), 128, 0, s>>>(first, n, a, v, p->steps,
+                                                                         p->dt);
+      return;
+    }
+  }
+  // EXACT here: few steps or another dt, guarded steps only, for which 384
+  // wires per SM is the line
+  if ((M == CKT_MODE_EXACT && n <= 384u * sms) || (M == CKT_MODE_FAST && n <= 320u * sms)) {
+    cnc_kernel<M, I, false><<<grid_for(n, 32), 32, 0, s>>>(first, n, a, v, p->steps, p->dt);
     return;
   }
+  if constexpr (M == CKT_MODE_FAST) {
+    if (n > 512u * sms && n <= 4096u * sms) {  // (up to one 256-thread block per SM is even)
+      cnc_pair_kernel<M, I, false, 128><<<grid_for(n, 256), 128, 0, s>>>(first, n, a, v, p->steps,
+                                                                        p->dt);
+      return;
+    }
+  }
   if constexpr (M == CKT_MODE_FAST || M == CKT_MODE_EXACT)  // two wires per thread, paired
-    cnc_pair_kernel<M, I><<<grid_for(n, 2 * kPairBlock), kPairBlock, 0, s>>>(first, n, a, v,
-                                                                             p->steps, p->dt);
+    cnc_pair_kernel<M, I, false, 256><<<grid_for(n, 512), 256, 0, s>>>(first, n, a, v, p->steps,
+                                                                      p->dt);
   else
-    cnc_kernel<M, I><<<grid_for(n), 256, 0, s>>>(first, n, a, v, p->steps, p->dt);
+    cnc_kernel<M, I, false><<<grid_for(n), 256, 0, s>>>(first, n, a, v, p->steps, p->dt);
 }
 
 int launch_cnc(uint32_t first, uint32_t n, const ckt_wires &w, const float *vp,
