@@ -171,6 +171,14 @@ __device__ __forceinline__ bool sound_wire(float i, float v, float L, float C, f
   return (i >= 0x1p-50f) & (v >= 0x1p-50f) & (fabsf(L) >= 0x1p-43f) & (fabsf(C) >= 0x1p-20f) &
          (__fmul_rn(v, fabsf(C)) >= __fmul_rn(0x1p-22f, dt));
 }
+// Orders magnitudes as integers, with zero above everything: finite values
+// by magnitude, then infinity (kOrderInf), NaN, zero.
+__device__ __forceinline__ uint32_t order(float a) { return 2u * __float_as_uint(a) - 1u; }
+constexpr uint32_t kOrderInf = 0xfeffffffu;
+// The same loop constants for the wide steps; i: the least order(I0).
+__device__ __forceinline__ bool wide_wire(uint32_t i, float L, float C) {
+  return (i >= order(0x1p-50f)) & (fabsf(L) >= 0x1p-43f) & (fabsf(C) >= 0x1p-20f);
+}
 // Which wires' values are NaN: bit 0 the first (or only) wire, bit 1 the second.
 __device__ __forceinline__ uint32_t nan_bits(float a) { return a != a ? 1u : 0u; }
 __device__ __forceinline__ uint32_t nan_bits(float2 a) {
@@ -339,6 +347,43 @@ struct DualExact {
       nv[k + 1] = __fadd2_rn(V0[k], SPLIT & 2u ? split_quot2(a3, kC) : recip_quot2(a3, kC));
     }
   }
+  // The same with every zero and infinite dividend's quotient as well: a * y.
+  // lowR, lowC collect the least order of the nonzero dividends.
+  static __device__ __forceinline__ float2 wide(float2 a, const Recip2 &k, uint32_t &low) {
+    const uint32_t tx = order(a.x), ty = order(a.y);
+    const float2 q = split_quot2(a, k), z = __fmul2_rn(a, k.y);
+    low = min(low, min(tx, ty));
+    return make_float2(tx >= kOrderInf ? z.x : q.x, ty >= kOrderInf ? z.y : q.y);
+  }
+  __device__ __forceinline__ void step_wide(float2 (&ni)[10], float2 (&nv)[11],
+                                            const float2 (&nI0)[10], const float2 (&V0)[9],
+                                            uint32_t &lowR, uint32_t &lowC) const {
+#pragma unroll
+    for (int k = 0; k < 10; k++) {
+      const float2 a1 = __fmul2_rn(L, __fadd2_rn(ni[k], nI0[k]));
+      ni[k] = wide(__ffma2_rn(dt_div(a1), neg1, __ffma2_rn(nv[k], neg1, nv[k + 1])), kR, lowR);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      nv[k + 1] = __fadd2_rn(
+          V0[k], wide(__fmul2_rn(dt2, __ffma2_rn(ni[k + 1], neg1, ni[k])), kC, lowC));
+  }
+  __device__ __forceinline__ bool can_wide(const float2 (&nI0)[10]) const {
+    uint32_t x = ~0u, y = ~0u;
+#pragma unroll
+    for (int k = 0; k < 10; k++) {
+      x = min(x, order(nI0[k].x));
+      y = min(y, order(nI0[k].y));
+    }
+    return wide_wire(x, L.x, kC.nb.x) & wide_wire(y, L.y, kC.nb.y);
+  }
+  static __device__ __forceinline__ uint32_t least_order(const float2 (&ni)[10]) {
+    uint32_t m = ~0u;
+#pragma unroll
+    for (int k = 0; k < 10; k++) m = min(m, min(order(ni[k].x), order(ni[k].y)));
+    return m;
+  }
+  __device__ __forceinline__ float most_C() const { return fmaxf(fabsf(kC.nb.x), fabsf(kC.nb.y)); }
   // The loop's constants keep every dividend's tininess from mattering
   // (exact_steps).
   __device__ __forceinline__ bool sound(const float2 (&nI0)[10], const float2 (&V0)[9]) const {
@@ -436,20 +481,35 @@ struct DualExact {
 //      - a1 / dt is right: i - I0 is 0 or at least half an ulp of I0, 2^-75,
 //        so with |L| >= 2^-43 a1 is 0 or at least 2^-118 = kDtTiny.
 //    (With LOW a1 needs no check either, see dt_outside.)
-// A failed block costs its own steps once more: the first blocks are short,
-// and after a failure the next blocks run guarded, 1, 2, 4 and 8 of them as
-// failures repeat (a loop's first steps from zero currents, a blow-up, a
-// wire in equilibrium with zero differences).
+// Where the constants are not sound, or a block failed, the next blocks are
+// careful ones: wide steps, which also divide zeros and infinities rightly (a
+// times RN(1/b)) and collect the least nonzero dividends -- by C, at least
+// 2^-77 |C| wanted, by R, 2^-66, so that a nonzero current is at least 2^-74
+// and, I0 being 0 or at least 2^-50 (wide_wire) and so the currents at the
+// block's start, a1 is 0 or at least kDtTiny -- or LOW ones, where a divisor
+// is unchecked.  A careful block that fails is done again with step(), and
+// the next 1, 2, 4 and 8 blocks are guarded outright as failures repeat.
+//
+// A failed block costs its own steps once more, so the first blocks are short
+// and after a failure sound blocks pause for 1, 2, 4 and 8 careful ones.
 //
 // Why: the guards' 58 compares and two branches per paired step held the loop
 // at 75% of the FP32 pipe, and the corrected quotients are 76 of its 163
 // operations.  A free step has 125 operations and nothing else.  The 19
 // three-input minima of LOW are not free beside it: FMAs of three register
 // pairs keep the register ports busy.  1,048,576 wires, 1000 steps, GB300:
-// guarded 5.88 ms, free with LOW 4.64 ms, without 3.83 ms, all NaN 3.59 ms
+// guarded 5.88 ms, free with LOW 4.64 ms, without 3.75 ms, all NaN 3.49 ms
 // (4.80 ms with corrected quotients); the 125 operations at the pipe's full
-// rate take 3.25 ms.  124,867 wires: 1.10 -> 0.64 ms.
-constexpr int kGuardedRun = 16;  // steps of a guarded block
+// rate take 3.25 ms.  From the generated state (zeros, overflow, all NaN
+// after 26 steps) 5.13 ms guarded, 3.96 ms with its first 32 steps guarded,
+// 3.73 ms with 10 guarded and 16 wide ones.
+constexpr int kGuardedRun = 16;  // steps between looks for all NaN (guarded loop)
+constexpr int kCarefulRun = 16;  // steps of a careful block
+// From zero currents or voltages the first steps run guarded: what the node
+// voltages start reaches one segment further per step, falling to 2^-110 on
+// its way, below what the other forms divide rightly.
+constexpr int kFrontRun = 10;
+enum CarefulForm { kGuarded, kLow, kWide };
 constexpr int kFirstRun = 8, kMostRun = 32;  // steps of a free block
 // Values per thread in shared memory: the state at a block's start (10
 // currents, 9 voltages), the two node voltages and yl of R and C.
@@ -486,7 +546,10 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
   const uint32_t lanes = __activemask();
   uint32_t split;
   bool sound;
-  int j = 0, run = kFirstRun, guarded = 0, penalty = 1;
+  CarefulForm how;
+  // careful: blocks before the next try of sound ones; skip: careful blocks
+  // before the next that is not guarded outright
+  int j = 0, run = kFirstRun, careful = 0, penalty = 1, skip = 0, again = 1;
   save_state<STRIDE>(save, ni, nv);
   save[19 * STRIDE] = nv[0];
   save[20 * STRIDE] = nv[10];
@@ -497,6 +560,8 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
     F nI0[10], V0[9];
     wires.load(nI0, V0);
     sound = __all_sync(lanes, pk.sound(nI0, V0));
+    skip = sound ? 0 : 1;
+    how = split == 3u && __all_sync(lanes, pk.can_wide(nI0)) ? kWide : kLow;
     save[21 * STRIDE] = pk.kR.yl;
     save[22 * STRIDE] = pk.kC.yl;
   }
@@ -507,68 +572,63 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
     // the switch only when every thread of the warp can take it, so that a
     // warp never runs the two loops one after the other
     if (__all_sync(lanes, nan == Stepper::kWires)) break;
-    if (guarded == 0) {
-      bool right = true;
-      if (sound) {
-        Stepper pk = wires.template stepper<Stepper>();
-        pk.kR.yl = save[21 * STRIDE];
-        pk.kC.yl = save[22 * STRIDE];
-        F nI0[10], V0[9];
-        wires.load(nI0, V0);
-        nv[0] = save[19 * STRIDE];
-        nv[10] = save[20 * STRIDE];
-        bool all_nan = false;
-        float none = 0.0f;
+    if (sound && careful == 0) {
+      Stepper pk = wires.template stepper<Stepper>();
+      pk.kR.yl = save[21 * STRIDE];
+      pk.kC.yl = save[22 * STRIDE];
+      F nI0[10], V0[9];
+      wires.load(nI0, V0);
+      nv[0] = save[19 * STRIDE];
+      nv[10] = save[20 * STRIDE];
+      bool right = true, all_nan = false;
+      float none = 0.0f;
 #pragma unroll 1
-        while (!all_nan && j < steps) {
-          const int n = min(run, steps - j);
-          // one loop per pair of quotient forms: a warp with one unchecked
-          // divisor (8% of paired warps) keeps the other's split quotients
-          if (split == 3u) {
-#pragma unroll 1
-            for (int i = 0; i < n; i++) pk.template step_free<3, false>(ni, nv, nI0, V0, none);
-          } else if (split == 2u) {
-#pragma unroll 1
-            for (int i = 0; i < n; i++) pk.template step_free<2, false>(ni, nv, nI0, V0, none);
-          } else if (split == 1u) {
-#pragma unroll 1
-            for (int i = 0; i < n; i++) pk.template step_free<1, false>(ni, nv, nI0, V0, none);
-          } else {
-#pragma unroll 1
-            for (int i = 0; i < n; i++) pk.template step_free<0, false>(ni, nv, nI0, V0, none);
-          }
-          right = (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
-          if (j + n == steps) right &= Stepper::least_current(ni) >= 0x1p-75f;
-          right = __all_sync(lanes, right);
-          if (!right) break;
-          j += n;
-          if (run == kMostRun) penalty = 1;
-          run = min(2 * run, kMostRun);
-          save_state<STRIDE>(save, ni, nv);
-          nan = Stepper::all_nan(ni, nv);
-          all_nan = __all_sync(lanes, nan == Stepper::kWires);
-        }
-      } else {
+      while (!all_nan && j < steps) {
         const int n = min(run, steps - j);
-        right = wires.template low<Stepper, STRIDE>(n, split == 3u, nan, save);
-        right = __all_sync(lanes, right);
-        if (right) {
-          j += n;
-          if (run == kMostRun) penalty = 1;
-          run = min(2 * run, kMostRun);
+        // one loop per pair of quotient forms: a warp with one unchecked
+        // divisor (8% of paired warps) keeps the other's split quotients
+        if (split == 3u) {
+#pragma unroll 1
+          for (int i = 0; i < n; i++) pk.template step_free<3, false>(ni, nv, nI0, V0, none);
+        } else if (split == 2u) {
+#pragma unroll 1
+          for (int i = 0; i < n; i++) pk.template step_free<2, false>(ni, nv, nI0, V0, none);
+        } else if (split == 1u) {
+#pragma unroll 1
+          for (int i = 0; i < n; i++) pk.template step_free<1, false>(ni, nv, nI0, V0, none);
         } else {
-          save_state<STRIDE>(save, ni, nv);
+#pragma unroll 1
+          for (int i = 0; i < n; i++) pk.template step_free<0, false>(ni, nv, nI0, V0, none);
         }
+        right = (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
+        if (j + n == steps) right &= Stepper::least_current(ni) >= 0x1p-75f;
+        right = __all_sync(lanes, right);
+        if (!right) break;
+        j += n;
+        if (run == kMostRun) penalty = 1;
+        run = min(2 * run, kMostRun);
+        save_state<STRIDE>(save, ni, nv);
+        nan = Stepper::all_nan(ni, nv);
+        all_nan = __all_sync(lanes, nan == Stepper::kWires);
       }
       if (right) continue;
-      guarded = penalty;
+      careful = penalty;
       penalty = min(2 * penalty, 8);
       run = kFirstRun;
     }
-    const int n = min(kGuardedRun, steps - j);
-    wires.template guarded<Stepper, STRIDE>(n, save);
+    const int n = min(j == 0 ? kFrontRun : kCarefulRun, steps - j);
+    const bool right =
+        wires.template careful<Stepper, STRIDE>(n, skip ? kGuarded : how, nan, lanes, save);
+    if (skip) {
+      skip--;
+    } else if (right) {
+      again = 1;
+    } else {
+      skip = again;
+      again = min(2 * again, 8);
+    }
     j += n;
-    guarded--;
+    if (careful) careful--;
   }
   if (j < steps) {
     const Stepper pk = wires.template stepper<Stepper>();
@@ -716,6 +776,34 @@ struct SoloExact {
       if (LOW) low = min_abs(low, a[k], a[k + 1]);
     if (LOW) low = fminf(low, fabsf(a[8]));
   }
+  static __device__ __forceinline__ float wide(float a, const Recip &k, uint32_t &low) {
+    const uint32_t t = order(a);
+    const float q = split_quot(a, k), z = __fmul_rn(a, k.y);
+    low = min(low, t);
+    return t >= kOrderInf ? z : q;
+  }
+  __device__ __forceinline__ void step_wide(float (&ni)[10], float (&nv)[11],
+                                            const float (&I0)[10], const float (&V0)[9],
+                                            uint32_t &lowR, uint32_t &lowC) const {
+#pragma unroll
+    for (int k = 0; k < 10; k++) {
+      const float a1 = __fmul_rn(L, __fsub_rn(ni[k], I0[k]));
+      ni[k] = wide(__fsub_rn(__fsub_rn(nv[k + 1], nv[k]), dt_quot(a1)), kR, lowR);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      nv[k + 1] = __fadd_rn(V0[k], wide(__fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1])), kC, lowC));
+  }
+  __device__ __forceinline__ bool can_wide(const float (&I0)[10]) const {
+    return wide_wire(least_order(I0), L, kC.nb);
+  }
+  static __device__ __forceinline__ uint32_t least_order(const float (&ni)[10]) {
+    uint32_t m = ~0u;
+#pragma unroll
+    for (int k = 0; k < 10; k++) m = min(m, order(ni[k]));
+    return m;
+  }
+  __device__ __forceinline__ float most_C() const { return fabsf(kC.nb); }
   __device__ __forceinline__ bool sound(const float (&I0)[10], const float (&V0)[9]) const {
     float i = fabsf(I0[0]), v = fabsf(V0[0]);
 #pragma unroll
@@ -788,44 +876,42 @@ struct WireSource {
   int64_t S;
   float dt;
 };
-// n guarded steps on the state in `save`.  Out of line, as the LOW steps
-// below: they are rare, and their registers (all dividends of a phase at
-// once) would spill the free steps' loop.
+// n steps on the state in `save`, of the given form; if those come out wrong,
+// n guarded ones.  Returns whether they were right.  Out of line: rare, and
+// the guarded steps' registers (all dividends of a phase at once) would spill
+// the free steps' loop.
 template <typename Stepper, int STRIDE, typename Wires, typename F>
-__device__ __noinline__ void guarded_steps(const Wires wires, int n, F *save) {
-  const Stepper pk = wires.template stepper<Stepper>();
-  F nI0[10], V0[9], ni[10], nv[11];
-  wires.load(nI0, V0);
-  load_state<STRIDE>(save, ni, nv);
-  nv[0] = save[19 * STRIDE];
-  nv[10] = save[20 * STRIDE];
-#pragma unroll 1
-  for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
-  save_state<STRIDE>(save, ni, nv);
-}
-// n free steps with LOW on the state in `save`; whether they were right.
-template <typename Stepper, int STRIDE, typename Wires, typename F>
-__device__ __noinline__ bool low_steps(const Wires wires, int n, bool split, uint32_t nan,
-                                       F *save) {
+__device__ __noinline__ bool careful_steps(const Wires wires, int n, CarefulForm how, uint32_t nan,
+                                           uint32_t lanes, F *save) {
   Stepper pk = wires.template stepper<Stepper>();
   pk.kR.yl = save[21 * STRIDE];
   pk.kC.yl = save[22 * STRIDE];
   F nI0[10], V0[9], ni[10], nv[11];
   wires.load(nI0, V0);
-  load_state<STRIDE>(save, ni, nv);
   nv[0] = save[19 * STRIDE];
   nv[10] = save[20 * STRIDE];
-  float low = __int_as_float(0x7f800000);
-  if (split) {
+  load_state<STRIDE>(save, ni, nv);
+  bool right = false;
+  if (how == kWide) {
+    right = Stepper::least_order(ni) >= order(0x1p-74f);
+    uint32_t lowR = ~0u, lowC = ~0u;
 #pragma unroll 1
-    for (int i = 0; i < n; i++) pk.template step_free<3, true>(ni, nv, nI0, V0, low);
-  } else {
+    for (int i = 0; i < n; i++) pk.step_wide(ni, nv, nI0, V0, lowR, lowC);
+    right &= lowR >= order(0x1p-66f) && lowC >= order(__fmul_rn(0x1p-77f, pk.most_C()));
+  } else if (how == kLow) {
+    float low = __int_as_float(0x7f800000);
 #pragma unroll 1
     for (int i = 0; i < n; i++) pk.template step_free<0, true>(ni, nv, nI0, V0, low);
+    right = low >= kCLo && (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
+  }
+  right = __all_sync(lanes, right);
+  if (!right) {
+    load_state<STRIDE>(save, ni, nv);
+#pragma unroll 1
+    for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
   }
   save_state<STRIDE>(save, ni, nv);
-  return low >= (split ? kSplitLo : kCLo) &&
-         (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
+  return right;
 }
 struct SoloWire : WireSource {
   int64_t w;
@@ -840,12 +926,9 @@ struct SoloWire : WireSource {
     for (int k = 0; k < 9; k++) V0[k] = vol[k * S + w];
   }
   template <typename Stepper, int STRIDE>
-  __device__ __forceinline__ void guarded(int n, float *save) const {
-    guarded_steps<Stepper, STRIDE>(*this, n, save);
-  }
-  template <typename Stepper, int STRIDE>
-  __device__ __forceinline__ bool low(int n, bool split, uint32_t nan, float *save) const {
-    return low_steps<Stepper, STRIDE>(*this, n, split, nan, save);
+  __device__ __forceinline__ bool careful(int n, CarefulForm how, uint32_t nan, uint32_t lanes,
+                                          float *save) const {
+    return careful_steps<Stepper, STRIDE>(*this, n, how, nan, lanes, save);
   }
 };
 struct DualWires : WireSource {
@@ -862,12 +945,9 @@ struct DualWires : WireSource {
     for (int k = 0; k < 9; k++) V0[k] = make_float2(vol[k * S + wa], vol[k * S + wb]);
   }
   template <typename Stepper, int STRIDE>
-  __device__ __forceinline__ void guarded(int n, float2 *save) const {
-    guarded_steps<Stepper, STRIDE>(*this, n, save);
-  }
-  template <typename Stepper, int STRIDE>
-  __device__ __forceinline__ bool low(int n, bool split, uint32_t nan, float2 *save) const {
-    return low_steps<Stepper, STRIDE>(*this, n, split, nan, save);
+  __device__ __forceinline__ bool careful(int n, CarefulForm how, uint32_t nan, uint32_t lanes,
+                                          float2 *save) const {
+    return careful_steps<Stepper, STRIDE>(*this, n, how, nan, lanes, save);
   }
 };
 
@@ -1166,6 +1246,24 @@ struct LaneWire {
       low = fminf(low, last ? 1.0f : fabsf(ae.y));
     }
   }
+  // As DualExact::step_wide.
+  __device__ __forceinline__ void step_wide(LaneState &s, uint32_t &lowR, uint32_t &lowC) const {
+    const float2 neg1 = make_float2(-1.0f, -1.0f);
+    const float2 a1 = __fmul2_rn(make_float2(L, L), __fadd2_rn(s.x, nX0));
+    s.x = DualExact<true>::wide(
+        __ffma2_rn(dt_quot2(a1), neg1, __fadd2_rn(s.e, make_float2(s.nb, s.nb))), R, lowR);
+    const float l = __shfl_sync(0xffffffffu, s.x.y, left);
+    const float r = __shfl_sync(0xffffffffu, s.x.x, right);
+    const float vb =
+        __fadd_rn(-nVb, SoloExact<true>::wide(__fmul_rn(dt, __fsub_rn(-s.x.x, s.x.y)), C, lowC));
+    s.nb = -vb;
+    const float va = __fadd_rn(
+        Ve.x, SoloExact<true>::wide(first ? 1.0f : __fmul_rn(dt, __fadd_rn(l, s.x.x)), C, lowC));
+    const float vc = __fadd_rn(
+        Ve.y, SoloExact<true>::wide(last ? 1.0f : __fmul_rn(dt, __fadd_rn(s.x.y, r)), C, lowC));
+    if (!first) s.e.x = va;
+    if (!last) s.e.y = vc;
+  }
   // The reference's step for every state and divisor.
   __device__ __forceinline__ float dt_div(float a) const {
     return tiny_nonzero(a, kDtTiny) ? __fdiv_rn(a, dt) : dt_quot(a);
@@ -1230,10 +1328,10 @@ __global__ void __launch_bounds__(32)
   x.okR = divisor_ok(r, kRMin, kRMax);
   x.okC = divisor_ok(c, kCMin, kCMax);
 
-  int guarded = __all_sync(kAll, x.okR && x.okC) ? 0 : steps;
   uint32_t split = 0;
-  bool sound = false;
-  if (guarded == 0) {
+  bool sound = false, wide = false;
+  const bool eligible = __all_sync(kAll, x.okR && x.okC);
+  if (eligible) {
     const float nb[2] = {x.R.nb.x, x.C.nb}, y[2] = {x.R.y.x, x.C.y};
     float yl[2] = {x.R.yl.x, x.C.yl};
     const uint32_t checked = check_split(nb, y, yl);
@@ -1244,12 +1342,15 @@ __global__ void __launch_bounds__(32)
                                         min_abs(fabsf(x.nVb), x.first ? 1.0f : x.Ve.x,
                                                 x.last ? 1.0f : x.Ve.y),
                                         x.L, c, dt));
+    wide = split == 3u &&
+           __all_sync(kAll, wide_wire(min(order(I0), order(I1)), x.L, c));
   }
   x.E.nb = make_float2(x.C.nb, x.C.nb);
   x.E.y = make_float2(x.first ? 0.0f : x.C.y, x.last ? 0.0f : x.C.y);
   x.E.yl = make_float2(x.first ? 0.0f : x.C.yl, x.last ? 0.0f : x.C.yl);
 
-  int j = 0, run = kFirstRun, penalty = 1;
+  // as exact_steps: careful, skip count blocks
+  int j = 0, run = kFirstRun, careful = 0, penalty = 1, skip = sound ? 0 : 1, again = 1;
 #pragma unroll 1
   while (j < steps) {
     // which lanes' state is all NaN (each answers for what it computes)
@@ -1257,32 +1358,26 @@ __global__ void __launch_bounds__(32)
         kAll, (s.x.x != s.x.x && s.x.y != s.x.y && s.nb != s.nb && (x.first || s.e.x != s.e.x) &&
                (x.last || s.e.y != s.e.y)) ||
                   !mine);
+    const bool exempt = !mine || (nan & wire_lanes) == wire_lanes;
     float low = __int_as_float(0x7f800000);
     if (nan == kAll) {  // stays so: any form of quotient gives NaN, nothing to check
       x.steps_free<3, false>(s, steps - j, low);
       break;
     }
-    if (guarded == 0) {
-      const LaneState start = s;
-      const int n = min(run, steps - j);
-      bool right = true;
-      if (sound) {
-        if (split == 3u) x.steps_free<3, false>(s, n, low);
-        else if (split == 2u) x.steps_free<2, false>(s, n, low);
-        else if (split == 1u) x.steps_free<1, false>(s, n, low);
-        else x.steps_free<0, false>(s, n, low);
-        if (j + n == steps) right = fminf(fabsf(s.x.x), fabsf(s.x.y)) >= 0x1p-75f;
-      } else if (split == 3u) {
-        x.steps_free<3, true>(s, n, low);
-        right = low >= kSplitLo;
-      } else {
-        x.steps_free<0, true>(s, n, low);
-        right = low >= kCLo;
-      }
+    auto holds_nan = [&s]() {
       const float sum = __fadd_rn(__fadd_rn(s.x.x, s.x.y), __fadd_rn(__fadd_rn(s.e.x, s.e.y), s.nb));
-      right &= sum == sum;
-      right |= !mine || (nan & wire_lanes) == wire_lanes;
-      if (__all_sync(kAll, right)) {
+      return sum != sum;
+    };
+    const LaneState start = s;
+    if (sound && careful == 0) {
+      const int n = min(run, steps - j);
+      if (split == 3u) x.steps_free<3, false>(s, n, low);
+      else if (split == 2u) x.steps_free<2, false>(s, n, low);
+      else if (split == 1u) x.steps_free<1, false>(s, n, low);
+      else x.steps_free<0, false>(s, n, low);
+      bool right = !holds_nan();
+      if (j + n == steps) right &= fminf(fabsf(s.x.x), fabsf(s.x.y)) >= 0x1p-75f;
+      if (__all_sync(kAll, right || exempt)) {
         j += n;
         if (run == kMostRun) penalty = 1;
         run = min(2 * run, kMostRun);
@@ -1290,14 +1385,38 @@ __global__ void __launch_bounds__(32)
       }
       s = start;
       run = kFirstRun;
-      guarded = penalty;
+      careful = penalty;
       penalty = min(2 * penalty, 8);
     }
-    const int n = min(kGuardedRun, steps - j);
+    const int n = min(j == 0 ? kFrontRun : kCarefulRun, steps - j);
+    if (skip == 0 && eligible) {
+      bool right;
+      if (wide) {
+        right = min(order(s.x.x), order(s.x.y)) >= order(0x1p-74f);
+        uint32_t lowR = ~0u, lowC = ~0u;
 #pragma unroll 1
-    for (int i = 0; i < n; i++) x.step(s);
+        for (int i = 0; i < n; i++) x.step_wide(s, lowR, lowC);
+        right &= lowR >= order(0x1p-66f) && lowC >= order(__fmul_rn(0x1p-77f, fabsf(c)));
+      } else {
+        x.steps_free<0, true>(s, n, low);
+        right = low >= kCLo && !holds_nan();
+      }
+      right = __all_sync(kAll, right || exempt);
+      if (!right) {
+        s = start;
+        skip = again + 1;  // this block and the next ones guarded
+        again = min(2 * again, 8);
+      } else {
+        again = 1;
+      }
+    }
+    if (skip || !eligible) {
+#pragma unroll 1
+      for (int i = 0; i < n; i++) x.step(s);
+      if (skip) skip--;
+    }
     j += n;
-    guarded--;
+    if (careful) careful--;
   }
   if (mine) {
     a.cur[2 * g * S + w] = -s.x.x;
