@@ -9,6 +9,7 @@
 // (the benchmark's tasks do the same), so the schedules differ only in where
 // the reductions land and how they reach the target.
 #include <algorithm>
+#include <numeric>
 
 #include "ckt_internal.h"
 
@@ -39,6 +40,24 @@ __device__ __forceinline__ uint32_t hist_key(const HistArgs &a, uint64_t e) {
   return (uint32_t)__umul64hi(a.mod_magic * (uint32_t)r, (uint64_t)a.buckets);
 }
 
+// The same for elements 2^16 apart: their indices agree in the low 16 bits,
+// the ones that choose a seed each round, so a thread that keeps to one
+// residue chooses once.  Only the low 32 bits of the state reach the key.
+struct HashColumn {
+  uint32_t seed[16];
+  __device__ __forceinline__ HashColumn(const HistArgs &a, uint32_t residue) {
+    const uint32_t ival = a.base + residue;
+#pragma unroll
+    for (int j = 0; j < 16; j++) seed[j] = ((ival >> j) & 1u) ? a.seed1 : a.seed2;
+  }
+  __device__ __forceinline__ uint32_t key(const HistArgs &a, uint32_t e) const {
+    uint32_t r = a.base + e;
+#pragma unroll
+    for (int j = 0; j < 16; j++) r = (0xDEECE66Du * r + 0xBu) ^ seed[j];
+    return (uint32_t)__umul64hi(a.mod_magic * r, (uint64_t)a.buckets);
+  }
+};
+
 __device__ __forceinline__ uint64_t gtid() {
   return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 }
@@ -60,6 +79,71 @@ __global__ void __launch_bounds__(kFoldBlock) fold_smem_kernel(HistArgs a, uint3
   __syncthreads();
   for (uint32_t b = threadIdx.x; b < a.buckets; b += blockDim.x) {
     const uint32_t v = fold[b];
+    if (v) atomicAdd(hist + b, v);
+  }
+}
+
+// One block per SM folds the first `folded` buckets (all of them, if they fit)
+// into shared memory and adds the rest to the target directly.  WIDE: 32-bit
+// counters; otherwise two 16-bit counters per word, twice the buckets: the
+// thread whose add takes a counter to 2^15 moves 2^15 to the target, and the
+// block meets every kFoldRound elements per thread, so a counter gets at most
+// 2^14 more adds before that has happened, whatever the keys are.
+//
+// Elements are cut into units: 1024 residues mod 2^16 (a thread each) times a
+// range of rows of 2^16 elements; `parts` ranges, so that 64 * parts units
+// spread evenly over the blocks.
+//
+// Why: the L2 takes about 2.0e11 of these adds a second (0.66 a clock and SM)
+// whatever their addresses, and that bound the global folds; shared memory
+// takes them as fast as the hash gives them (5e11 a second).  2^29 elements
+// on a GB300, 16 rounds of the hash included: 50,000 buckets 1.12 ms (1.31
+// with a seed chosen per element and round), 110,000 1.31, 262,144 1.80,
+// 524,288 2.13, 1,048,576 2.34 ms; with the folds in L2 2.6 ms each.
+constexpr int kFoldRound = 16;
+constexpr uint32_t kFold16Buckets = 115712;  // 226 KB
+// Above this a block's share is too small a part of the buckets.
+constexpr uint32_t kFold16Most = 1u << 20;
+// Below this many elements the grid of 64 * parts units is not filled.
+constexpr uint64_t kFoldUnitsLeast = 1u << 23;
+
+template <bool WIDE>
+__global__ void __launch_bounds__(kFoldBlock)
+    fold_units_kernel(HistArgs a, uint32_t *hist, uint32_t folded, uint32_t parts) {
+  extern __shared__ uint32_t fold[];
+  const uint32_t words = WIDE ? folded : (folded + 1) / 2;
+  for (uint32_t b = threadIdx.x; b < words; b += kFoldBlock) fold[b] = 0u;  // identity
+  __syncthreads();
+  const uint64_t rows = (a.total + 65535u) >> 16;
+  for (uint32_t unit = blockIdx.x; unit < 64u * parts; unit += gridDim.x) {
+    const uint32_t residue = (unit & 63u) * kFoldBlock + threadIdx.x, part = unit >> 6;
+    const HashColumn column(a, residue);
+    const uint64_t m0 = rows * part / parts, m1 = rows * (part + 1) / parts;
+    for (uint64_t m = m0; m < m1; m += kFoldRound) {
+#pragma unroll 4
+      for (uint32_t i = 0; i < kFoldRound; i++) {
+        const uint64_t e = (m + i) << 16 | residue;
+        if (m + i >= m1 || e >= a.total) continue;
+        const uint32_t k = column.key(a, (uint32_t)e);
+        if (k >= folded) {
+          atomicAdd(hist + k, 1u);
+        } else if (WIDE) {
+          atomicAdd(fold + k, 1u);
+        } else {
+          const uint32_t shift = (k & 1u) * 16u;
+          const uint32_t before = atomicAdd(fold + (k >> 1), 1u << shift);
+          if (((before >> shift) & 0xffffu) == 0x7fffu) {
+            atomicSub(fold + (k >> 1), 0x8000u << shift);
+            atomicAdd(hist + k, 0x8000u);
+          }
+        }
+      }
+      if (!WIDE) __syncthreads();
+    }
+  }
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < folded; b += kFoldBlock) {
+    const uint32_t v = WIDE ? fold[b] : (fold[b >> 1] >> ((b & 1u) * 16u)) & 0xffffu;
     if (v) atomicAdd(hist + b, v);
   }
 }
@@ -353,7 +437,19 @@ int ckt_hist_run(const ckt_hist_params *p, int32_t schedule, uint32_t *hist, voi
       break;
     }
     case CKT_RED_FOLD: {
-      if (pl.smem_fold) {
+      if (p->buckets <= kFold16Most && a.total >= kFoldUnitsLeast) {
+        const uint32_t folded = std::min(p->buckets, pl.smem_fold ? p->buckets : kFold16Buckets);
+        // 64 * parts units, a multiple of the blocks and at least 8 for each
+        const uint32_t blocks = (uint32_t)smc;
+        const uint32_t step = blocks / std::gcd(blocks, 64u);
+        const uint32_t parts = step * std::max(1u, 8u * blocks / (64u * step));
+        const size_t smem = pl.smem_fold ? 4ull * folded : 4ull * ((folded + 1) / 2);
+        const auto kernel = pl.smem_fold ? fold_units_kernel<true> : fold_units_kernel<false>;
+        CKT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(2 * kFold16Buckets)));
+        kernel<<<blocks, kFoldBlock, smem, s>>>(a, hist, folded, parts);
+        CKT_CHECK_LAUNCH();
+      } else if (pl.smem_fold) {
         const size_t smem = 4ull * p->buckets;
         CKT_CUDA(cudaFuncSetAttribute(fold_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(4 * CKT_HIST_SMEM_FOLD_BUCKETS)));
