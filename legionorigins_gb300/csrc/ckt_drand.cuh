@@ -127,5 +127,70 @@ CKT_HD float node_capacitance(uint64_t x) {
   return u64_to_float(x + (1ull << 48)) * kTwoM48;
 }
 
+// The least x that fails the in-piece test (pct_below is monotone in x: 100 x
+// rounded to 53 bits never decreases); 2^48 when none does.
+inline uint64_t first_crossing(uint64_t threshold) {
+  uint64_t lo = 0, hi = 1ull << 48;
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) / 2;
+    if (pct_below(mid, threshold)) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// trunc_mul by two 32-bit products: rounding x n to 53 bits can reach the next
+// multiple of 2^48 only from the last 2^32 before it.
+CKT_HD uint32_t trunc_mul_fast(uint64_t x, uint32_t n) {
+  const uint64_t low = (x & 0xffffffffull) * n, high = (x >> 32) * n + (low >> 32);
+  if ((high & 0xffffu) == 0xffffu) return trunc_mul(x, n);
+  return (uint32_t)(high >> 16);
+}
+
+// (float)(u * scale + offset), double arithmetic, u = x * 2^-48: evaluated as
+// a 64-bit fixed-point sum where that settles the float.
+struct Affine {
+  uint64_t scale, offset;  // in units of 2^(e - 64)
+  int32_t exponent;        // e: scale + offset <= 2^(e - 1); 0x7fffffff: not usable
+};
+inline Affine make_affine(double scale, double offset) {
+  Affine a = {0, 0, 0x7fffffff};
+  const double sum = scale + offset;
+  if (!(scale >= 0) || !(offset >= 0) || !(sum > 8.6736173798840355e-19) ||  // 2^-60
+      !(sum < 1152921504606846976.0))                                       // 2^60
+    return a;
+  int e = -60;
+  double lim = 8.6736173798840355e-19;
+  while (!(sum <= lim)) {
+    lim *= 2;
+    e++;
+  }
+  e++;  // sum <= 2^(e - 1)
+  double unit = 1.0;  // 2^(64 - e)
+  for (int i = 0; i < 64 - e; i++) unit *= 2;
+  for (int i = 0; i < e - 64; i++) unit /= 2;
+  a.scale = (uint64_t)(scale * unit + 0.5);
+  a.offset = (uint64_t)(offset * unit + 0.5);
+  a.exponent = e;
+  return a;
+}
+// The sum is right to two units; the double expression's two roundings move
+// it by at most 2^-52 of itself.  Unless a boundary between two floats lies
+// that near, the float of the one is the float of the other; otherwise (and
+// for very small sums) false.
+CKT_HD bool affine_float(uint64_t x, const Affine &a, float *out) {
+  const uint64_t f = mulhi64(x << 16, a.scale) + a.offset;
+  if (f < (1ull << 40) || a.exponent == 0x7fffffff) return false;
+  const int shift = 63 - msb64(f);  // <= 23
+  const uint64_t g = f << shift, low = g & ((1ull << 40) - 1), half = 1ull << 39;
+  const uint64_t margin = (4ull << shift) + (1ull << 13);
+  if (low - (half - margin) <= 2 * margin) return false;
+  // f units of 2^(e - 64): the top bit weighs 2^(63 - shift + e - 64)
+  const uint32_t bits = ((uint32_t)(126 - shift + a.exponent) << 23) +
+                        ((uint32_t)(g >> 40) - 0x800000u) + (low > half ? 1u : 0u);
+  memcpy(out, &bits, sizeof(bits));
+  return true;
+}
+
 }  // namespace drand
 }  // namespace ckt

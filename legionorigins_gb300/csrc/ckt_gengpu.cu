@@ -11,10 +11,13 @@
 // decoded in parallel by speculation: the stream is cut into chunks of
 // kChunk draws, each chunk is decoded from all 7 possible entry phases (a
 // wire starts at most 6 draws past a chunk boundary), the chunks' phase maps
-// are composed to fix every chunk's true entry phase and first wire index,
-// and every chunk then emits its wires.  Node pointers, locations and the
-// graph follow in data-parallel kernels; per-node contribution lists are
-// sorted by (wire, end) so the graph is identical to the host-built one.
+// are composed, by groups of kGroup chunks and then over the groups, to fix
+// every group's true entry phase and first wire index, and a block per group
+// then emits its wires.  Locations and the graph follow in data-parallel
+// kernels; per-node contribution lists are sorted by (wire, end) so the graph
+// is identical to the host-built one.
+//
+// 4,194,304 wires, 1,048,576 nodes on a GB300 (GENERATOR_TIMES)
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -27,8 +30,9 @@ namespace {
 
 constexpr uint64_t kA = 0x5DEECE66Dull, kC = 0xBull, kMask = 0xffffffffffffull;
 constexpr int kChunk = 256;       // draws per chunk
-constexpr int kMapBlock = 256;    // chunks per block of the map composition
-constexpr int kTopTile = 1024;    // blocks per shared-memory tile of the top-level walk
+constexpr int kGroup = 64;        // chunks per group
+constexpr int kNear = 1024;       // draws reached by one entry of the near table
+constexpr int kMapsBlock = 128;   // chunks per block of the decoding
 
 struct Jump {
   uint64_t a[48], c[48];  // state after 2^i draws: a[i]*x + c[i]
@@ -49,10 +53,11 @@ Jump make_jump() {
   return j;
 }
 
-// State after k draws, k < kChunk: a[k]*x + c[k], for jumps from a chunk's
-// start to a wire inside it (lanes index it independently, so it lives in
-// global memory, not the constant bank).
-__device__ uint64_t g_near_a[kChunk], g_near_c[kChunk];
+// State after k draws, k < kNear, and after k chunks, k < kMapsBlock:
+// a[k]*x + c[k], for jumps from a block's first draw (lanes index it
+// independently, so it lives in global memory, not the constant bank).
+__device__ uint64_t g_near_a[kNear], g_near_c[kNear];
+__device__ uint64_t g_chunk_a[kMapsBlock], g_chunk_c[kMapsBlock];
 
 // The jump tables never change: they are copied to each device once.  (A
 // per-call copy from pageable memory would wait for the stream's earlier
@@ -69,16 +74,24 @@ int ensure_jump_table() {
   if (!loaded[dev]) {
     const Jump jump = make_jump();
     CKT_CUDA(cudaMemcpyToSymbol(g_jump, &jump, sizeof(Jump)));
-    std::vector<uint64_t> na(kChunk), nc(kChunk);
+    std::vector<uint64_t> na(kNear), nc(kNear), ca(kMapsBlock), cc(kMapsBlock);
     uint64_t a = 1, c = 0;
-    for (int k = 0; k < kChunk; k++) {
-      na[k] = a;
-      nc[k] = c;
+    for (int64_t k = 0; k < (int64_t)kMapsBlock * kChunk; k++) {
+      if (k < kNear) {
+        na[k] = a;
+        nc[k] = c;
+      }
+      if (k % kChunk == 0) {
+        ca[k / kChunk] = a;
+        cc[k / kChunk] = c;
+      }
       c = (kA * c + kC) & kMask;  // one more draw: x -> A x + C
       a = (kA * a) & kMask;
     }
-    CKT_CUDA(cudaMemcpyToSymbol(g_near_a, na.data(), kChunk * sizeof(uint64_t)));
-    CKT_CUDA(cudaMemcpyToSymbol(g_near_c, nc.data(), kChunk * sizeof(uint64_t)));
+    CKT_CUDA(cudaMemcpyToSymbol(g_near_a, na.data(), kNear * sizeof(uint64_t)));
+    CKT_CUDA(cudaMemcpyToSymbol(g_near_c, nc.data(), kNear * sizeof(uint64_t)));
+    CKT_CUDA(cudaMemcpyToSymbol(g_chunk_a, ca.data(), kMapsBlock * sizeof(uint64_t)));
+    CKT_CUDA(cudaMemcpyToSymbol(g_chunk_c, cc.data(), kMapsBlock * sizeof(uint64_t)));
     loaded[dev] = true;
   }
   return CKT_OK;
@@ -97,210 +110,297 @@ __device__ __forceinline__ uint64_t next(uint64_t &x) {
   return x;
 }
 
+__device__ __forceinline__ uint64_t near_jump(uint64_t x, uint32_t k) {
+  return (__ldg(g_near_a + k) * x + __ldg(g_near_c + k)) & kMask;
+}
+__device__ __forceinline__ uint64_t chunk_jump(uint64_t x, uint32_t k) {
+  return (__ldg(g_chunk_a + k) * x + __ldg(g_chunk_c + k)) & kMask;
+}
+
 // random_element of the piece's node set (its reversed order, see
 // ckt_gen.cpp): first + npp - 1 - (int)(drand48() * npp).
 __device__ __forceinline__ uint32_t pick(uint64_t x, uint32_t piece, uint32_t npp) {
-  return piece * npp + npp - 1 - drand::trunc_mul(x, npp);
+  return piece * npp + npp - 1 - drand::trunc_mul_fast(x, npp);
 }
 
 struct GenArgs {
   int32_t P, npp, wpp;
   double L_off, L_scale;
-  uint64_t pct_thr;  // drand::pct_threshold(pct)
+  drand::Affine L, C, leak;  // their fixed-point forms
+  uint64_t crossing;  // a wire leaves its piece when its 5th draw is at least this
   uint64_t seed_state;
   int64_t W, N;
 };
 
-// The wire leaves its piece: !(100 * drand48() < pct) with more than one piece.
-__device__ __forceinline__ bool crosses(const GenArgs &g, uint64_t x5) {
-  return g.P > 1 && !drand::pct_below(x5, g.pct_thr);
+// Node values: draws 3x, 3x+1, 3x+2 (circuit.cc:1121-1125).  A node per
+// thread, every store coalesced.
+__global__ void __launch_bounds__(256)
+    gen_nodes_kernel(GenArgs g, float *charge, float *nvolt, float *cap, float *leak,
+                     int32_t *locator) {
+  __shared__ uint64_t first;
+  if (threadIdx.x == 0) first = skip(g.seed_state, 3 * 256 * (uint64_t)blockIdx.x);
+  __syncthreads();
+  const int64_t n = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (n >= g.N) return;
+  uint64_t x = near_jump(first, 3 * threadIdx.x);
+  charge[n] = 0.f;
+  nvolt[n] = drand::node_voltage(next(x));
+  cap[n] = drand::node_capacitance(next(x));
+  next(x);
+  float l;
+  if (!drand::affine_float(x, g.leak, &l))
+    l = __double2float_rn(__dmul_rn((double)0.1f, drand::value(x)));
+  leak[n] = l;
+  locator[n] = 1;
 }
 
-// Node values: draws 3x, 3x+1, 3x+2 (circuit.cc:1121-1125).
-__global__ void gen_nodes_kernel(GenArgs g, float *charge, float *nvolt, float *cap, float *leak,
-                                 int32_t *locator) {
-  const int64_t x0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 16;
-  if (x0 >= g.N) return;
-  uint64_t x = skip(g.seed_state, 3 * (uint64_t)x0);
-  const int64_t x1 = min(g.N, x0 + 16);
-  for (int64_t n = x0; n < x1; n++) {
-    charge[n] = 0.f;
-    nvolt[n] = drand::node_voltage(next(x));
-    cap[n] = drand::node_capacitance(next(x));
-    leak[n] = __double2float_rn(__dmul_rn((double)0.1f, drand::value(next(x))));
-    locator[n] = 1;
+// Arrays set to zero by the decoding kernel.
+struct Zeroed {
+  uint32_t *p[4];
+  uint64_t words[4];
+};
+// Slice `part` of `parts` of the 16-byte words of every array.
+__device__ __forceinline__ void zero_slice(const Zeroed &z, uint64_t thread, uint64_t threads,
+                                           uint32_t part, uint32_t parts) {
+  for (int r = 0; r < 4; r++) {
+    const uint64_t head = min(z.words[r], (uint64_t)((0 - (reinterpret_cast<uintptr_t>(z.p[r]) >> 2)) & 3u));
+    const uint64_t quads = (z.words[r] - head) / 4, tail = head + 4 * quads;
+    uint4 *q = reinterpret_cast<uint4 *>(z.p[r] + head);
+    const uint64_t end = quads * (part + 1) / parts;
+    for (uint64_t i = quads * part / parts + thread; i < end; i += threads)
+      q[i] = make_uint4(0, 0, 0, 0);
+    if (part == 0 && thread < head) z.p[r][thread] = 0;
+    if (part == 0 && thread < z.words[r] - tail) z.p[r][tail + thread] = 0;
   }
 }
 
 // Per chunk and entry phase q: where the chain leaves the chunk (0..6 past
-// its end) and how many wires start inside it.  Only a wire's 5th draw (the
-// in-piece test) matters here, so the state advances for every draw and is
-// converted to a double only where some phase needs that test.
-constexpr int kChunkWords = (kChunk + 4 + 31) / 32;  // in-piece test bits of a chunk's draws
-constexpr int kMapsBlock = 128;
+// its end) and how many wires start inside it, as 9 bits (count << 3 | exit)
+// at bit 9q; and the crossing test of every draw, as bits.  A chain stays in
+// one residue class of draws mod 6 until a wire crosses, so it hops from one
+// set bit of its class to the next (a few per chunk at 95% in-piece) instead
+// of from wire to wire.  The currents' and voltages' zeros (76 bytes a wire,
+// most of the generator's memory traffic) are written here, a slice between
+// every 32 draws, under the arithmetic.
+constexpr int kChunkWords = (kChunk + 4 + 31) / 32;  // a wire's test lies 4 draws past its start
 
 __global__ void __launch_bounds__(kMapsBlock)
-    chunk_maps_kernel(GenArgs g, int64_t base, int64_t nchunks, uint8_t *exit_phase,
-                      uint32_t *count) {
+    decode_kernel(GenArgs g, int64_t base, int64_t nchunks, uint32_t *bits, uint64_t *maps,
+                  Zeroed zero) {
   __shared__ uint32_t sbits[kChunkWords][kMapsBlock];
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchunks) return;
-  // 1. the cross-piece test of every draw of the chunk, as bits (the same
-  //    work on every lane)
-  uint64_t x = skip(g.seed_state, (uint64_t)(base + c * kChunk));
-#pragma unroll
-  for (int wd = 0; wd < kChunkWords; wd++) {
-    uint32_t bits = 0;
-    for (int k = 0; k < 32; k++) bits |= (crosses(g, next(x)) ? 1u : 0u) << k;
-    sbits[wd][threadIdx.x] = bits;
-  }
-  // 2. each entry phase hops wire to wire: 6 draws, or 7 when the wire's
-  //    5th draw says it leaves its piece
-#pragma unroll
-  for (int q = 0; q < 7; q++) {
-    uint32_t s = (uint32_t)q, n = 0;
-    while (s < (uint32_t)kChunk) {
-      const uint32_t t = s + 4;
-      s += 6u + ((sbits[t >> 5][threadIdx.x] >> (t & 31u)) & 1u);
-      n++;
-    }
-    exit_phase[c * 7 + q] = (uint8_t)(s - (uint32_t)kChunk);
-    count[c * 7 + q] = n;
-  }
-}
-
-// The chunk maps of kMapBlock consecutive chunks composed in shared memory:
-// for every phase q the block might be entered with, each chunk's entry
-// phase and the wires before it inside the block, and the block's own map.
-__global__ void __launch_bounds__(128)
-    map_block_kernel(int64_t nchunks, const uint8_t *__restrict__ exit_phase,
-                     const uint32_t *__restrict__ count, uint8_t *rel_phase, uint32_t *rel_base,
-                     uint8_t *bexit, uint32_t *bcount) {
-  __shared__ uint8_t se[kMapBlock * 7];
-  __shared__ uint32_t sc[kMapBlock * 7];
-  const int64_t c0 = (int64_t)blockIdx.x * kMapBlock;
-  const int n = (int)min((int64_t)kMapBlock, nchunks - c0);
-  for (int i = threadIdx.x; i < n * 7; i += blockDim.x) {
-    se[i] = exit_phase[c0 * 7 + i];
-    sc[i] = count[c0 * 7 + i];
-  }
+  __shared__ uint64_t first;
+  const uint64_t threads = (uint64_t)gridDim.x * kMapsBlock;
+  const int64_t c = (int64_t)blockIdx.x * kMapsBlock + threadIdx.x;
+  if (threadIdx.x == 0)
+    first = skip(g.seed_state, (uint64_t)base + (uint64_t)blockIdx.x * kMapsBlock * kChunk);
   __syncthreads();
-  if (threadIdx.x < 7) {
-    const int q = threadIdx.x;
-    int ph = q;
-    uint32_t tot = 0;
-    for (int k = 0; k < n; k++) {
-      rel_phase[(c0 + k) * 7 + q] = (uint8_t)ph;
-      rel_base[(c0 + k) * 7 + q] = tot;
-      tot += sc[k * 7 + ph];
-      ph = se[k * 7 + ph];
-    }
-    bexit[blockIdx.x * 7 + q] = (uint8_t)ph;
-    bcount[blockIdx.x * 7 + q] = tot;
+  uint64_t x = chunk_jump(first, threadIdx.x);
+#pragma unroll 1
+  for (int wd = 0; wd < kChunkWords; wd++) {
+    const int draws = wd < kChunk / 32 ? 32 : 4;
+    uint32_t b = 0;
+#pragma unroll 4
+    for (int k = 0; k < draws; k++) b |= (next(x) >= g.crossing ? 1u : 0u) << k;
+    sbits[wd][threadIdx.x] = b;
+    if (c < nchunks) bits[(int64_t)wd * nchunks + c] = b;
+    zero_slice(zero, (uint64_t)c, threads, wd, kChunkWords);
   }
+  if (c >= nchunks) return;
+  uint64_t map = 0;
+#pragma unroll 1
+  for (uint32_t q = 0; q < 7; q++) {
+    uint32_t s = q, n = 0;  // the next wire's start, the wires before it
+    while (s < (uint32_t)kChunk) {
+      // the next draw t >= s + 4 of the class of s + 4 that crosses
+      uint32_t wd = (s + 4) >> 5, r = (s + 4) % 6u;
+      // draws of residue r in word wd: bits k with 32 wd + k = r mod 6
+      uint32_t m = sbits[wd][threadIdx.x] & (0x41041041u << ((r + 4 * wd) % 6u)) &
+                   (~0u << ((s + 4) & 31u));
+      while (!m && ++wd < (uint32_t)kChunkWords)
+        m = sbits[wd][threadIdx.x] & (0x41041041u << ((r + 4 * wd) % 6u));
+      const uint32_t at = m ? 32 * wd + (uint32_t)__ffs((int)m) - 1 - 4 : ~0u;  // that wire's start
+      if (at >= (uint32_t)kChunk) {  // none starts in this chunk
+        const uint32_t k = ((uint32_t)kChunk - 1 - s) / 6 + 1;
+        n += k;
+        s += 6 * k;
+      } else {
+        n += (at - s) / 6 + 1;
+        s = at + 7;
+      }
+    }
+    map |= (uint64_t)(n << 3 | (s - (uint32_t)kChunk)) << (9 * q);
+  }
+  maps[c] = map;
 }
 
-// The chain through the blocks from phase 0 (the first wire starts at the
-// first wire draw): every block's entry phase and first wire.  One block;
-// the maps pass through shared memory a tile at a time, so the walk's
-// dependent steps are shared-memory reads.
-__global__ void __launch_bounds__(256)
-    map_top_kernel(int64_t nblocks, const uint8_t *__restrict__ bexit,
-                   const uint32_t *__restrict__ bcount, uint8_t *bphase, uint64_t *bbase) {
-  __shared__ uint8_t se[kTopTile * 7];
-  __shared__ uint32_t sc[kTopTile * 7];
-  int ph = 0;
-  uint64_t tot = 0;
-  for (int64_t b0 = 0; b0 < nblocks; b0 += kTopTile) {
-    const int n = (int)min((int64_t)kTopTile, nblocks - b0);
+// One chunk's step of a chain at phase ph: 9 bits of its map.
+__device__ __forceinline__ uint32_t map_at(uint64_t map, uint32_t ph) {
+  return (uint32_t)(map >> (9 * ph)) & 511u;
+}
+
+// A group's chunk maps composed, a warp per group, a lane per entry phase:
+// wires << 3 | exit phase.
+__global__ void __launch_bounds__(128)
+    group_maps_kernel(int64_t nchunks, int64_t ngroups, const uint64_t *__restrict__ maps,
+                      uint32_t *gmap) {
+  __shared__ uint64_t sm[4][kGroup];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const int64_t g = (int64_t)blockIdx.x * 4 + warp;
+  if (g >= ngroups) return;
+  const int n = (int)min((int64_t)kGroup, nchunks - g * kGroup);
+  for (int k = (int)lane; k < n; k += 32) sm[warp][k] = maps[g * kGroup + k];
+  __syncwarp();
+  if (lane >= 7) return;
+  uint32_t ph = lane, wires = 0;
+  for (int k = 0; k < n; k++) {
+    const uint32_t e = map_at(sm[warp][k], ph);
+    wires += e >> 3;
+    ph = e & 7u;
+  }
+  gmap[g * 7 + lane] = wires << 3 | ph;
+}
+
+// The chain through the groups from phase 0 (the first wire starts at the
+// first wire draw): every group's entry phase and first wire.  One block; a
+// tile of groups at a time in shared memory, cut into kTopSegments whose maps
+// are composed side by side, then chained, then walked side by side.
+constexpr int kTopTile = 4096, kTopSegments = 128;
+
+__global__ void __launch_bounds__(1024)
+    top_kernel(int64_t ngroups, const uint32_t *__restrict__ gmap, uint8_t *gphase,
+               uint64_t *gbase) {
+  extern __shared__ uint32_t sm[];  // [7 * kTopTile]
+  __shared__ uint32_t seg[kTopSegments][7];
+  __shared__ uint64_t seg_base[kTopSegments];
+  __shared__ uint32_t seg_phase[kTopSegments], phase;
+  __shared__ uint64_t wires;
+  if (threadIdx.x == 0) {
+    phase = 0;
+    wires = 0;
+  }
+  for (int64_t g0 = 0; g0 < ngroups; g0 += kTopTile) {
+    const int n = (int)min((int64_t)kTopTile, ngroups - g0);
+    const int len = (n + kTopSegments - 1) / kTopSegments;
+    for (int i = threadIdx.x; i < 7 * n; i += blockDim.x) sm[i] = gmap[g0 * 7 + i];
     __syncthreads();
-    for (int i = threadIdx.x; i < n * 7; i += blockDim.x) {
-      se[i] = bexit[b0 * 7 + i];
-      sc[i] = bcount[b0 * 7 + i];
+    if (threadIdx.x < 7 * kTopSegments) {
+      const int q = threadIdx.x % 7, sg = threadIdx.x / 7;
+      uint32_t ph = (uint32_t)q, tot = 0;
+      for (int k = sg * len; k < min(n, (sg + 1) * len); k++) {
+        const uint32_t e = sm[k * 7 + ph];
+        tot += e >> 3;
+        ph = e & 7u;
+      }
+      seg[sg][q] = tot << 3 | ph;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      for (int k = 0; k < n; k++) {
-        bphase[b0 + k] = (uint8_t)ph;
-        bbase[b0 + k] = tot;
-        tot += sc[k * 7 + ph];
-        ph = se[k * 7 + ph];
+      uint32_t ph = phase;
+      uint64_t tot = wires;
+      for (int sg = 0; sg < kTopSegments; sg++) {
+        seg_phase[sg] = ph;
+        seg_base[sg] = tot;
+        const uint32_t e = seg[sg][ph];
+        tot += e >> 3;
+        ph = e & 7u;
+      }
+      phase = ph;
+      wires = tot;
+    }
+    __syncthreads();
+    if (threadIdx.x < kTopSegments) {
+      uint32_t ph = seg_phase[threadIdx.x];
+      uint64_t tot = seg_base[threadIdx.x];
+      for (int k = threadIdx.x * len; k < min(n, ((int)threadIdx.x + 1) * len); k++) {
+        gphase[g0 + k] = (uint8_t)ph;
+        gbase[g0 + k] = tot;
+        const uint32_t e = sm[k * 7 + ph];
+        tot += e >> 3;
+        ph = e & 7u;
       }
     }
+    __syncthreads();
   }
 }
 
-// Every chunk walks its wires from its entry phase and records where each
-// starts in the draw stream (relative to the first wire draw).
-__global__ void wire_starts_kernel(GenArgs g, int64_t base, int64_t nchunks,
-                                   const uint8_t *__restrict__ rel_phase,
-                                   const uint32_t *__restrict__ rel_base,
-                                   const uint8_t *__restrict__ bphase,
-                                   const uint64_t *__restrict__ bbase, uint32_t *starts,
-                                   uint64_t *chunk_state) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchunks) return;
-  const int64_t b = c / kMapBlock;
-  const int qb = bphase[b];  // the block's entry phase selects the chunk's entry
-  int64_t w = (int64_t)bbase[b] + rel_base[c * 7 + qb];
-  if (w >= g.W) return;
-  const int64_t p0 = base + c * kChunk;
-  uint32_t sr = rel_phase[c * 7 + qb];  // relative to p0
-  uint64_t x = skip(g.seed_state, (uint64_t)p0);
-  chunk_state[c] = x;
-  uint32_t t = 0;
-  while (sr < (uint32_t)kChunk && w < g.W) {
-    starts[w] = (uint32_t)(c * kChunk + sr);
-    while (t <= sr + 4) {  // advance to the wire's in-piece draw
-      next(x);
-      t++;
+// A group's wires (circuit.cc:1158-1186): the chunks' entry phases and the
+// wires' starts in shared memory, then a wire per thread: jump to its first
+// draw, draw R, L, C, the in-node, the in-piece test and the out-node, store
+// every field coalesced, and count the two nodes' degrees.  What a count
+// returns is the entry's place among its node's, so that filling the lists
+// needs no second round of atomics.
+constexpr int kGroupWires = kGroup * ((kChunk + 5) / 6);
+
+__global__ void __launch_bounds__(256)
+    gen_wires_kernel(GenArgs g, int64_t base, int64_t nchunks, const uint32_t *__restrict__ bits,
+                     const uint64_t *__restrict__ maps, const uint8_t *__restrict__ gphase,
+                     const uint64_t *__restrict__ gbase, uint32_t *in_ptr, uint32_t *out_ptr,
+                     float *L, float *R, float *C, int32_t *locator, uint32_t *deg,
+                     uint32_t *rank_in, uint32_t *rank_out) {
+  __shared__ uint64_t smaps[kGroup], state[kGroup], first;
+  __shared__ uint32_t sbits[kChunkWords][kGroup], before[kGroup + 1], phase[kGroup];
+  __shared__ uint16_t starts[kGroupWires];  // chunk << 8 | draw
+  const int64_t c0 = (int64_t)blockIdx.x * kGroup;
+  const uint64_t w0 = gbase[blockIdx.x];
+  if (w0 >= (uint64_t)g.W) return;  // the stream is cut for 7 draws a wire
+  const uint32_t n = (uint32_t)min((int64_t)kGroup, nchunks - c0);
+  if (threadIdx.x < n) smaps[threadIdx.x] = maps[c0 + threadIdx.x];
+  if (threadIdx.x == 128) first = skip(g.seed_state, (uint64_t)(base + c0 * kChunk));
+  for (uint32_t i = threadIdx.x; i < kChunkWords * kGroup; i += 256) {
+    const uint32_t wd = i / kGroup, k = i % kGroup;
+    if (k < n) sbits[wd][k] = bits[(int64_t)wd * nchunks + c0 + k];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t ph = gphase[blockIdx.x], tot = 0;
+    for (uint32_t k = 0; k < n; k++) {
+      phase[k] = ph;
+      before[k] = tot;
+      const uint32_t e = map_at(smaps[k], ph);
+      tot += e >> 3;
+      ph = e & 7u;
     }
-    sr += crosses(g, x) ? 7u : 6u;
-    w++;
+    before[n] = tot;
   }
-}
-
-// One thread per wire (circuit.cc:1158-1186): jump to its first draw, draw
-// R, L, C, the in-node, the in-piece test and the out-node, and store every
-// field coalesced.
-__global__ void gen_wires_kernel(GenArgs g, const uint32_t *__restrict__ starts,
-                                 const uint64_t *__restrict__ chunk_state, uint32_t *in_ptr,
-                                 uint32_t *out_ptr, float *L, float *R, float *C,
-                                 int32_t *locator) {
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= g.W) return;
-  const uint32_t st = starts[w], k = st % (uint32_t)kChunk;
-  uint64_t x = (__ldg(g_near_a + k) * chunk_state[st / (uint32_t)kChunk] + __ldg(g_near_c + k)) &
-               kMask;
-  const uint64_t xR = next(x), xL = next(x), xC = next(x), xIn = next(x), xPct = next(x);
-  const uint32_t n = (uint32_t)(w / g.wpp);
-  R[w] = drand::resistance(xR);
-  L[w] = __double2float_rn(__dadd_rn(__dmul_rn(drand::value(xL), g.L_scale), g.L_off));
-  C[w] = __double2float_rn(__dmul_rn(drand::value(xC), 0.1));
-  in_ptr[w] = pick(xIn, n, (uint32_t)g.npp);
-  if (!crosses(g, xPct)) {
-    out_ptr[w] = pick(next(x), n, (uint32_t)g.npp);
-  } else {
-    int nn = (int)drand::trunc_mul(next(x), (uint32_t)(g.P - 1));
-    if (nn >= (int)n) nn++;
-    const uint32_t o = pick(next(x), (uint32_t)nn, (uint32_t)g.npp);
-    out_ptr[w] = o;
-    locator[o] = 0;
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + n)
+    state[threadIdx.x - 64] = chunk_jump(first, threadIdx.x - 64);
+  __syncthreads();
+  if (threadIdx.x < n) {
+    uint32_t s = phase[threadIdx.x];
+    for (uint32_t i = before[threadIdx.x]; s < (uint32_t)kChunk; i++) {
+      starts[i] = (uint16_t)(threadIdx.x << 8 | s);
+      s += 6u + ((sbits[(s + 4) >> 5][threadIdx.x] >> ((s + 4) & 31u)) & 1u);
+    }
   }
-}
-
-// Locations (circuit.cc:1228-1244) and node degrees.
-__global__ void gen_locs_kernel(GenArgs g, const uint32_t *in_ptr, const uint32_t *out_ptr,
-                                const int32_t *locator, uint8_t *in_loc, uint8_t *out_loc,
-                                uint32_t *deg) {
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= g.W) return;
-  const uint32_t n = (uint32_t)(w / g.wpp), a = in_ptr[w], b = out_ptr[w];
-  in_loc[w] = locator[a] ? CKT_PRIVATE_PTR : CKT_SHARED_PTR;
-  out_loc[w] = (b / (uint32_t)g.npp != n) ? CKT_GHOST_PTR
-                                          : (locator[b] ? CKT_PRIVATE_PTR : CKT_SHARED_PTR);
-  atomicAdd(deg + a, 1u);
-  atomicAdd(deg + b, 1u);
+  __syncthreads();
+  const uint32_t total = (uint32_t)min((uint64_t)before[n], (uint64_t)g.W - w0);
+  for (uint32_t i = threadIdx.x; i < total; i += 256) {
+    const uint32_t w = (uint32_t)w0 + i, st = starts[i];
+    uint64_t x = near_jump(state[st >> 8], st & 255u);
+    const uint64_t xR = next(x), xL = next(x), xC = next(x), xIn = next(x), xPct = next(x);
+    const uint32_t piece = w / (uint32_t)g.wpp;
+    float l, c;
+    if (!drand::affine_float(xL, g.L, &l))
+      l = __double2float_rn(__dadd_rn(__dmul_rn(drand::value(xL), g.L_scale), g.L_off));
+    if (!drand::affine_float(xC, g.C, &c)) c = __double2float_rn(__dmul_rn(drand::value(xC), 0.1));
+    const uint32_t a = pick(xIn, piece, (uint32_t)g.npp);
+    uint32_t b;
+    if (xPct < g.crossing) {
+      b = pick(next(x), piece, (uint32_t)g.npp);
+    } else {
+      uint32_t to = drand::trunc_mul_fast(next(x), (uint32_t)(g.P - 1));
+      if (to >= piece) to++;
+      b = pick(next(x), to, (uint32_t)g.npp);
+      locator[b] = 0;
+    }
+    rank_in[w] = atomicAdd(deg + a, 1u);
+    rank_out[w] = atomicAdd(deg + b, 1u);
+    in_ptr[w] = a;
+    out_ptr[w] = b;
+    R[w] = drand::resistance(xR);
+    L[w] = l;
+    C[w] = c;
+  }
 }
 
 // Exclusive scan of deg[0..n) into off[0..n] (off[n] = total), three passes.
@@ -343,40 +443,72 @@ __global__ void scan_blocks_kernel(const uint32_t *in, int64_t n, uint32_t *out,
   }
 }
 
-__global__ void scan_sums_kernel(uint32_t *sums, int64_t nblocks, uint32_t *total) {
-  uint32_t run = 0;
-  for (int64_t b = 0; b < nblocks; b++) {
-    const uint32_t v = sums[b];
-    sums[b] = run;
-    run += v;
+// Exclusive scan of the blocks' sums, one block; *total = their sum.
+__global__ void __launch_bounds__(1024)
+    scan_sums_kernel(uint32_t *sums, int64_t nblocks, uint32_t *total) {
+  __shared__ uint32_t warp_tot[32], carry;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry = 0;
+  for (int64_t b0 = 0; b0 < nblocks; b0 += 1024) {
+    const int64_t b = b0 + threadIdx.x;
+    const uint32_t v = b < nblocks ? sums[b] : 0u;
+    uint32_t incl = v;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_tot[wid] = incl;
+    __syncthreads();
+    uint32_t before = carry;
+    for (uint32_t k = 0; k < wid; k++) before += warp_tot[k];
+    if (b < nblocks) sums[b] = before + incl - v;
+    __syncthreads();
+    if (threadIdx.x == 1023) carry = before + incl;
+    __syncthreads();
   }
-  *total = run;
+  if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void scan_add_kernel(uint32_t *out, int64_t n, const uint32_t *sums) {
+// The blocks' sums added, and private nodes marked.  sums NULL: no wires.
+__global__ void scan_add_kernel(uint32_t *out, int64_t n, const uint32_t *sums,
+                                const int32_t *locator) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += sums[i / ((int64_t)kScanBlock * kScanItems)];
+  if (i >= n) return;
+  const uint32_t o = sums ? out[i] + sums[i / ((int64_t)kScanBlock * kScanItems)] : 0u;
+  out[i] = o | (locator[i] ? kPrivateBit : 0u);
 }
 
-__global__ void csr_fill_kernel(int64_t W, const uint32_t *in_ptr, const uint32_t *out_ptr,
-                                uint32_t *cursor, uint32_t *tmp) {
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= W) return;
-  tmp[atomicAdd(cursor + in_ptr[w], 1u)] = (uint32_t)(w << 1);
-  tmp[atomicAdd(cursor + out_ptr[w], 1u)] = (uint32_t)(w << 1) | 1u;
+// Locations (circuit.cc:1228-1244), and every wire end into its node's list
+// at the place its count gave it.
+__global__ void __launch_bounds__(256)
+    place_kernel(GenArgs g, const uint32_t *__restrict__ in_ptr,
+                 const uint32_t *__restrict__ out_ptr, const uint32_t *__restrict__ off,
+                 const uint32_t *__restrict__ rank_in, const uint32_t *__restrict__ rank_out,
+                 uint8_t *in_loc, uint8_t *out_loc, uint32_t *tmp) {
+  const uint32_t w = blockIdx.x * 256 + threadIdx.x;
+  if (w >= (uint32_t)g.W) return;
+  const uint32_t a = in_ptr[w], b = out_ptr[w], oa = off[a], ob = off[b];
+  const uint32_t first = w / (uint32_t)g.wpp * (uint32_t)g.npp;
+  in_loc[w] = oa & kPrivateBit ? CKT_PRIVATE_PTR : CKT_SHARED_PTR;
+  out_loc[w] = b - first >= (uint32_t)g.npp
+                   ? CKT_GHOST_PTR
+                   : (ob & kPrivateBit ? CKT_PRIVATE_PTR : CKT_SHARED_PTR);
+  tmp[(oa & kOffsetMask) + rank_in[w]] = w << 1;
+  tmp[(ob & kOffsetMask) + rank_out[w]] = w << 1 | 1u;
 }
 
 // Per node: sort its contributions by (wire, end), then write the entries
-// with their piece-group flags, the wire ends' slots and the flag bits, and
-// mark private nodes in the offsets.  A warp takes 32 consecutive nodes: their
+// with their piece-group flags, the wire ends' slots and the flag bits.  A
+// warp takes 32 consecutive nodes: their
 // runs are one contiguous span, staged in shared memory (coalesced in and
 // out), sorted there a node per lane; a span larger than the stage is sorted
 // in place in tmp instead.
 constexpr uint32_t kFinishSpan = 512;  // entries per warp staged in shared memory
 
 __global__ void __launch_bounds__(256)
-    csr_finish_kernel(GenArgs g, uint32_t *off, const int32_t *locator, uint32_t *tmp,
-                      uint32_t *ent, uint32_t *slot_in, uint32_t *slot_out, uint32_t *gstart) {
+    csr_finish_kernel(GenArgs g, const uint32_t *__restrict__ off, uint32_t *tmp, uint32_t *ent,
+                      uint32_t *slot_in, uint32_t *slot_out, uint32_t *gstart) {
   __shared__ uint32_t sbuf[8][kFinishSpan];
   const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
   const int64_t x0 = ((int64_t)blockIdx.x * 8 + wp) * 32;
@@ -418,7 +550,6 @@ __global__ void __launch_bounds__(256)
       if (end) slot_out[w] = i;
       else slot_in[w] = i;
     }
-    if (locator[x]) atomicOr(off + x, kPrivateBit);
   }
   __syncwarp();
   if (staged) {
@@ -462,40 +593,39 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
   if (jr) return jr;
   GenArgs g;
   g.P = P; g.npp = npp; g.wpp = wpp;
-  g.pct_thr = drand::pct_threshold(p->pct_wire_in_piece);
+  g.crossing = P > 1 ? drand::first_crossing(drand::pct_threshold(p->pct_wire_in_piece))
+                     : 1ull << 48;
   g.L_off = p->L_offset; g.L_scale = p->L_scale;
+  g.L = drand::make_affine(g.L_scale, g.L_off);
+  g.C = drand::make_affine(0.1, 0.0);
+  g.leak = drand::make_affine((double)0.1f, 0.0);
   g.seed_state = (((uint64_t)p->random_seed & 0xffffffffull) << 16) | 0x330Eull;
   g.W = W; g.N = N;
 
-  gen_nodes_kernel<<<grid_for((N + 15) / 16), 256, 0, s>>>(g, o->charge, o->node_voltage,
-                                                          o->node_capacitance, o->node_leakage,
-                                                          o->locator);
+  gen_nodes_kernel<<<grid_for(N), 256, 0, s>>>(g, o->charge, o->node_voltage, o->node_capacitance,
+                                              o->node_leakage, o->locator);
   CKT_CHECK_LAUNCH();
-  CKT_CUDA(cudaMemsetAsync(o->off, 0, (N + 1) * 4, s));
   if (W == 0) {
-    // No contributions: only the private-node flags of the offsets remain
-    // (every node is private); the entry arrays are never touched.
-    csr_finish_kernel<<<grid_for(N), 256, 0, s>>>(g, o->off, o->locator, nullptr, nullptr,
-                                                  nullptr, nullptr, nullptr);
+    // No contributions: the offsets hold the private-node flags only (every
+    // node is private); the entry arrays are never touched.
+    scan_add_kernel<<<grid_for(N), 256, 0, s>>>(o->off, N, nullptr, o->locator);
     CKT_CHECK_LAUNCH();
+    CKT_CUDA(cudaMemsetAsync(o->off + N, 0, 4, s));
     return CKT_OK;
   }
 
-  // Scratch: chunk maps and their composition, degree cursors, unsorted
+  // Scratch: draw tests, chunk and group maps, degrees and places, unsorted
   // contributions.
   const int64_t base = 3 * N;
   const int64_t nchunks = (7 * W + 8 + kChunk - 1) / kChunk;
-  const int64_t nblocks = (nchunks + kMapBlock - 1) / kMapBlock;
+  const int64_t ngroups = (nchunks + kGroup - 1) / kGroup;
   const int64_t scan_blocks = (N + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
-  const size_t sz_exit = nchunks * 7, sz_cnt = nchunks * 7 * 4, sz_rph = nchunks * 7,
-               sz_rb = nchunks * 7 * 4, sz_bexit = nblocks * 7, sz_bcnt = nblocks * 7 * 4,
-               sz_bph = nblocks, sz_bb = nblocks * 8, sz_deg = (N + 1) * 4,
-               sz_sums = (scan_blocks + 1) * 4, sz_tmp = 2 * W * 4, sz_starts = W * 4,
-               sz_cstate = nchunks * 8;
+  const size_t sz_bits = nchunks * kChunkWords * 4, sz_maps = nchunks * 8, sz_gmap = ngroups * 7 * 4,
+               sz_gph = ngroups, sz_gb = ngroups * 8, sz_deg = N * 4,
+               sz_sums = (scan_blocks + 1) * 4, sz_rank = W * 4, sz_tmp = 2 * W * 4;
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  const size_t total = al(sz_exit) + al(sz_cnt) + al(sz_rph) + al(sz_rb) + al(sz_bexit) +
-                       al(sz_bcnt) + al(sz_bph) + al(sz_bb) + al(sz_deg) + al(sz_sums) +
-                       al(sz_tmp) + al(sz_starts) + al(sz_cstate);
+  const size_t total = al(sz_bits) + al(sz_maps) + al(sz_gmap) + al(sz_gph) + al(sz_gb) +
+                       al(sz_deg) + al(sz_sums) + 2 * al(sz_rank) + al(sz_tmp);
   char *scratch = nullptr;
   CKT_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&scratch), total, s));
   char *q = scratch;
@@ -504,59 +634,52 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
     q += al(b);
     return r;
   };
-  uint8_t *exit_phase = (uint8_t *)take(sz_exit);
-  uint32_t *count = (uint32_t *)take(sz_cnt);
-  uint8_t *rel_phase = (uint8_t *)take(sz_rph);
-  uint32_t *rel_base = (uint32_t *)take(sz_rb);
-  uint8_t *bexit = (uint8_t *)take(sz_bexit);
-  uint32_t *bcount = (uint32_t *)take(sz_bcnt);
-  uint8_t *bphase = (uint8_t *)take(sz_bph);
-  uint64_t *bbase = (uint64_t *)take(sz_bb);
+  uint32_t *bits = (uint32_t *)take(sz_bits);
+  uint64_t *maps = (uint64_t *)take(sz_maps);
+  uint32_t *gmap = (uint32_t *)take(sz_gmap);
+  uint8_t *gphase = (uint8_t *)take(sz_gph);
+  uint64_t *gbase = (uint64_t *)take(sz_gb);
   uint32_t *deg = (uint32_t *)take(sz_deg);
   uint32_t *sums = (uint32_t *)take(sz_sums);
+  uint32_t *rank_in = (uint32_t *)take(sz_rank);
+  uint32_t *rank_out = (uint32_t *)take(sz_rank);
   uint32_t *tmp = (uint32_t *)take(sz_tmp);
-  uint32_t *starts = (uint32_t *)take(sz_starts);
-  uint64_t *chunk_state = (uint64_t *)take(sz_cstate);
   int rc = CKT_OK;
   auto ok = [&rc](cudaError_t e) {
     if (rc == CKT_OK && e != cudaSuccess)
       rc = set_error(CKT_ECUDA, "device generator: %s", cudaGetErrorString(e));
   };
 
-  chunk_maps_kernel<<<grid_for(nchunks, kMapsBlock), kMapsBlock, 0, s>>>(g, base, nchunks,
-                                                                          exit_phase, count);
+  const Zeroed zero = {{reinterpret_cast<uint32_t *>(o->current),
+                        reinterpret_cast<uint32_t *>(o->voltage), deg, o->gstart},
+                       {10 * (uint64_t)W, 9 * (uint64_t)W, (uint64_t)N,
+                        (uint64_t)(2 * W + 31) / 32}};
+  decode_kernel<<<grid_for(nchunks, kMapsBlock), kMapsBlock, 0, s>>>(g, base, nchunks, bits, maps,
+                                                                    zero);
   ok(cudaGetLastError());
-  map_block_kernel<<<(unsigned)nblocks, 128, 0, s>>>(nchunks, exit_phase, count, rel_phase,
-                                                      rel_base, bexit, bcount);
+  group_maps_kernel<<<grid_for(ngroups, 4), 128, 0, s>>>(nchunks, ngroups, maps, gmap);
   ok(cudaGetLastError());
-  map_top_kernel<<<1, 256, 0, s>>>(nblocks, bexit, bcount, bphase, bbase);
+  ok(cudaFuncSetAttribute(top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          7 * kTopTile * 4));
+  top_kernel<<<1, 1024, 7 * 4 * (size_t)std::min<int64_t>(ngroups, kTopTile), s>>>(ngroups, gmap,
+                                                                                  gphase, gbase);
   ok(cudaGetLastError());
-  wire_starts_kernel<<<grid_for(nchunks, 128), 128, 0, s>>>(
-      g, base, nchunks, rel_phase, rel_base, bphase, bbase, starts, chunk_state);
-  ok(cudaGetLastError());
-  gen_wires_kernel<<<grid_for(W), 256, 0, s>>>(g, starts, chunk_state, o->in_ptr, o->out_ptr,
-                                               o->inductance, o->resistance, o->capacitance,
-                                               o->locator);
-  ok(cudaGetLastError());
-  ok(cudaMemsetAsync(deg, 0, sz_deg, s));
-  gen_locs_kernel<<<grid_for(W), 256, 0, s>>>(g, o->in_ptr, o->out_ptr, o->locator, o->in_loc,
-                                              o->out_loc, deg);
+  gen_wires_kernel<<<(unsigned)ngroups, 256, 0, s>>>(
+      g, base, nchunks, bits, maps, gphase, gbase, o->in_ptr, o->out_ptr, o->inductance,
+      o->resistance, o->capacitance, o->locator, deg, rank_in, rank_out);
   ok(cudaGetLastError());
   scan_blocks_kernel<<<(unsigned)scan_blocks, kScanBlock, 0, s>>>(deg, N, o->off, sums);
   ok(cudaGetLastError());
-  scan_sums_kernel<<<1, 1, 0, s>>>(sums, scan_blocks, o->off + N);
+  scan_sums_kernel<<<1, 1024, 0, s>>>(sums, scan_blocks, o->off + N);
   ok(cudaGetLastError());
-  scan_add_kernel<<<grid_for(N), 256, 0, s>>>(o->off, N, sums);
+  scan_add_kernel<<<grid_for(N), 256, 0, s>>>(o->off, N, sums, o->locator);
   ok(cudaGetLastError());
-  ok(cudaMemcpyAsync(deg, o->off, N * 4, cudaMemcpyDeviceToDevice, s));  // fill cursors
-  csr_fill_kernel<<<grid_for(W), 256, 0, s>>>(W, o->in_ptr, o->out_ptr, deg, tmp);
+  place_kernel<<<grid_for(W), 256, 0, s>>>(g, o->in_ptr, o->out_ptr, o->off, rank_in, rank_out,
+                                           o->in_loc, o->out_loc, tmp);
   ok(cudaGetLastError());
-  ok(cudaMemsetAsync(o->gstart, 0, ((2 * W + 31) / 32) * 4, s));
-  csr_finish_kernel<<<grid_for(N), 256, 0, s>>>(g, o->off, o->locator, tmp, o->ent, o->slot_in,
-                                                o->slot_out, o->gstart);
+  csr_finish_kernel<<<grid_for(N), 256, 0, s>>>(g, o->off, tmp, o->ent, o->slot_in, o->slot_out,
+                                                o->gstart);
   ok(cudaGetLastError());
-  ok(cudaMemsetAsync(o->current, 0, 10 * W * 4, s));
-  ok(cudaMemsetAsync(o->voltage, 0, 9 * W * 4, s));
   cudaFreeAsync(scratch, s);
   return rc;
 }
