@@ -494,14 +494,8 @@ int ckt_batch_run_sequential(ckt_batch *b, int32_t mode, int32_t per_piece, void
         CKT_CUDA(cudaStreamSynchronize(s));
       }
     } else {
-      const uint32_t n4 = c.N / 4;
-      if (n4)
-        uv_all_vec4_kernel<<<grid_for(n4), 256, 0, s>>>(
-            n4, reinterpret_cast<float4 *>(c.charge), reinterpret_cast<float4 *>(c.nvolt),
-            reinterpret_cast<const float4 *>(c.cap), reinterpret_cast<const float4 *>(c.leak));
-      if (c.N > 4 * n4)
-        uv_all_scalar_kernel<<<1, 256, 0, s>>>(4 * n4, c.N - 4 * n4, c.charge, c.nvolt, c.cap,
-                                               c.leak);
+      uv_all_vec4_kernel<<<grid_for((c.N + 3) / 4), 256, 0, s>>>(c.N, c.charge, c.nvolt, c.cap,
+                                                                c.leak);
       CKT_CHECK_LAUNCH();
     }
   }

@@ -113,8 +113,9 @@ constexpr uint32_t kTileBlock = 32 * (kTileWarps + 1);  // consumer warps + one 
 constexpr uint32_t kTileStages = 3;
 // Shared memory of one stage: I[0] and I[9] slices of a chunk (a ghost
 // step's in-end and out-end runs in their place), then the step's block
-// (header + entries).
-constexpr uint32_t kStageVals = 2 * kChunkWires;
+// (header + entries).  The I[9] slice may start up to 3 floats into its
+// place (DcTileArgs::shift).
+constexpr uint32_t kStageVals = 2 * kChunkWires + 4;
 constexpr uint32_t kStageBlockWords = kStepHeaderWords + kStepEntriesMax;
 constexpr uint32_t kStageBytes = (kStageVals + kStageBlockWords) * 4;
 
@@ -124,7 +125,8 @@ struct DcTileArgs {
   const uint32_t *ent;
   const float *ghost;  // ghost steps' values, packed by ghost_pack_kernel
   const uint32_t *mask;  // per tile: nodes whose folds are added at the end
-  const float *I0, *I9;  // 16-byte aligned; slices may be read up to a multiple of 4 wires
+  const float *I0, *I9;  // I0 16-byte aligned; its slices are read up to a multiple of 4 wires
+  uint32_t shift;        // floats from the 16-byte boundary below I9 to I9
   float *charge, *voltage;
   const float *cap, *leak;
   uint32_t *error;
@@ -166,16 +168,20 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 
 // One lane sums its list of node runs in a step: entries [b, e) of the
 // step's block, runs back to back, each opened by a head entry; an entry's
-// current is svals[end * kChunkWires + index].
+// current is svals[index], an out-end's svals[kChunkWires + index], or with
+// SHIFT svals[out + index].
+template <bool SHIFT>
 __device__ __forceinline__ void dc_tile_lane_walk(const uint32_t *sent, const float *svals,
-                                                  uint32_t b, uint32_t e, float2 *ssum,
-                                                  float dt) {
+                                                  uint32_t out, uint32_t b, uint32_t e,
+                                                  float2 *ssum, float dt) {
   uint32_t node = 0xffffffffu;
   float acc = 0.0f, fold = 0.0f;
   for (uint32_t p = b; p < e; p++) {
     const uint32_t u = sent[p];
-    const uint32_t end = (u & kTeEnd) ? 1u : 0u;
-    const float v = svals[end * kChunkWires + (u & (kChunkWires - 1))];
+    const bool end = (u & kTeEnd) != 0u;
+    static_assert(kTeEnd == kChunkWires, "the end bit is the out-ends' offset");
+    const float v = SHIFT ? svals[(end ? out : 0u) + (u & (kChunkWires - 1))]
+                          : svals[u & (2 * kChunkWires - 1)];
     if (u & kTeHead) {
       if (node != 0xffffffffu) ssum[node] = make_float2(acc, fold);
       node = (u >> kTeNodeShift) & (kTileNodesMax - 1);
@@ -220,10 +226,11 @@ __device__ __forceinline__ void fence_proxy_async_global() {
 //  * Few ghost ends (whole slices would be mostly unused): a thread takes
 //    kPackPer entries spread over the list and reads each current directly,
 //    all its loads in flight together.
+// VEC9: I9 is 16-byte aligned and its row extends to a multiple of 4 wires.
 // Either way the tile pass may already be running (programmatic dependent
 // launch); it waits for this grid before its first ghost step's copy.
 constexpr uint32_t kPackBlock = 512, kPackPer = 4;
-template <bool STAGED>
+template <bool STAGED, bool VEC9>
 __global__ void __launch_bounds__(kPackBlock, 3) ghost_pack_kernel(const uint2 *__restrict__ list,
                                                                    const uint32_t *__restrict__ blk,
                                                                    uint32_t n, uint32_t W,
@@ -252,15 +259,18 @@ __global__ void __launch_bounds__(kPackBlock, 3) ghost_pack_kernel(const uint2 *
     e[j] = k < last ? list[k] : make_uint2(0xffffffffu, 0u);
   }
   if (STAGED) {
-    const uint32_t nw4 = (min(kPackWires, W - w0) + 3u) / 4u;  // arrays extend to a multiple of 4
-    const float4 *src0 = reinterpret_cast<const float4 *>(I0 + w0);
+    const uint32_t nw = min(kPackWires, W - w0), nw4 = (nw + 3u) / 4u;
+    const float4 *src0 = reinterpret_cast<const float4 *>(I0 + w0);  // row 0 ends inside the array
     const float4 *src1 = reinterpret_cast<const float4 *>(I9 + w0);
+    float *sf = reinterpret_cast<float *>(sv);
     for (uint32_t i = threadIdx.x; i < nw4; i += kPackBlock) {
       if (d & kPackHasIn) sv[i] = __ldcs(src0 + i);
-      if (d & kPackHasOut) sv[kPackWires / 4 + i] = __ldcs(src1 + i);
+      if (VEC9 && (d & kPackHasOut)) sv[kPackWires / 4 + i] = __ldcs(src1 + i);
     }
+    if (!VEC9 && (d & kPackHasOut))
+      for (uint32_t i = threadIdx.x; i < nw; i += kPackBlock)
+        sf[kPackWires + i] = __ldcs(I9 + w0 + i);
     __syncthreads();
-    const float *sf = reinterpret_cast<const float *>(sv);
 #pragma unroll
     for (uint32_t j = 0; j < kPackPer; j++)
       if (e[j].x != 0xffffffffu)
@@ -286,8 +296,9 @@ __global__ void __launch_bounds__(kPackBlock, 3) ghost_pack_kernel(const uint2 *
 // and the warps run through the steps independently, each handing its stage
 // back through the stage's `empty` barrier.  UV = true also applies
 // update_voltages to the tile's nodes (the fused node pass: charge ends at
-// zero).
-template <bool UV>
+// zero).  SHIFT: row 9 of the currents is not 16-byte aligned, or may end off
+// a multiple of 4 wires.
+template <bool UV, bool SHIFT>
 __global__ void __launch_bounds__(kTileBlock, 1) dc_tile_kernel(DcTileArgs a) {
   extern __shared__ __align__(128) unsigned char dct_smem[];
   const uint32_t TN = a.tile_nodes;
@@ -298,6 +309,8 @@ __global__ void __launch_bounds__(kTileBlock, 1) dc_tile_kernel(DcTileArgs a) {
   uint64_t *empty = full + kTileStages;
   uint64_t *maskbar = empty + kTileStages, *nodebar = maskbar + 1;
   volatile uint32_t *abort = reinterpret_cast<volatile uint32_t *>(nodebar + 1);
+  // per stage: where its out-ends' currents start
+  volatile uint32_t *out_at = abort + 1;
   auto vals_of = [&](uint32_t slot) {
     return reinterpret_cast<float *>(stage0 + slot * kStageBytes);
   };
@@ -340,18 +353,29 @@ __global__ void __launch_bounds__(kTileBlock, 1) dc_tile_kernel(DcTileArgs a) {
     // in-end and out-end values: [0, n0) and [kChunkWires, kChunkWires + n1)
     const float *src0, *src1;
     uint32_t n0, n1;
+    fence_proxy_async_smem();
     if ((st.z & kGhostStep) == 0u) {
-      n0 = n1 = (min(kChunkWires, a.W - st.z * kChunkWires) + 3u) & ~3u;
+      const uint32_t len = min(kChunkWires, a.W - st.z * kChunkWires);
+      n0 = (len + 3u) & ~3u;
       src0 = a.I0 + st.z * kChunkWires;
-      src1 = a.I9 + st.z * kChunkWires;
+      // from the boundary below I9's slice, in whole 16 bytes; where those
+      // would pass row 9's last wire, its last floats go one by one
+      const uint32_t shift = SHIFT ? a.shift : 0u, end = shift + len;
+      src1 = a.I9 + st.z * kChunkWires - shift;
+      n1 = (end + 3u) & ~3u;
+      if (SHIFT) out_at[slot] = kChunkWires + shift;
+      if (SHIFT && st.z * kChunkWires + n1 - a.shift > a.W) {
+        n1 = end & ~3u;
+        for (uint32_t i = n1; i < end; i++) vals_of(slot)[kChunkWires + i] = src1[i];
+      }
     } else {
       n0 = (((st.z >> kGhostCountBits) & kGhostCountMask) + 3u) & ~3u;
       n1 = ((st.z & kGhostCountMask) + 3u) & ~3u;
       src0 = a.ghost + st.w;
       src1 = src0 + n0;
+      if (SHIFT) out_at[slot] = kChunkWires;
     }
-    uint64_t *bar = full + slot;
-    fence_proxy_async_smem();
+    uint64_t *bar = full + slot;  // (its arrival releases out_at and the floats above)
     mbar_expect_tx(bar, (st.y + n0 + n1) * 4);
     if (n0) bulk_g2s(vals_of(slot), src0, n0 * 4, bar);
     if (n1) bulk_g2s(vals_of(slot) + kChunkWires, src1, n1 * 4, bar);
@@ -444,7 +468,8 @@ __global__ void __launch_bounds__(kTileBlock, 1) dc_tile_kernel(DcTileArgs a) {
       const uint32_t last = hdr[kTileLanes];
       const uint32_t l = threadIdx.x;  // consumer lane list (warp * 32 + lane)
       const uint32_t b = hdr[l], e = l + 1 < kTileLanes ? hdr[l + 1] : last;
-      dc_tile_lane_walk(blk + kStepHeaderWords, vals_of(slot), b, e, ssum, a.dt);
+      dc_tile_lane_walk<SHIFT>(blk + kStepHeaderWords, vals_of(slot), SHIFT ? out_at[slot] : 0u, b,
+                               e, ssum, a.dt);
       __syncwarp();
       if (lane == 0) mbar_arrive(empty + slot);
     }

@@ -185,5 +185,6 @@ struct ckt_graph {
   // Bound of the tiled pass's copy waits; a wait that runs out sets the
   // error word instead of hanging the block.
   uint64_t tile_timeout_ns = 2000000000ull;
+  bool tile_timeout_set = false;  // by ckt_graph_set_tile_timeout
   int64_t device_bytes = 0;
 };

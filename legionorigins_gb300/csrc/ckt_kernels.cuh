@@ -1669,13 +1669,23 @@ __device__ __forceinline__ float uv_one(float v, float q, float c, float l) {
   return __fmul_rn(__fadd_rn(v, __fdiv_rn(q, c)), __fsub_rn(1.0f, l));
 }
 
-// Whole node range, four nodes per thread with 16-byte loads and stores.
+// Whole node range, four nodes per thread with 16-byte loads and stores; the
+// last N mod 4 one by one, in the same launch.
 static __global__ void __launch_bounds__(256)
-    uv_all_vec4_kernel(uint32_t n4, float4 *__restrict__ q, float4 *__restrict__ v,
-                       const float4 *__restrict__ c, const float4 *__restrict__ l) {
+    uv_all_vec4_kernel(uint32_t N, float *__restrict__ charge, float *__restrict__ voltage,
+                       const float *__restrict__ cap, const float *__restrict__ leak) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n4) return;
-  const float4 qq = q[i], vv = v[i], cc = c[i], ll = l[i];
+  if (i >= N / 4u) {
+    if (i == N / 4u)
+      for (uint32_t x = N & ~3u; x < N; x++) {
+        voltage[x] = uv_one(voltage[x], charge[x], cap[x], leak[x]);
+        charge[x] = 0.0f;
+      }
+    return;
+  }
+  float4 *q = reinterpret_cast<float4 *>(charge), *v = reinterpret_cast<float4 *>(voltage);
+  const float4 qq = q[i], vv = v[i], cc = reinterpret_cast<const float4 *>(cap)[i],
+               ll = reinterpret_cast<const float4 *>(leak)[i];
   float4 r;
   r.x = uv_one(vv.x, qq.x, cc.x, ll.x);
   r.y = uv_one(vv.y, qq.y, cc.y, ll.y);

@@ -155,26 +155,28 @@ static int check_graph_wires(const ckt_graph *g, const ckt_wires &w) {
   return CKT_OK;
 }
 
-// The tiled node pass needs 16-byte aligned current slices that may be read
-// up to a multiple of 4 wires: current 16-byte aligned, seg_stride a
-// multiple of 4 (then seg_stride >= W rounds W up).
+// The tiled node pass needs row 0 of the currents 16-byte aligned.  A block
+// per tile of 8192 nodes streams its wires' currents, one step after another,
+// for about 40 us however few tiles there are; the gather form's blocks of
+// 256 nodes spread over the GPU and take less while they are few.  Fused pass
+// on a GB300, tiled / gather, 95% in-piece: 8,192 nodes 45 / 19 us, 65,536
+// 41 / 19, 262,144 42 / 29, 524,288 42 / 42, 660,000 47 / 49, 768,000 39 / 53,
+// 1,048,576 45 / 69 us.  A caller who set a bound for the tiled pass's waits gets the
+// tiled pass.
 static bool tile_plan_usable(const ckt_graph *g, const ckt_wires &w) {
   return g->num_tiles > 0 && (reinterpret_cast<uintptr_t>(w.current) & 15u) == 0 &&
-         (w.seg_stride & 3) == 0;
+         (g->tile_timeout_set || 8u * g->num_tiles >= 5u * (uint32_t)device_sms());
 }
 
-
-template <bool UV>
-static int launch_dc_tile(const ckt_graph *g, const ckt_wires &w, const ckt_nodes &n, float dt,
-                          cudaStream_t s) {
+template <bool UV, bool SHIFT>
+static int launch_dc_tile_t(const ckt_graph *g, const ckt_wires &w, const ckt_nodes &n, float dt,
+                            cudaStream_t s) {
   static thread_local int configured_device = -1;
   int dev = 0;
   CKT_CUDA(cudaGetDevice(&dev));
   if (configured_device != dev) {
     const int most = (int)dc_tile_smem_bytes(kTileNodesMax);
-    CKT_CUDA(cudaFuncSetAttribute(dc_tile_kernel<true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CKT_CUDA(cudaFuncSetAttribute(dc_tile_kernel<false>,
+    CKT_CUDA(cudaFuncSetAttribute(dc_tile_kernel<UV, SHIFT>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     configured_device = dev;
   }
@@ -186,6 +188,7 @@ static int launch_dc_tile(const ckt_graph *g, const ckt_wires &w, const ckt_node
   a.mask = g->tile_mask;
   a.I0 = w.current;
   a.I9 = w.current + 9 * w.seg_stride;
+  a.shift = (uint32_t)(reinterpret_cast<uintptr_t>(a.I9) >> 2) & 3u;
   a.charge = n.charge;
   a.voltage = n.voltage;
   a.cap = n.capacitance;
@@ -225,24 +228,31 @@ static int launch_dc_tile(const ckt_graph *g, const ckt_wires &w, const ckt_node
   if (g->ghost_n > 0) {
     const uint32_t n = (uint32_t)g->ghost_n;
     if (g->ghost_staged) {
-      ghost_pack_kernel<true><<<g->ghost_blocks, kPackBlock, 0, s>>>(
+      ghost_pack_kernel<true, !SHIFT><<<g->ghost_blocks, kPackBlock, 0, s>>>(
           g->ghost_list, g->ghost_block, n, (uint32_t)g->W, a.I0, a.I9, g->ghost);
     } else {
       const uint32_t per_block = kPackBlock * kPackPer;
-      ghost_pack_kernel<false><<<(n + per_block - 1) / per_block, kPackBlock, 0, s>>>(
+      ghost_pack_kernel<false, true><<<(n + per_block - 1) / per_block, kPackBlock, 0, s>>>(
           g->ghost_list, g->ghost_block, n, (uint32_t)g->W, a.I0, a.I9, g->ghost);
     }
     CKT_CHECK_LAUNCH();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
   }
-  CKT_CUDA(cudaLaunchKernelEx(&cfg, dc_tile_kernel<UV>, a));
+  CKT_CUDA(cudaLaunchKernelEx(&cfg, dc_tile_kernel<UV, SHIFT>, a));
   if (order) {
     CKT_CUDA(cudaEventRecord(g->ghost_done, s));
     g->ghost_stream = s;
     g->ghost_used = true;
   }
   return CKT_OK;
+}
+
+template <bool UV>
+static int launch_dc_tile(const ckt_graph *g, const ckt_wires &w, const ckt_nodes &n, float dt,
+                          cudaStream_t s) {
+  return (w.seg_stride & 3) == 0 ? launch_dc_tile_t<UV, false>(g, w, n, dt, s)
+                                 : launch_dc_tile_t<UV, true>(g, w, n, dt, s);
 }
 
 // A tiled node pass that ran out of a copy wait left its tile's results
@@ -437,23 +447,14 @@ int ckt_update_voltages_all(const ckt_graph *graph, ckt_nodes nodes, void *strea
                          reinterpret_cast<uintptr_t>(nodes.capacitance) |
                          reinterpret_cast<uintptr_t>(nodes.leakage)) &
                         15u) == 0;
-  uint64_t done = 0;
-  if (aligned && N >= 4) {
-    const uint64_t n4 = N / 4;
-    uv_all_vec4_kernel<<<grid_for(n4), 256, 0, s>>>(
-        (uint32_t)n4, reinterpret_cast<float4 *>(nodes.charge),
-        reinterpret_cast<float4 *>(nodes.voltage),
-        reinterpret_cast<const float4 *>(nodes.capacitance),
-        reinterpret_cast<const float4 *>(nodes.leakage));
-    CKT_CHECK_LAUNCH();
-    done = n4 * 4;
-  }
-  if (done < N) {
-    uv_all_scalar_kernel<<<grid_for(N - done), 256, 0, s>>>(
-        (uint32_t)done, (uint32_t)(N - done), nodes.charge, nodes.voltage, nodes.capacitance,
-        nodes.leakage);
-    CKT_CHECK_LAUNCH();
-  }
+  if (aligned)
+    uv_all_vec4_kernel<<<grid_for((N + 3) / 4), 256, 0, s>>>((uint32_t)N, nodes.charge,
+                                                             nodes.voltage, nodes.capacitance,
+                                                             nodes.leakage);
+  else
+    uv_all_scalar_kernel<<<grid_for(N), 256, 0, s>>>(0u, (uint32_t)N, nodes.charge, nodes.voltage,
+                                                     nodes.capacitance, nodes.leakage);
+  CKT_CHECK_LAUNCH();
   return CKT_OK;
 }
 
