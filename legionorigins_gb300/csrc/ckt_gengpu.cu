@@ -17,7 +17,12 @@
 // kernels; per-node contribution lists are sorted by (wire, end) so the graph
 // is identical to the host-built one.
 //
-// 4,194,304 wires, 1,048,576 nodes on a GB300 (GENERATOR_TIMES)
+// 4,194,304 wires, 1,048,576 nodes on a GB300: 345 us, of which decode 20,
+// gen_wires 123 (26 of it zeros, 35 the degree counts' returned adds), place
+// 87 (17 zeros; 8.4 M reads and 8.4 M writes at random in L2), csr_finish 66,
+// nodes 12, the map composition 15, the scan 13; 600 us when phases hopped
+// wire by wire, three expressions per wire ran on the FP64 pipe, degrees and
+// lists took a round of atomics each and zeros their own passes.
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -129,6 +134,7 @@ struct GenArgs {
   drand::Affine L, C, leak;  // their fixed-point forms
   uint64_t crossing;  // a wire leaves its piece when its 5th draw is at least this
   uint64_t seed_state;
+  uint64_t wpp_magic;  // floor(2^64 / wpp) + 1: w / wpp = high64(w * wpp_magic), w < 2^32
   int64_t W, N;
 };
 
@@ -154,82 +160,76 @@ __global__ void __launch_bounds__(256)
   locator[n] = 1;
 }
 
-// Arrays set to zero by the decoding kernel.
+// Arrays set to zero beside a kernel's other work, 16 bytes at a time.  The
+// currents' and voltages' zeros are 76 bytes a wire, most of the generator's
+// memory traffic (47 us of it at the copy rate, beside whichever kernel).
 struct Zeroed {
-  uint32_t *p[4];
-  uint64_t words[4];
+  uint32_t *p[2];
+  uint64_t words[2];
 };
-// Slice `part` of `parts` of the 16-byte words of every array.
-__device__ __forceinline__ void zero_slice(const Zeroed &z, uint64_t thread, uint64_t threads,
-                                           uint32_t part, uint32_t parts) {
-  for (int r = 0; r < 4; r++) {
-    const uint64_t head = min(z.words[r], (uint64_t)((0 - (reinterpret_cast<uintptr_t>(z.p[r]) >> 2)) & 3u));
-    const uint64_t quads = (z.words[r] - head) / 4, tail = head + 4 * quads;
+__device__ __forceinline__ void zero_slice(const Zeroed &z, uint64_t thread, uint64_t threads) {
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const uint64_t off = (0 - (reinterpret_cast<uintptr_t>(z.p[r]) >> 2)) & 3u;
+    const uint64_t head = min(z.words[r], off), quads = (z.words[r] - head) / 4;
+    const uint64_t tail = head + 4 * quads;
     uint4 *q = reinterpret_cast<uint4 *>(z.p[r] + head);
-    const uint64_t end = quads * (part + 1) / parts;
-    for (uint64_t i = quads * part / parts + thread; i < end; i += threads)
-      q[i] = make_uint4(0, 0, 0, 0);
-    if (part == 0 && thread < head) z.p[r][thread] = 0;
-    if (part == 0 && thread < z.words[r] - tail) z.p[r][tail + thread] = 0;
+    for (uint64_t i = thread; i < quads; i += threads) q[i] = make_uint4(0, 0, 0, 0);
+    if (thread < head) z.p[r][thread] = 0;
+    if (thread < z.words[r] - tail) z.p[r][tail + thread] = 0;
   }
 }
 
 // Per chunk and entry phase q: where the chain leaves the chunk (0..6 past
 // its end) and how many wires start inside it, as 9 bits (count << 3 | exit)
-// at bit 9q; and the crossing test of every draw, as bits.  A chain stays in
-// one residue class of draws mod 6 until a wire crosses, so it hops from one
-// set bit of its class to the next (a few per chunk at 95% in-piece) instead
-// of from wire to wire.  The currents' and voltages' zeros (76 bytes a wire,
-// most of the generator's memory traffic) are written here, a slice between
-// every 32 draws, under the arithmetic.
+// at bit 9q; and the crossing test of every draw, as bits.  The chains are
+// followed backwards, all at once: a wire that starts at draw s is followed
+// by one at s + 6, or s + 7 if draw s + 4 crosses, so f(s) = f(s + 6 or 7)
+// with one wire more; the last 8 values of f stay in registers and no lane
+// leaves the others (hopping forward from each phase, lanes did: 9,200
+// instructions a warp against 3,700).
 constexpr int kChunkWords = (kChunk + 4 + 31) / 32;  // a wire's test lies 4 draws past its start
 
 __global__ void __launch_bounds__(kMapsBlock)
     decode_kernel(GenArgs g, int64_t base, int64_t nchunks, uint32_t *bits, uint64_t *maps,
                   Zeroed zero) {
-  __shared__ uint32_t sbits[kChunkWords][kMapsBlock];
   __shared__ uint64_t first;
   const uint64_t threads = (uint64_t)gridDim.x * kMapsBlock;
   const int64_t c = (int64_t)blockIdx.x * kMapsBlock + threadIdx.x;
   if (threadIdx.x == 0)
     first = skip(g.seed_state, (uint64_t)base + (uint64_t)blockIdx.x * kMapsBlock * kChunk);
   __syncthreads();
-  uint64_t x = chunk_jump(first, threadIdx.x);
-#pragma unroll 1
-  for (int wd = 0; wd < kChunkWords; wd++) {
-    const int draws = wd < kChunk / 32 ? 32 : 4;
-    uint32_t b = 0;
-#pragma unroll 4
-    for (int k = 0; k < draws; k++) b |= (next(x) >= g.crossing ? 1u : 0u) << k;
-    sbits[wd][threadIdx.x] = b;
-    if (c < nchunks) bits[(int64_t)wd * nchunks + c] = b;
-    zero_slice(zero, (uint64_t)c, threads, wd, kChunkWords);
-  }
+  zero_slice(zero, (uint64_t)c, threads);
   if (c >= nchunks) return;
-  uint64_t map = 0;
-#pragma unroll 1
-  for (uint32_t q = 0; q < 7; q++) {
-    uint32_t s = q, n = 0;  // the next wire's start, the wires before it
-    while (s < (uint32_t)kChunk) {
-      // the next draw t >= s + 4 of the class of s + 4 that crosses
-      uint32_t wd = (s + 4) >> 5, r = (s + 4) % 6u;
-      // draws of residue r in word wd: bits k with 32 wd + k = r mod 6
-      uint32_t m = sbits[wd][threadIdx.x] & (0x41041041u << ((r + 4 * wd) % 6u)) &
-                   (~0u << ((s + 4) & 31u));
-      while (!m && ++wd < (uint32_t)kChunkWords)
-        m = sbits[wd][threadIdx.x] & (0x41041041u << ((r + 4 * wd) % 6u));
-      const uint32_t at = m ? 32 * wd + (uint32_t)__ffs((int)m) - 1 - 4 : ~0u;  // that wire's start
-      if (at >= (uint32_t)kChunk) {  // none starts in this chunk
-        const uint32_t k = ((uint32_t)kChunk - 1 - s) / 6 + 1;
-        n += k;
-        s += 6 * k;
-      } else {
-        n += (at - s) / 6 + 1;
-        s = at + 7;
-      }
+  // the state in the upper 48 bits of y: no masking, and compared as it is
+  uint64_t y = chunk_jump(first, threadIdx.x) << 16;
+  const uint64_t crossing = g.crossing << 16;
+  const bool any = g.crossing >> 48 == 0;  // 2^48: no draw crosses
+  uint32_t test[kChunkWords];
+#pragma unroll
+  for (int wd = 0; wd < kChunkWords; wd++) {
+    uint32_t b = 0;
+#pragma unroll
+    for (int k = 0; k < (wd < kChunk / 32 ? 32 : 4); k++) {
+      y = kA * y + (kC << 16);
+      if (y >= crossing) b |= 1u << k;
     }
-    map |= (uint64_t)(n << 3 | (s - (uint32_t)kChunk)) << (9 * q);
+    test[wd] = any ? b : 0u;
+    bits[(int64_t)wd * nchunks + c] = test[wd];
   }
+  uint32_t f[8];  // f(s) at s mod 8; past the end: no wire, exit s - kChunk
+#pragma unroll
+  for (uint32_t j = 0; j < 8; j++) f[j] = j;
+#pragma unroll
+  for (int wd = kChunk / 32 - 1; wd >= 0; wd--) {
+    const uint32_t b = __funnelshift_r(test[wd], test[wd + 1], 4);  // bit k: draw 32 wd + k + 4
+#pragma unroll
+    for (int k = 31; k >= 0; k--)
+      f[k & 7] = ((b >> k) & 1u ? f[(k + 7) & 7] : f[(k + 6) & 7]) + 8u;
+  }
+  uint64_t map = 0;
+#pragma unroll
+  for (int q = 0; q < 7; q++) map |= (uint64_t)f[q] << (9 * q);
   maps[c] = map;
 }
 
@@ -281,7 +281,8 @@ __global__ void __launch_bounds__(1024)
   for (int64_t g0 = 0; g0 < ngroups; g0 += kTopTile) {
     const int n = (int)min((int64_t)kTopTile, ngroups - g0);
     const int len = (n + kTopSegments - 1) / kTopSegments;
-    for (int i = threadIdx.x; i < 7 * n; i += blockDim.x) sm[i] = gmap[g0 * 7 + i];
+#pragma unroll 8
+    for (int i = threadIdx.x; i < 7 * n; i += 1024) sm[i] = gmap[g0 * 7 + i];
     __syncthreads();
     if (threadIdx.x < 7 * kTopSegments) {
       const int q = threadIdx.x % 7, sg = threadIdx.x / 7;
@@ -336,10 +337,11 @@ __global__ void __launch_bounds__(256)
                      const uint64_t *__restrict__ maps, const uint8_t *__restrict__ gphase,
                      const uint64_t *__restrict__ gbase, uint32_t *in_ptr, uint32_t *out_ptr,
                      float *L, float *R, float *C, int32_t *locator, uint32_t *deg,
-                     uint32_t *rank_in, uint32_t *rank_out) {
+                     uint32_t *rank_in, uint32_t *rank_out, Zeroed zero) {
   __shared__ uint64_t smaps[kGroup], state[kGroup], first;
   __shared__ uint32_t sbits[kChunkWords][kGroup], before[kGroup + 1], phase[kGroup];
   __shared__ uint16_t starts[kGroupWires];  // chunk << 8 | draw
+  zero_slice(zero, (uint64_t)blockIdx.x * 256 + threadIdx.x, (uint64_t)gridDim.x * 256);
   const int64_t c0 = (int64_t)blockIdx.x * kGroup;
   const uint64_t w0 = gbase[blockIdx.x];
   if (w0 >= (uint64_t)g.W) return;  // the stream is cut for 7 draws a wire
@@ -378,7 +380,8 @@ __global__ void __launch_bounds__(256)
     const uint32_t w = (uint32_t)w0 + i, st = starts[i];
     uint64_t x = near_jump(state[st >> 8], st & 255u);
     const uint64_t xR = next(x), xL = next(x), xC = next(x), xIn = next(x), xPct = next(x);
-    const uint32_t piece = w / (uint32_t)g.wpp;
+    const uint32_t piece =
+        g.wpp == 1 ? w : (uint32_t)__umul64hi(g.wpp_magic, (uint64_t)w);
     float l, c;
     if (!drand::affine_float(xL, g.L, &l))
       l = __double2float_rn(__dadd_rn(__dmul_rn(drand::value(xL), g.L_scale), g.L_off));
@@ -485,7 +488,8 @@ __global__ void __launch_bounds__(256)
     place_kernel(GenArgs g, const uint32_t *__restrict__ in_ptr,
                  const uint32_t *__restrict__ out_ptr, const uint32_t *__restrict__ off,
                  const uint32_t *__restrict__ rank_in, const uint32_t *__restrict__ rank_out,
-                 uint8_t *in_loc, uint8_t *out_loc, uint32_t *tmp) {
+                 uint8_t *in_loc, uint8_t *out_loc, uint32_t *tmp, Zeroed zero) {
+  zero_slice(zero, (uint64_t)blockIdx.x * 256 + threadIdx.x, (uint64_t)gridDim.x * 256);
   const uint32_t w = blockIdx.x * 256 + threadIdx.x;
   if (w >= (uint32_t)g.W) return;
   const uint32_t a = in_ptr[w], b = out_ptr[w], oa = off[a], ob = off[b];
@@ -498,73 +502,91 @@ __global__ void __launch_bounds__(256)
   tmp[(ob & kOffsetMask) + rank_out[w]] = w << 1 | 1u;
 }
 
-// Per node: sort its contributions by (wire, end), then write the entries
-// with their piece-group flags, the wire ends' slots and the flag bits.  A
-// warp takes 32 consecutive nodes: their
-// runs are one contiguous span, staged in shared memory (coalesced in and
-// out), sorted there a node per lane; a span larger than the stage is sorted
-// in place in tmp instead.
-constexpr uint32_t kFinishSpan = 512;  // entries per warp staged in shared memory
+// Per node: its contributions in the order of (wire, end), with their
+// piece-group flags, the wire ends' slots and the flag bits.  A warp takes 32
+// consecutive nodes, whose runs are one contiguous span, staged in shared
+// memory.  A lane takes an entry, not a node: its place is the number of
+// smaller entries in its run; lanes of one run read the same words, so banks
+// hardly conflict (a node per lane, insertion-sorting its run, reads words 8
+// apart).  A span larger than the stage is sorted in place in tmp instead, a
+// node per lane.
+constexpr uint32_t kFinishSpan = 384;  // entries per warp staged (256 on average)
 
 __global__ void __launch_bounds__(256)
     csr_finish_kernel(GenArgs g, const uint32_t *__restrict__ off, uint32_t *tmp, uint32_t *ent,
                       uint32_t *slot_in, uint32_t *slot_out, uint32_t *gstart) {
-  __shared__ uint32_t sbuf[8][kFinishSpan];
+  __shared__ uint32_t sbuf[8][kFinishSpan], sout[8][kFinishSpan], soff[8][33];
+  __shared__ uint32_t sfirst[8][kFinishSpan / 32];  // bit j: entry j opens a run
   const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
   const int64_t x0 = ((int64_t)blockIdx.x * 8 + wp) * 32;
   if (x0 >= g.N) return;
   const int64_t xe = min(g.N, x0 + 32), x = x0 + lane;
-  const uint32_t lo = off[x0] & kOffsetMask, hi = off[xe] & kOffsetMask;
+  const uint32_t b = off[min(x, xe)] & kOffsetMask;
+  const uint32_t lo = __shfl_sync(0xffffffffu, b, 0), hi = off[xe] & kOffsetMask;
   const uint32_t span = hi - lo;
-  const bool staged = span <= kFinishSpan;
-  uint32_t *buf = sbuf[wp];
-  if (staged)
+  // the first wire of a wire's piece
+  auto piece_first = [&g](uint32_t w) {
+    return g.wpp == 1 ? w : (uint32_t)__umul64hi(g.wpp_magic, (uint64_t)w) * (uint32_t)g.wpp;
+  };
+  if (span <= kFinishSpan) {
+    uint32_t *buf = sbuf[wp], *out = sout[wp], *run = soff[wp], *opens = sfirst[wp];
+    run[lane] = b - lo;
+    if (lane == 0) run[32] = span;
+    if (lane < kFinishSpan / 32) opens[lane] = 0;
+#pragma unroll 4
     for (uint32_t j = lane; j < span; j += 32) buf[j] = tmp[lo + j];
-  __syncwarp();
-  if (x < xe) {
-    const uint32_t b = off[x] & kOffsetMask, e = off[x + 1] & kOffsetMask;
-    uint32_t *run = staged ? buf : tmp;    // entry i lives at run[i - rb]
-    const uint32_t rb = staged ? lo : 0u;
-    for (uint32_t i = b + 1; i < e; i++) {
-      const uint32_t v = run[i - rb];
-      uint32_t j = i;
-      while (j > b && run[j - 1 - rb] > v) {
-        run[j - rb] = run[j - 1 - rb];
-        j--;
-      }
-      run[j - rb] = v;
+    __syncwarp();
+    if (run[lane] < run[lane + 1]) atomicOr(opens + (run[lane] >> 5), 1u << (run[lane] & 31u));
+    for (uint32_t j = lane; j < span; j += 32) {
+      uint32_t n = 0;  // the last node whose run starts at or before j
+#pragma unroll
+      for (uint32_t step = 16; step; step >>= 1)
+        if (run[n + step] <= j) n += step;
+      const uint32_t end = run[n + 1], v = buf[j];
+      uint32_t place = run[n];
+#pragma unroll 4
+      for (uint32_t i = place; i < end; i++) place += buf[i] < v ? 1u : 0u;
+      out[place] = v;
     }
-    int64_t last_piece = -1;
-    for (uint32_t i = b; i < e; i++) {
-      const uint32_t v = run[i - rb], w = v >> 1, end = v & 1u;
-      const int64_t piece = w / g.wpp;
-      const uint32_t start = piece != last_piece ? 1u : 0u;
-      last_piece = piece;
-      const uint32_t val = (w << 2) | (end << 1) | start;
-      if (staged) {
-        buf[i - lo] = val;
-      } else {
-        ent[i] = val;
-        if (start) atomicOr(gstart + (i >> 5), 1u << (i & 31));
-      }
-      if (end) slot_out[w] = i;
-      else slot_in[w] = i;
-    }
-  }
-  __syncwarp();
-  if (staged) {
+    __syncwarp();
     for (uint32_t j0 = 0; j0 < span; j0 += 32) {
       const uint32_t j = j0 + lane;
-      const uint32_t val = j < span ? buf[j] : 0u;
-      if (j < span) ent[lo + j] = val;
+      bool start = false;
+      if (j < span) {
+        const uint32_t v = out[j], w = v >> 1;
+        start = ((opens[j0 >> 5] >> lane) & 1u) || out[j - 1] >> 1 < piece_first(w);
+        ent[lo + j] = (w << 2) | ((v & 1u) << 1) | (start ? 1u : 0u);
+        if (v & 1u) slot_out[w] = lo + j;
+        else slot_in[w] = lo + j;
+      }
       // the group-start bits of these 32 entries, into their one or two words
-      const uint32_t m = __ballot_sync(0xffffffffu, (val & 1u) != 0u);
+      const uint32_t m = __ballot_sync(0xffffffffu, start);
       if (lane == 0 && m) {
         const uint32_t i0 = lo + j0, sh = i0 & 31u, wd = i0 >> 5;
         atomicOr(gstart + wd, m << sh);
         if (sh && (m >> (32 - sh))) atomicOr(gstart + wd + 1, m >> (32 - sh));
       }
     }
+    return;
+  }
+  if (x >= xe) return;
+  const uint32_t e = off[x + 1] & kOffsetMask;
+  for (uint32_t i = b + 1; i < e; i++) {
+    const uint32_t v = tmp[i];
+    uint32_t j = i;
+    while (j > b && tmp[j - 1] > v) {
+      tmp[j] = tmp[j - 1];
+      j--;
+    }
+    tmp[j] = v;
+  }
+  for (uint32_t i = b; i < e; i++) {
+    const uint32_t v = tmp[i], w = v >> 1;
+    const bool start = i == b || tmp[i - 1] >> 1 < piece_first(w);
+    ent[i] = (w << 2) | ((v & 1u) << 1) | (start ? 1u : 0u);
+    if (start) atomicOr(gstart + (i >> 5), 1u << (i & 31));
+    if (v & 1u) slot_out[w] = i;
+    else slot_in[w] = i;
   }
 }
 
@@ -601,6 +623,7 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
   g.leak = drand::make_affine((double)0.1f, 0.0);
   g.seed_state = (((uint64_t)p->random_seed & 0xffffffffull) << 16) | 0x330Eull;
   g.W = W; g.N = N;
+  g.wpp_magic = wpp > 1 ? UINT64_MAX / (uint64_t)wpp + 1 : 0;
 
   gen_nodes_kernel<<<grid_for(N), 256, 0, s>>>(g, o->charge, o->node_voltage, o->node_capacitance,
                                               o->node_leakage, o->locator);
@@ -650,12 +673,13 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
       rc = set_error(CKT_ECUDA, "device generator: %s", cudaGetErrorString(e));
   };
 
-  const Zeroed zero = {{reinterpret_cast<uint32_t *>(o->current),
-                        reinterpret_cast<uint32_t *>(o->voltage), deg, o->gstart},
-                       {10 * (uint64_t)W, 9 * (uint64_t)W, (uint64_t)N,
-                        (uint64_t)(2 * W + 31) / 32}};
+  const Zeroed counts = {{deg, o->gstart}, {(uint64_t)N, (uint64_t)(2 * W + 31) / 32}};
+  const Zeroed with_wires = {{reinterpret_cast<uint32_t *>(o->current), nullptr},
+                             {10 * (uint64_t)W, 0}};
+  const Zeroed with_places = {{reinterpret_cast<uint32_t *>(o->voltage), nullptr},
+                              {9 * (uint64_t)W, 0}};
   decode_kernel<<<grid_for(nchunks, kMapsBlock), kMapsBlock, 0, s>>>(g, base, nchunks, bits, maps,
-                                                                    zero);
+                                                                    counts);
   ok(cudaGetLastError());
   group_maps_kernel<<<grid_for(ngroups, 4), 128, 0, s>>>(nchunks, ngroups, maps, gmap);
   ok(cudaGetLastError());
@@ -666,7 +690,7 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
   ok(cudaGetLastError());
   gen_wires_kernel<<<(unsigned)ngroups, 256, 0, s>>>(
       g, base, nchunks, bits, maps, gphase, gbase, o->in_ptr, o->out_ptr, o->inductance,
-      o->resistance, o->capacitance, o->locator, deg, rank_in, rank_out);
+      o->resistance, o->capacitance, o->locator, deg, rank_in, rank_out, with_wires);
   ok(cudaGetLastError());
   scan_blocks_kernel<<<(unsigned)scan_blocks, kScanBlock, 0, s>>>(deg, N, o->off, sums);
   ok(cudaGetLastError());
@@ -675,7 +699,7 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
   scan_add_kernel<<<grid_for(N), 256, 0, s>>>(o->off, N, sums, o->locator);
   ok(cudaGetLastError());
   place_kernel<<<grid_for(W), 256, 0, s>>>(g, o->in_ptr, o->out_ptr, o->off, rank_in, rank_out,
-                                           o->in_loc, o->out_loc, tmp);
+                                           o->in_loc, o->out_loc, tmp, with_places);
   ok(cudaGetLastError());
   csr_finish_kernel<<<grid_for(N), 256, 0, s>>>(g, o->off, tmp, o->ent, o->slot_in, o->slot_out,
                                                 o->gstart);
