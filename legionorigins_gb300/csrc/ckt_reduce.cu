@@ -21,14 +21,20 @@ struct HistArgs {
   uint32_t buckets;
   uint64_t total;      // elements
   uint32_t seed1, seed2;
-  uint64_t mod_magic;  // remainder constant for `buckets` (see hist_key)
+  uint64_t mod_magic;  // remainder constant for `buckets` (see hist_mod)
 };
 
+// r % buckets by Lemire, Kaser and Kurz's direct computation ("Faster
+// Remainder by Direct Computation", 2019): for 32-bit r and d >= 1 with
+// M = floor((2^64 - 1) / d) + 1 (mod 2^64), r % d = high64((M * r mod 2^64) * d).
+__device__ __forceinline__ uint32_t hist_mod(const HistArgs &a, uint32_t r) {
+  const uint64_t p = a.mod_magic * r;
+  const uint64_t low = (p & 0xffffffffull) * a.buckets;
+  return (uint32_t)(((p >> 32) * a.buckets + (low >> 32)) >> 32);
+}
+
 // Key of element e: myrand(start + i) % buckets (reducetest.cc:323-333,
-// 341-344), with start + i = base + e in 32-bit unsigned arithmetic.  The
-// remainder uses Lemire, Kaser and Kurz's direct computation ("Faster
-// Remainder by Direct Computation", 2019): for 32-bit a and d >= 1 with
-// M = floor((2^64 - 1) / d) + 1 (mod 2^64), a % d = high64((M * a mod 2^64) * d).
+// 341-344), with start + i = base + e in 32-bit unsigned arithmetic.
 __device__ __forceinline__ uint32_t hist_key(const HistArgs &a, uint64_t e) {
   const uint32_t ival = a.base + (uint32_t)e;
   uint64_t r = ival;
@@ -37,7 +43,7 @@ __device__ __forceinline__ uint32_t hist_key(const HistArgs &a, uint64_t e) {
     r = (0x5DEECE66Dull * r + 0xBull) & 0xFFFFFFFFFFFFull;
     r ^= ((ival >> j) & 1u) ? a.seed1 : a.seed2;
   }
-  return (uint32_t)__umul64hi(a.mod_magic * (uint32_t)r, (uint64_t)a.buckets);
+  return hist_mod(a, (uint32_t)r);
 }
 
 // The same for elements 2^16 apart: their indices agree in the low 16 bits,
@@ -54,7 +60,7 @@ struct HashColumn {
     uint32_t r = a.base + e;
 #pragma unroll
     for (int j = 0; j < 16; j++) r = (0xDEECE66Du * r + 0xBu) ^ seed[j];
-    return (uint32_t)__umul64hi(a.mod_magic * r, (uint64_t)a.buckets);
+    return hist_mod(a, r);
   }
 };
 
@@ -88,7 +94,8 @@ __global__ void __launch_bounds__(kFoldBlock) fold_smem_kernel(HistArgs a, uint3
 // counters; otherwise two 16-bit counters per word, twice the buckets: the
 // thread whose add takes a counter to 2^15 moves 2^15 to the target, and the
 // block meets every kFoldRound elements per thread, so a counter gets at most
-// 2^14 more adds before that has happened, whatever the keys are.
+// 28 * 1024 more adds before that has happened and stays below 2^16, whatever
+// the keys are.
 //
 // Elements are cut into units: 1024 residues mod 2^16 (a thread each) times a
 // range of rows of 2^16 elements; `parts` ranges, so that 64 * parts units
@@ -97,10 +104,10 @@ __global__ void __launch_bounds__(kFoldBlock) fold_smem_kernel(HistArgs a, uint3
 // Why: the L2 takes about 2.0e11 of these adds a second (0.66 a clock and SM)
 // whatever their addresses, and that bound the global folds; shared memory
 // takes them as fast as the hash gives them (5e11 a second).  2^29 elements
-// on a GB300, 16 rounds of the hash included: 50,000 buckets 1.12 ms (1.31
-// with a seed chosen per element and round), 110,000 1.31, 262,144 1.80,
+// on a GB300, 16 rounds of the hash included: 50,000 buckets 0.91 ms (1.31
+// with a seed chosen per element and round), 110,000 1.07, 262,144 1.77,
 // 524,288 2.13, 1,048,576 2.34 ms; with the folds in L2 2.6 ms each.
-constexpr int kFoldRound = 16;
+constexpr int kFoldRound = 28;
 constexpr uint32_t kFold16Buckets = 115712;  // 226 KB
 // Above this a block's share is too small a part of the buckets.
 constexpr uint32_t kFold16Most = 1u << 20;
@@ -120,11 +127,13 @@ __global__ void __launch_bounds__(kFoldBlock)
     const HashColumn column(a, residue);
     const uint64_t m0 = rows * part / parts, m1 = rows * (part + 1) / parts;
     for (uint64_t m = m0; m < m1; m += kFoldRound) {
+      // this thread's elements of the round: the last row may end before it
+      uint32_t n = (uint32_t)min((uint64_t)kFoldRound, m1 - m);
+      if (((m + n - 1) << 16 | residue) >= a.total) n--;
+      uint32_t e = (uint32_t)(m << 16) | residue;
 #pragma unroll 4
-      for (uint32_t i = 0; i < kFoldRound; i++) {
-        const uint64_t e = (m + i) << 16 | residue;
-        if (m + i >= m1 || e >= a.total) continue;
-        const uint32_t k = column.key(a, (uint32_t)e);
+      for (uint32_t i = 0; i < n; i++, e += 1u << 16) {
+        const uint32_t k = column.key(a, e);
         if (k >= folded) {
           atomicAdd(hist + k, 1u);
         } else if (WIDE) {
