@@ -66,9 +66,9 @@ PCT, SEED, INNER_STEPS, OUTER_LOOPS = 95.0, 12345, 1000, 10
 L_OFFSET, L_SCALE = 0.001, 0.01
 FLOPS_PER_WIRE_STEP = 96  # the reference's own count (apps/circuit/circuit.cc:324)
 # FP32-pipe operations calc_new_currents issues per wire-step in its common
-# path: EXACT 67 plain operations + 10 split-reciprocal quotients by dt (2
-# each) + 19 corrected quotients by R and C (4 each); FAST 48.
-FP32_OPS_PER_WIRE_STEP = {0: 163, 1: 48}
+# path: EXACT 67 plain operations + 29 split-reciprocal quotients by dt, R
+# and C (2 each); FAST 48.
+FP32_OPS_PER_WIRE_STEP = {0: 125, 1: 48}
 CNC_TRAFFIC_PER_WIRE = (103.879424e6 + 21.284608e6) / 1048576  # measured DRAM bytes per wire
 
 

@@ -86,6 +86,13 @@ def make(oracle, state, P, npp, wpp):
         c.L[:] = 4e-6
         c.node_voltage[:] = 0
         c.voltage[:2] = a, 2 * a
+    elif state == "negative":      # divisors of either sign
+        for d in (c.R, c.C):
+            d[some] = -d[some]
+    elif state == "wide_divisors":  # over and past the eligible ranges
+        c.R[:] = np.exp2(rng.uniform(-8.2, 8.2, W))
+        c.C[:] = np.exp2(rng.uniform(-31, 31, W))
+        c.L[:] *= np.exp2(rng.uniform(-25, 5, W)).astype(np.float32)
     elif state == "overflow":      # blows up within the first blocks
         c.L[:] = rng.uniform(1e-5, 1e-3, W)
     elif state == "nan_wires":     # all-NaN wires beside finite ones
@@ -96,7 +103,8 @@ def make(oracle, state, P, npp, wpp):
 
 
 STATES = ["stable", "zeros", "signed_zeros", "tiny", "tiny_voltages", "equilibrium",
-          "unchecked_R", "unchecked_C", "moved", "near_ties", "overflow", "nan_wires", "nan_node"]
+          "unchecked_R", "unchecked_C", "moved", "near_ties", "negative", "wide_divisors",
+          "overflow", "nan_wires", "nan_node"]
 
 
 @pytest.mark.parametrize("shape", [(1, 3, 1), (3, 100, 701), (61, 300, 1201)],
