@@ -53,17 +53,19 @@ typedef enum {
   /* IEEE fp32 exactly as the reference writes it (correctly rounded
    * divides, no contraction): bit-identical to the reference CPU task.  Its
    * divisors (dt, R, C) are loop-invariant, so each wire carries their
-   * reciprocals and every quotient is formed from them and corrected to the
-   * IEEE quotient (Markstein's theorem); dividends where that construction
-   * is not proven exact, and wires whose divisors lie outside its range, use
-   * the divide routine.  Two wires per thread, paired FP32 instructions. */
+   * reciprocals in two parts, checked to round every quotient as division
+   * does, or corrected to the IEEE quotient (Markstein's theorem); dividends
+   * where neither is proven exact, and wires whose divisors lie outside the
+   * range, use the divide routine.  Two wires per thread on paired FP32
+   * instructions, one wire per thread or five lanes per wire in smaller
+   * launches. */
   CKT_MODE_EXACT = 0,
   /* Loop-invariant quotients L/dt, 1/R and dt/C hoisted out of the inner
    * loop, each current carried before its 1/R scale, fused multiply-adds:
    * 48 FP32 operations per wire-step, within 1e-5 relative of EXACT in the
    * finite regime and with its NaN/Inf classes.  Issued as paired FP32
-   * instructions (two wires per instruction in the per-piece and
-   * index-space kernels, two segments in the batched kernel). */
+   * instructions (two wires per instruction, or two segments in small
+   * launches and the batched kernel's one-wire tiles). */
   CKT_MODE_FAST = 1,
   /* FAST arithmetic issued one operation per instruction: bit-identical to
    * CKT_MODE_FAST (kept to check the paired forms and to measure them). */
@@ -571,8 +573,10 @@ typedef enum {
   /* redfold (:378-400): a fold instance per thread block, initialised to the
    * identity, receives the block's reductions and is then applied to the
    * target.  The fold lives in shared memory when buckets <=
-   * CKT_HIST_SMEM_FOLD_BUCKETS, otherwise in a few L2-resident copies in the
-   * scratch buffer. */
+   * CKT_HIST_SMEM_FOLD_BUCKETS; up to 2^20 buckets and from 2^23 elements
+   * shared memory holds the first buckets' fold (16-bit counters) and the
+   * others reduce straight into the target; otherwise the fold is a few
+   * L2-resident copies in the scratch buffer. */
   CKT_RED_FOLD = 1,
   /* localize (:351-375): the owner of a range of buckets copies that range
    * of the target into its shared memory, applies every reduction that falls
