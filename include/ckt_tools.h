@@ -65,6 +65,9 @@ int ckt_check_wide_quotient(uint64_t seed, uint64_t count, int32_t divisor,
  * (device memory, 4 x uint64). */
 int ckt_check_split_quotient(uint64_t seed, uint64_t count, int32_t divisor,
                              unsigned long long *counts, void *stream);
+/* The same for the split quotient with a truncated product. */
+int ckt_check_cut_quotient(uint64_t seed, uint64_t count, int32_t divisor,
+                           unsigned long long *counts, void *stream);
 
 #ifdef __cplusplus
 }

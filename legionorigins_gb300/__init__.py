@@ -221,6 +221,7 @@ TOOLS_SIGNATURES = {
                                                 _P]),
     "ckt_check_wide_quotient": (ctypes.c_int, [ctypes.c_uint64, ctypes.c_uint64, _I32, _P, _P]),
     "ckt_check_split_quotient": (ctypes.c_int, [ctypes.c_uint64, ctypes.c_uint64, _I32, _P, _P]),
+    "ckt_check_cut_quotient": (ctypes.c_int, [ctypes.c_uint64, ctypes.c_uint64, _I32, _P, _P]),
 }
 
 _lib = None

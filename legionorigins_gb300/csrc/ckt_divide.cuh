@@ -71,8 +71,22 @@
 //    moving yl by one ulp up or down cures 95% of those.  The moved sum is off
 //    by less than 2.5 2^-48, so its candidates are A < B with |r| in {1, 3}
 //    and A >= B with |r| = 1, all tried.  A divisor that stays unchecked
-//    (0.06%) keeps the corrected quotient.  The bound needs RN(a*yl) normal:
-//    |a| >= kSplitLo (|yl| is 0 or at least 2^-48 / |b|, and |b| <= 2^30).
+//    (0.06%) keeps the corrected quotient, or takes the next form.  The bound
+//    needs RN(a*yl) normal: |a| >= kSplitLo (|yl| is 0 or at least
+//    2^-48 / |b|, and |b| <= 2^30).
+//
+//  * The same with the product rounded toward zero (cut_yl):
+//        q = RN(a*y + RZ(a*yl)).
+//    Other divisors fail here than above: with yl as made or one ulp larger
+//    in magnitude 99.8% pass, and all of those left unchecked above that were
+//    tried (2,000).  A warp's lanes share one form, so a warp with an
+//    unchecked divisor takes this one if all its divisors pass.  With
+//    |yl| <= 2^-25 the truncation is below 2^-48 and the sum is off a/b by
+//    less than 2.5 2^-48 (1.5 2^-48 as made), so the dividends to try are
+//    those with |r| < 5 for A < B and |r| < 2.5 for A >= B.  r has B's power
+//    of two, 2^k, as a factor and is odd beyond it; with B = 2^k B' they are
+//    A = +-2^(k-25) and +-3 2^(k-25) mod B' (A < B), +-2^(k-24) mod B'
+//    (A >= B), and none from k = 3 on.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -253,6 +267,69 @@ __device__ __forceinline__ uint32_t check_split(const float (&nb)[N], const floa
     fail ^= bit;
   }
   return right;
+}
+
+// a / b with cut_yl's yl: the split quotient with its product truncated.
+__device__ __forceinline__ float cut_quot(float a, const Recip &k) {
+  return __fmaf_rn(a, k.y, __fmul_rz(a, k.yl));
+}
+__device__ __forceinline__ float2 cut_quot2(float2 a, const Recip2 &k) {
+  return __ffma2_rn(a, k.y, __fmul2_rz(a, k.yl));
+}
+// yl for which cut_quot is RN(a/b) for every dividend of split_quot's range;
+// NaN if neither yl as made nor the next larger in magnitude is.  Out of
+// line: 8% of paired warps call it, once.
+static __device__ __noinline__ float cut_yl(float b) {
+  const float none = __int_as_float(0x7fffffff);
+  if (!(fabsf(b) >= kSplitMin)) return none;
+  const Recip k = make_recip(b);
+  const uint32_t bits = __float_as_uint(b), B = (bits & 0x7fffffu) | 0x800000u;
+  const uint32_t twos = __ffs((int)B) - 1;
+  if (twos > 2u) return k.yl;
+  const float scale = __uint_as_float(bits & 0xff800000u);
+  Recip n = {-__uint_as_float(0x3f800000u | (bits & 0x7fffffu)), __fmul_rn(k.y, scale),
+             __fmul_rn(k.yl, scale)};
+  const uint32_t Bo = B >> twos, e = 25u - twos;
+  uint32_t x = (3u * Bo) ^ 2u;  // as split_base
+  x *= 2u - Bo * x;
+  x *= 2u - Bo * x;
+  x *= 2u - Bo * x;
+  const uint32_t t = (0u - x) & ((1u << e) - 1u);
+  const uint32_t A1 = (uint32_t)((1ull + (uint64_t)Bo * t) >> e);  // 2^(k-25) mod B'
+  const uint32_t A2 = 2u * A1 >= Bo ? 2u * A1 - Bo : 2u * A1;
+  const uint32_t A3 = A1 + A2 >= Bo ? A1 + A2 - Bo : A1 + A2;
+  // the members of those classes in [2^23, 2^24) (others are no dividends)
+  const bool k0 = twos == 0u, k1 = twos == 1u;
+  const uint32_t A[6] = {k0 ? max(A1, Bo - A1) : (k1 ? A1 + Bo : A1 + 2u * Bo),
+                         k0 ? max(A3, Bo - A3) : (k1 ? 2u * Bo - A1 : A1 + 3u * Bo),
+                         k0 ? Bo + A2 : (k1 ? A2 + 2u * Bo : 3u * Bo - A1),
+                         k0 ? 2u * Bo - A2 : (k1 ? 3u * Bo - A2 : 4u * Bo - A1),
+                         k1 ? A2 + 3u * Bo : 0u,
+                         k1 ? 4u * Bo - A2 : 0u};
+#pragma unroll 1
+  for (int d = 0; d < 2; d++) {
+    const Recip m = {n.nb, n.y, __int_as_float(__float_as_int(n.yl) + d)};
+    bool right = fabsf(m.yl) <= 0x1p-25f;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      const float a = __fmul_rn(__uint2float_rn(A[i]), 0x1p-23f);
+      right &= (A[i] - 0x800000u >= 0x800000u) | (cut_quot(a, m) == recip_quot(a, n));
+    }
+    if (right) return __int_as_float(__float_as_int(k.yl) + d);
+  }
+  return none;
+}
+
+// The quotient of a free step.
+enum QuotForm : uint32_t { kCorrected, kSplit, kCut };
+template <QuotForm FORM>
+__device__ __forceinline__ float free_quot(float a, const Recip &k) {
+  return FORM == kCut ? cut_quot(a, k) : (FORM == kSplit ? split_quot(a, k) : recip_quot(a, k));
+}
+template <QuotForm FORM>
+__device__ __forceinline__ float2 free_quot2(float2 a, const Recip2 &k) {
+  return FORM == kCut ? cut_quot2(a, k)
+                      : (FORM == kSplit ? split_quot2(a, k) : recip_quot2(a, k));
 }
 
 // True for a nonzero |a| below tiny (NaN: false).

@@ -331,11 +331,15 @@ struct DualExact {
     kC.yl = make_float2(yl[2], yl[3]);
     return ((right & 3u) == 3u ? 1u : 0u) | (right >= 12u ? 2u : 0u);
   }
-  // step() without guards and branches.  SPLIT bit 0 (1): the quotients by R
-  // (C) are split quotients (2 operations), otherwise corrected ones (4).
+  static __device__ __forceinline__ float2 cut(const Recip2 &k) {
+    return make_float2(cut_yl(-k.nb.x), cut_yl(-k.nb.y));
+  }
+  // step() without guards and branches.  FR, FC: the form of the quotients by
+  // R and C: split, with a rounded or a truncated product (2 operations), or
+  // corrected (4).
   // LOW: low collects the least |dividend| of
   // R and C (NaN ones apart).  exact_steps says when the result is step()'s.
-  template <uint32_t SPLIT, bool LOW>
+  template <QuotForm FR, QuotForm FC, bool LOW>
   __device__ __forceinline__ void step_free(float2 (&ni)[10], float2 (&nv)[11],
                                             const float2 (&nI0)[10], const float2 (&V0)[9],
                                             float &low) const {
@@ -344,13 +348,13 @@ struct DualExact {
       const float2 a1 = __fmul2_rn(L, __fadd2_rn(ni[k], nI0[k]));
       const float2 a2 = sub2(sub2(nv[k + 1], nv[k]), dt_div(a1));
       if (LOW) low = min_abs(low, a2.x, a2.y);
-      ni[k] = SPLIT & 1u ? split_quot2(a2, kR) : recip_quot2(a2, kR);
+      ni[k] = free_quot2<FR>(a2, kR);
     }
 #pragma unroll
     for (int k = 0; k < 9; k++) {
       const float2 a3 = __fmul2_rn(dt2, sub2(ni[k], ni[k + 1]));
       if (LOW) low = min_abs(low, a3.x, a3.y);
-      nv[k + 1] = __fadd2_rn(V0[k], SPLIT & 2u ? split_quot2(a3, kC) : recip_quot2(a3, kC));
+      nv[k + 1] = __fadd2_rn(V0[k], free_quot2<FC>(a3, kC));
     }
   }
   // The same with every zero and infinite dividend's quotient as well: a * y.
@@ -470,8 +474,8 @@ struct DualExact {
 //    the currents beside it.  So a wire's state that holds no NaN at the end
 //    was right throughout; one that was all NaN at the start stays so.
 //  * Tiny dividends and zeros.  Both quotients are right for |a| >= 2^-77 |b|
-//    (split: RN(a yl) is normal, |yl| >= 2^-48 / |b|; corrected: the remainder
-//    is representable, |b| >= 2^-20).  Below that the true quotient and the
+//    (split: a yl, rounded or truncated, is normal, |yl| >= 2^-48 / |b|;
+//    corrected: the remainder is representable, |b| >= 2^-20).  Below that the true quotient and the
 //    computed one are both at most 2^-76 -- the wrong bits, or a zero of the
 //    wrong sign, of something that small.  A block of LOW steps fails when it
 //    met a dividend below kSplitLo (corrected: kCLo).  Steps without LOW need
@@ -526,7 +530,20 @@ constexpr int kSavedState = 23;
 // from finite values, 107 and 208 us from the generated state; 32 steps 192
 // and 153, 164 and 143 us.
 constexpr int kFreeSteps = 32;
-
+// The quotient forms of a warp's free steps.  8% of paired warps hold a divisor
+// that check_split leaves unchecked; with corrected quotients by R (C) such a
+// warp's steps are 16% (14%) longer, and a small launch takes as long as its
+// slowest warp.  So those warps try truncated products, which all but 7% (solo;
+// paired 14%) of them can take; the trial costs them about 3 steps.  us per
+// 1000 steps, GB300, before / with it / with no divisor unchecked: 1024 wires
+// 61 / 57 / 55, 4096 68 / 64 / 63, 16,000 104 / 97..118 / 90 (a corrected warp
+// left or not), 124,867 521 / 508 / 494, 262,144 1021 / 991 / 935, 4,194,304
+// 14439 / 14127 / 14010.
+// Corrected quotients remain for C alone (divisors below kSplitMin) or for both.
+__device__ __forceinline__ void normalize_forms(QuotForm &FR, QuotForm &FC) {
+  const bool mixed = (FR == kCorrected) != (FC == kCorrected);
+  if (FR == kCorrected || (mixed && FR == kCut)) FR = FC = kCorrected;
+}
 template <int STRIDE, typename F>
 __device__ __forceinline__ void save_state(F *save, const F (&ni)[10], const F (&nv)[11]) {
 #pragma unroll
@@ -550,7 +567,7 @@ template <int STRIDE, typename Stepper, typename Wires, typename F>
 __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&ni)[10],
                                             F (&nv)[11], F *save) {
   const uint32_t lanes = __activemask();
-  uint32_t split;
+  QuotForm FR, FC;  // of the warp
   bool sound;
   CarefulForm how;
   // careful: blocks before the next try of sound ones; skip: careful blocks
@@ -562,12 +579,28 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
   {
     Stepper pk = wires.template stepper<Stepper>();
     const uint32_t checked = pk.check();
-    split = (__all_sync(lanes, checked & 1u) ? 1u : 0u) | (__all_sync(lanes, checked & 2u) ? 2u : 0u);
+    FR = __all_sync(lanes, checked & 1u) ? kSplit : kCorrected;
+    FC = __all_sync(lanes, checked & 2u) ? kSplit : kCorrected;
+    if (FR == kCorrected) {
+      const F yl = Stepper::cut(pk.kR);
+      if (__all_sync(lanes, !nan_bits(yl))) {
+        FR = kCut;
+        pk.kR.yl = yl;
+      }
+    }
+    if (FC == kCorrected) {
+      const F yl = Stepper::cut(pk.kC);
+      if (__all_sync(lanes, !nan_bits(yl))) {
+        FC = kCut;
+        pk.kC.yl = yl;
+      }
+    }
+    normalize_forms(FR, FC);
     F nI0[10], V0[9];
     wires.load(nI0, V0);
     sound = __all_sync(lanes, pk.sound(nI0, V0));
     skip = sound ? 0 : 1;
-    how = split == 3u && __all_sync(lanes, pk.can_wide(nI0)) ? kWide : kLow;
+    how = FR == kSplit && FC == kSplit && __all_sync(lanes, pk.can_wide(nI0)) ? kWide : kLow;
     save[21 * STRIDE] = pk.kR.yl;
     save[22 * STRIDE] = pk.kC.yl;
   }
@@ -593,18 +626,39 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
         const int n = min(run, steps - j);
         // one loop per pair of quotient forms: a warp with one unchecked
         // divisor (8% of paired warps) keeps the other's split quotients
-        if (split == 3u) {
+        // A loop per pair of forms, the usual one last (as a chain of ifs or
+        // with it first the loops' code differs by 1 to 4% either way).
+        switch (FR * 3 + FC) {
+          case kCut * 3 + kSplit:
 #pragma unroll 1
-          for (int i = 0; i < n; i++) pk.template step_free<3, false>(ni, nv, nI0, V0, none);
-        } else if (split == 2u) {
+            for (int i = 0; i < n; i++)
+              pk.template step_free<kCut, kSplit, false>(ni, nv, nI0, V0, none);
+            break;
+          case kSplit * 3 + kCut:
 #pragma unroll 1
-          for (int i = 0; i < n; i++) pk.template step_free<2, false>(ni, nv, nI0, V0, none);
-        } else if (split == 1u) {
+            for (int i = 0; i < n; i++)
+              pk.template step_free<kSplit, kCut, false>(ni, nv, nI0, V0, none);
+            break;
+          case kCut * 3 + kCut:
 #pragma unroll 1
-          for (int i = 0; i < n; i++) pk.template step_free<1, false>(ni, nv, nI0, V0, none);
-        } else {
+            for (int i = 0; i < n; i++)
+              pk.template step_free<kCut, kCut, false>(ni, nv, nI0, V0, none);
+            break;
+          case kSplit * 3 + kCorrected:
 #pragma unroll 1
-          for (int i = 0; i < n; i++) pk.template step_free<0, false>(ni, nv, nI0, V0, none);
+            for (int i = 0; i < n; i++)
+              pk.template step_free<kSplit, kCorrected, false>(ni, nv, nI0, V0, none);
+            break;
+          case kCorrected * 3 + kCorrected:
+#pragma unroll 1
+            for (int i = 0; i < n; i++)
+              pk.template step_free<kCorrected, kCorrected, false>(ni, nv, nI0, V0, none);
+            break;
+          default:
+#pragma unroll 1
+            for (int i = 0; i < n; i++)
+              pk.template step_free<kSplit, kSplit, false>(ni, nv, nI0, V0, none);
+            break;
         }
         right = (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
         if (j + n == steps) right &= Stepper::least_current(ni) >= 0x1p-75f;
@@ -758,7 +812,8 @@ struct SoloExact {
     kC.yl = yl[1];
     return right;
   }
-  template <uint32_t SPLIT, bool LOW>
+  static __device__ __forceinline__ float cut(const Recip &k) { return cut_yl(-k.nb); }
+  template <QuotForm FR, QuotForm FC, bool LOW>
   __device__ __forceinline__ void step_free(float (&ni)[10], float (&nv)[11],
                                             const float (&I0)[10], const float (&V0)[9],
                                             float &low) const {
@@ -767,7 +822,7 @@ struct SoloExact {
     for (int k = 0; k < 10; k++) {
       const float a1 = __fmul_rn(L, __fsub_rn(ni[k], I0[k]));
       a[k] = __fsub_rn(__fsub_rn(nv[k + 1], nv[k]), dt_quot(a1));
-      ni[k] = SPLIT & 1u ? split_quot(a[k], kR) : recip_quot(a[k], kR);
+      ni[k] = free_quot<FR>(a[k], kR);
     }
 #pragma unroll
     for (int k = 0; k < 10; k += 2)
@@ -775,7 +830,7 @@ struct SoloExact {
 #pragma unroll
     for (int k = 0; k < 9; k++) {
       a[k] = __fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1]));
-      nv[k + 1] = __fadd_rn(V0[k], SPLIT & 2u ? split_quot(a[k], kC) : recip_quot(a[k], kC));
+      nv[k + 1] = __fadd_rn(V0[k], free_quot<FC>(a[k], kC));
     }
 #pragma unroll
     for (int k = 0; k < 8; k += 2)
@@ -907,7 +962,7 @@ __device__ __noinline__ bool careful_steps(const Wires wires, int n, CarefulForm
   } else if (how == kLow) {
     float low = __int_as_float(0x7f800000);
 #pragma unroll 1
-    for (int i = 0; i < n; i++) pk.template step_free<0, true>(ni, nv, nI0, V0, low);
+    for (int i = 0; i < n; i++) pk.template step_free<kCorrected, kCorrected, true>(ni, nv, nI0, V0, low);
     right = low >= kCLo && (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
   }
   right = __all_sync(lanes, right);
@@ -1222,21 +1277,21 @@ struct LaneWire {
   int left, right;  // lanes of the neighbours (the lane itself at the wire's ends)
   bool first, last, okR, okC;  // okR, okC: eligible divisors (divisor_ok)
 
-  // SPLIT, LOW: as DualExact::step_free.  The voltages at the wire's ends
+  // FR, FC, LOW: as DualExact::step_free.  The voltages at the wire's ends
   // stay: V + a * 0.
-  template <uint32_t SPLIT, bool LOW>
+  template <QuotForm FR, QuotForm FC, bool LOW>
   __device__ __forceinline__ void step_free(LaneState &s, float &low) const {
     const float2 neg1 = make_float2(-1.0f, -1.0f);
     const float2 a1 = __fmul2_rn(make_float2(L, L), __fadd2_rn(s.x, nX0));
     const float2 a2 =
         __ffma2_rn(dt_quot2(a1), neg1, __fadd2_rn(s.e, make_float2(s.nb, s.nb)));
-    s.x = SPLIT & 1u ? split_quot2(a2, R) : recip_quot2(a2, R);
+    s.x = free_quot2<FR>(a2, R);
     const float l = __shfl_sync(0xffffffffu, s.x.y, left);
     const float r = __shfl_sync(0xffffffffu, s.x.x, right);
     const float a3 = __fmul_rn(dt, __fadd_rn(s.x.x, s.x.y));
-    s.nb = __fadd_rn(nVb, SPLIT & 2u ? split_quot(a3, C) : recip_quot(a3, C));
+    s.nb = __fadd_rn(nVb, free_quot<FC>(a3, C));
     const float2 ae = __fmul2_rn(make_float2(dt, dt), __fadd2_rn(make_float2(l, r), s.x));
-    s.e = __fadd2_rn(Ve, SPLIT & 2u ? split_quot2(ae, E) : recip_quot2(ae, E));
+    s.e = __fadd2_rn(Ve, free_quot2<FC>(ae, E));
     if (LOW) {
       low = min_abs(low, a2.x, a2.y);
       low = min_abs(low, a3, first ? 1.0f : ae.x);
@@ -1280,10 +1335,10 @@ struct LaneWire {
     if (!first) s.e.x = __fadd_rn(Ve.x, any_quot(da, C, okC, kCLo, kCHi));
     if (!last) s.e.y = __fadd_rn(Ve.y, any_quot(dc, C, okC, kCLo, kCHi));
   }
-  template <uint32_t SPLIT, bool LOW>
+  template <QuotForm FR, QuotForm FC, bool LOW>
   __device__ __forceinline__ void steps_free(LaneState &s, int n, float &low) const {
 #pragma unroll 4
-    for (int i = 0; i < n; i++) step_free<SPLIT, LOW>(s, low);
+    for (int i = 0; i < n; i++) step_free<FR, FC, LOW>(s, low);
   }
 };
 
@@ -1325,7 +1380,7 @@ __global__ void __launch_bounds__(32)
   x.okR = divisor_ok(r, kRMin, kRMax);
   x.okC = divisor_ok(c, kCMin, kCMax);
 
-  uint32_t split = 0;
+  QuotForm FR = kCorrected, FC = kCorrected;
   bool sound = false, wide = false;
   const bool eligible = __all_sync(kAll, x.okR && x.okC);
   if (eligible) {
@@ -1334,12 +1389,28 @@ __global__ void __launch_bounds__(32)
     const uint32_t checked = check_split(nb, y, yl);
     x.R.yl = make_float2(yl[0], yl[0]);
     x.C.yl = yl[1];
-    split = (__all_sync(kAll, checked & 1u) ? 1u : 0u) | (__all_sync(kAll, checked & 2u) ? 2u : 0u);
+    FR = __all_sync(kAll, checked & 1u) ? kSplit : kCorrected;
+    FC = __all_sync(kAll, checked & 2u) ? kSplit : kCorrected;
+    if (FR == kCorrected) {
+      const float cut = cut_yl(r);
+      if (__all_sync(kAll, cut == cut)) {
+        FR = kCut;
+        x.R.yl = make_float2(cut, cut);
+      }
+    }
+    if (FC == kCorrected) {
+      const float cut = cut_yl(c);
+      if (__all_sync(kAll, cut == cut)) {
+        FC = kCut;
+        x.C.yl = cut;
+      }
+    }
+    normalize_forms(FR, FC);
     sound = __all_sync(kAll, sound_wire(fminf(fabsf(I0), fabsf(I1)),
                                         min_abs(fabsf(x.nVb), x.first ? 1.0f : x.Ve.x,
                                                 x.last ? 1.0f : x.Ve.y),
                                         x.L, c, dt));
-    wide = split == 3u &&
+    wide = FR == kSplit && FC == kSplit &&
            __all_sync(kAll, wide_wire(min(order(I0), order(I1)), x.L, c));
   }
   x.E.nb = make_float2(x.C.nb, x.C.nb);
@@ -1358,7 +1429,7 @@ __global__ void __launch_bounds__(32)
     const bool exempt = !mine || (nan & wire_lanes) == wire_lanes;
     float low = __int_as_float(0x7f800000);
     if (nan == kAll) {  // stays so: any form of quotient gives NaN, nothing to check
-      x.steps_free<3, false>(s, steps - j, low);
+      x.steps_free<kSplit, kSplit, false>(s, steps - j, low);
       break;
     }
     auto holds_nan = [&s]() {
@@ -1368,10 +1439,12 @@ __global__ void __launch_bounds__(32)
     const LaneState start = s;
     if (sound && careful == 0) {
       const int n = min(run, steps - j);
-      if (split == 3u) x.steps_free<3, false>(s, n, low);
-      else if (split == 2u) x.steps_free<2, false>(s, n, low);
-      else if (split == 1u) x.steps_free<1, false>(s, n, low);
-      else x.steps_free<0, false>(s, n, low);
+      if (FR == kSplit && FC == kSplit) x.steps_free<kSplit, kSplit, false>(s, n, low);
+      else if (FR == kCut && FC == kSplit) x.steps_free<kCut, kSplit, false>(s, n, low);
+      else if (FR == kSplit && FC == kCut) x.steps_free<kSplit, kCut, false>(s, n, low);
+      else if (FR == kCut && FC == kCut) x.steps_free<kCut, kCut, false>(s, n, low);
+      else if (FR == kSplit && FC == kCorrected) x.steps_free<kSplit, kCorrected, false>(s, n, low);
+      else x.steps_free<kCorrected, kCorrected, false>(s, n, low);
       bool right = !holds_nan();
       if (j + n == steps) right &= fminf(fabsf(s.x.x), fabsf(s.x.y)) >= 0x1p-75f;
       if (__all_sync(kAll, right || exempt)) {
@@ -1395,7 +1468,7 @@ __global__ void __launch_bounds__(32)
         for (int i = 0; i < n; i++) x.step_wide(s, lowR, lowC);
         right &= lowR >= order(0x1p-66f) && lowC >= order(__fmul_rn(0x1p-77f, fabsf(c)));
       } else {
-        x.steps_free<0, true>(s, n, low);
+        x.steps_free<kCorrected, kCorrected, true>(s, n, low);
         right = low >= kCLo && !holds_nan();
       }
       right = __all_sync(kAll, right || exempt);

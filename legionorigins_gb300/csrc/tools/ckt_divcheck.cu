@@ -194,7 +194,10 @@ __global__ void __launch_bounds__(256)
 // The split quotient by a checked divisor (check_split) against the divide
 // routine: dividends that come nearest to a rounding boundary (the residues
 // r 2^-25 mod B and r 2^-24 mod B, r odd and small, above and below B) and
-// random ones, at any exponent the quotient is used for.
+// random ones, at any exponent the quotient is used for.  CUT: the form with
+// a truncated product (cut_yl); for B = 2^k B' the residues are r 2^(k-25) and
+// r 2^(k-24) mod B'.
+template <bool CUT>
 __global__ void __launch_bounds__(256)
     split_quotient_check_kernel(uint64_t seed, uint64_t count, int32_t divisor,
                                 unsigned long long *counts) {
@@ -213,18 +216,24 @@ __global__ void __launch_bounds__(256)
     const float nb[1] = {made.nb}, y[1] = {made.y};
     float yl[1] = {made.yl};
     drawn++;
-    if (!check_split(nb, y, yl)) continue;
+    if (CUT) yl[0] = cut_yl(b);
+    if (CUT ? yl[0] != yl[0] : !check_split(nb, y, yl)) continue;
     checked++;
     moved += yl[0] != made.yl;
     const Recip k = {made.nb, made.y, yl[0]};
     const uint32_t B = (__float_as_uint(b) & 0x7fffffu) | 0x800000u;
-    uint64_t A1 = 1;  // 2^-25 mod B for odd B, by halving
-    for (int q = 0; q < 25; q++) A1 = (A1 & 1u) ? (A1 + B) / 2 : A1 / 2;
+    const uint32_t twos = CUT ? __ffs((int)B) - 1 : 0, Bo = B >> twos;
+    uint64_t A1 = 1;  // 2^(k-25) mod B' (2^-25 mod B for odd B), by halving
+    for (uint32_t q = twos; q < 25; q++) A1 = (A1 & 1u) ? (A1 + Bo) / 2 : A1 / 2;
     for (uint32_t d = 0; d < 24; d++) {
       const uint32_t odd = 2u * (d % 6u) + 1u;
-      uint32_t A = (uint32_t)((odd * A1 * (d < 12 ? 1u : 2u)) % B);
-      if (d % 12u >= 6u) A = B - A;
-      if (d >= 12) A += B;
+      uint32_t A = (uint32_t)((odd * A1 * (d < 12 ? 1u : 2u)) % Bo);
+      if (d % 12u >= 6u) A = Bo - A;
+      if (!CUT && d >= 12) A += B;
+      if (CUT && A < 0x800000u) {  // any of the class in [2^23, 2^24)
+        A += (0x800000u - A + Bo - 1u) / Bo * Bo;
+        A += (uint32_t)(mix64(h1 + d) % ((0xffffffu - min(A, 0xffffffu)) / Bo + 1u)) * Bo;
+      }
       if (A < 0x800000u || A > 0xffffffu)
         A = 0x800000u | ((uint32_t)(mix64(h2 + d) >> 11) & 0x7fffffu);
       // 2^-77 |b| <= |a| < 2^127
@@ -232,7 +241,7 @@ __global__ void __launch_bounds__(256)
       const int e = lo + (int)((uint32_t)(mix64(h2 ^ d) >> 40) % (uint32_t)(127 - lo));
       const float a = ((h2 >> d) & 1u ? -1.0f : 1.0f) *
                       __uint_as_float((uint32_t)(e + 127) << 23 | (A & 0x7fffffu));
-      bad += !same_float(split_quot(a, k), __fdiv_rn(a, b));
+      bad += !same_float(CUT ? cut_quot(a, k) : split_quot(a, k), __fdiv_rn(a, b));
     }
   }
   warp_add(counts + 0, bad);
@@ -245,8 +254,9 @@ __global__ void __launch_bounds__(256)
 
 using namespace ckt;
 
-extern "C" int ckt_check_split_quotient(uint64_t seed, uint64_t count, int32_t divisor,
-                                        unsigned long long *counts, void *stream) {
+template <bool CUT>
+static int check_split_quotient(uint64_t seed, uint64_t count, int32_t divisor,
+                                unsigned long long *counts, void *stream) {
   CKT_REQUIRE(counts != nullptr, "counts is NULL");
   CKT_REQUIRE(divisor == 0 || divisor == 1, "divisor must be 0 (R) or 1 (C), got %d", divisor);
   if (count == 0) return CKT_OK;
@@ -255,9 +265,20 @@ extern "C" int ckt_check_split_quotient(uint64_t seed, uint64_t count, int32_t d
   CKT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const uint64_t want = (count + 255) / 256;
   const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)sms * 8);
-  split_quotient_check_kernel<<<grid, 256, 0, as_stream(stream)>>>(seed, count, divisor, counts);
+  split_quotient_check_kernel<CUT>
+      <<<grid, 256, 0, as_stream(stream)>>>(seed, count, divisor, counts);
   CKT_CHECK_LAUNCH();
   return CKT_OK;
+}
+
+extern "C" int ckt_check_split_quotient(uint64_t seed, uint64_t count, int32_t divisor,
+                                        unsigned long long *counts, void *stream) {
+  return check_split_quotient<false>(seed, count, divisor, counts, stream);
+}
+
+extern "C" int ckt_check_cut_quotient(uint64_t seed, uint64_t count, int32_t divisor,
+                                      unsigned long long *counts, void *stream) {
+  return check_split_quotient<true>(seed, count, divisor, counts, stream);
 }
 
 extern "C" int ckt_check_dt_quotient(uint64_t begin, uint64_t count, unsigned long long *counts,

@@ -875,6 +875,60 @@ int ocl_split_divisor(float b, float *y, float *yl)
   return 0;
 }
 
+/* a * b rounded toward zero (their product is exact in double). */
+static float sq_mul_rz(float a, float b)
+{
+  const double p = (double)a * b;
+  float f = (float)p;
+  if (fabs((double)f) > fabs(p)) f = wq_bits(wq_u(f) - 1u);
+  return f;
+}
+
+/* The same with the product truncated: every dividend of [2^23, 2^24) whose
+ * quotient comes as near to a rounding boundary as the error bound. */
+static int sq_cut_right(uint32_t B, float m, float y, float yl)
+{
+  if (fabsf(yl) > 0x1p-25f) return 0;
+  uint32_t Bo = B, k = 0;
+  while (!(Bo & 1u)) Bo >>= 1, k++;
+  if (k > 2) return 1;
+  uint64_t A1 = 1; /* 2^(k-25) mod Bo */
+  for (uint32_t i = 0; i < 25 - k; i++) A1 = (A1 & 1u) ? (A1 + Bo) / 2 : A1 / 2;
+  for (uint32_t f = 1; f <= 3; f++)
+    for (int neg = 0; neg < 2; neg++) {
+      const uint32_t c = (uint32_t)(f * A1 % Bo);
+      for (uint32_t A = neg ? Bo - c : c; A < (1u << 24); A += Bo) {
+        const float a = ldexpf((float)A, -23);
+        if (A >= (1u << 23) && fmaf(a, y, sq_mul_rz(a, yl)) != a / m) return 0;
+      }
+    }
+  return 1;
+}
+
+int ocl_cut_divisor(float b, float *y, float *yl)
+{
+  *y = 1.0f / b;
+  *yl = fmaf(-b, *y, 1.0f) / b;
+  const uint32_t B = (wq_u(b) & 0x7fffffu) | 0x800000u;
+  const float m = ldexpf((float)B, -23), my = 1.0f / m, myl = fmaf(-m, my, 1.0f) / m;
+  if (sq_cut_right(B, m, my, myl)) return 1;
+  if (sq_cut_right(B, m, my, wq_bits(wq_u(myl) + 1u))) {
+    *yl = wq_bits(wq_u(*yl) + 1u);
+    return 2;
+  }
+  return 0;
+}
+
+uint64_t ocl_cut_divisor_sweep(float b, float y, float yl, int exponent)
+{
+  uint64_t bad = 0;
+  for (uint32_t A = 1u << 23; A < 1u << 24; A++) {
+    const float a = ldexpf((float)A, exponent - 23);
+    bad += fmaf(a, y, sq_mul_rz(a, yl)) != a / b;
+  }
+  return bad;
+}
+
 uint64_t ocl_split_divisor_sweep(float b, float y, float yl, int exponent)
 {
   uint64_t bad = 0;

@@ -20,7 +20,7 @@
  *                       reduction-instance fold/apply order of
  *                       runtime/lowlevel.h:475-492 (pieces applied ascending)
  *   ocl_uv_f32/_f64     apps/circuit/circuit.cc:445-460, :1290-1307
- *   ocl_split_quotient_check, ocl_wide_quotient_check, ocl_split_divisor(_sweep)
+ *   ocl_split_quotient_check, ocl_wide_quotient_check, ocl_split_divisor(_sweep), ocl_cut_divisor(_sweep)
  *                       the division by dt of apps/circuit/circuit.cc:391-393
  *                       as the GPU's EXACT mode forms it (split reciprocal),
  *                       against IEEE division, over ranges of dividends
@@ -173,6 +173,10 @@ void ocl_wide_quotient_check(uint64_t seed, uint64_t n, int divisor, uint64_t *b
 int ocl_split_divisor(float b, float *y, float *yl);
 /* Mismatches of it among the 2^23 dividends of one binade. */
 uint64_t ocl_split_divisor_sweep(float b, float y, float yl, int exponent);
+/* The same with the product truncated, fma(a, y, RZ(a * yl)); 2: with yl one
+ * ulp larger in magnitude. */
+int ocl_cut_divisor(float b, float *y, float *yl);
+uint64_t ocl_cut_divisor_sweep(float b, float y, float yl, int exponent);
 
 #ifdef __cplusplus
 }

@@ -126,6 +126,10 @@ def lib():
         L.ocl_split_divisor.restype = i32
         L.ocl_split_divisor_sweep.argtypes = [f32, f32, f32, i32]
         L.ocl_split_divisor_sweep.restype = u64
+        L.ocl_cut_divisor.argtypes = [f32, P, P]
+        L.ocl_cut_divisor.restype = i32
+        L.ocl_cut_divisor_sweep.argtypes = [f32, f32, f32, i32]
+        L.ocl_cut_divisor_sweep.restype = u64
         _lib = L
     return _lib
 
@@ -408,3 +412,14 @@ def split_divisor(b: float):
 
 def split_divisor_sweep(b: float, y: float, yl: float, exponent: int) -> int:
     return lib().ocl_split_divisor_sweep(b, y, yl, exponent)
+
+
+def cut_divisor(b: float):
+    """As split_divisor, for the product truncated."""
+    y, yl = ctypes.c_float(), ctypes.c_float()
+    v = lib().ocl_cut_divisor(b, ctypes.byref(y), ctypes.byref(yl))
+    return v, y.value, yl.value
+
+
+def cut_divisor_sweep(b: float, y: float, yl: float, exponent: int) -> int:
+    return lib().ocl_cut_divisor_sweep(b, y, yl, exponent)
