@@ -1298,21 +1298,22 @@ struct LaneWire {
       low = fminf(low, last ? 1.0f : fabsf(ae.y));
     }
   }
-  // As DualExact::step_wide.
+  // As DualExact::step_wide, on the values themselves: a difference of
+  // negated values has the other sign only where it is not zero.
   __device__ __forceinline__ void step_wide(LaneState &s, uint32_t &lowR, uint32_t &lowC) const {
-    const float2 neg1 = make_float2(-1.0f, -1.0f);
-    const float2 a1 = __fmul2_rn(make_float2(L, L), __fadd2_rn(s.x, nX0));
-    s.x = DualExact<true>::wide(
-        __ffma2_rn(dt_quot2(a1), neg1, __fadd2_rn(s.e, make_float2(s.nb, s.nb))), R, lowR);
-    const float l = __shfl_sync(0xffffffffu, s.x.y, left);
-    const float r = __shfl_sync(0xffffffffu, s.x.x, right);
-    const float vb =
-        __fadd_rn(-nVb, SoloExact<true>::wide(__fmul_rn(dt, __fsub_rn(-s.x.x, s.x.y)), C, lowC));
-    s.nb = -vb;
+    const float2 i = make_float2(-s.x.x, s.x.y), I0 = make_float2(nX0.x, -nX0.y);
+    const float vb = -s.nb;
+    const float2 a1 = __fmul2_rn(make_float2(L, L), sub2(i, I0));
+    const float2 dv = sub2(make_float2(vb, s.e.y), make_float2(s.e.x, vb));
+    const float2 q = DualExact<true>::wide(sub2(dv, dt_quot2(a1)), R, lowR);
+    const float l = __shfl_sync(0xffffffffu, q.y, left);
+    const float r = __shfl_sync(0xffffffffu, q.x, right);
+    s.x = make_float2(-q.x, q.y);
+    s.nb = -__fadd_rn(-nVb, SoloExact<true>::wide(__fmul_rn(dt, __fsub_rn(q.x, q.y)), C, lowC));
     const float va = __fadd_rn(
-        Ve.x, SoloExact<true>::wide(first ? 1.0f : __fmul_rn(dt, __fadd_rn(l, s.x.x)), C, lowC));
+        Ve.x, SoloExact<true>::wide(first ? 1.0f : __fmul_rn(dt, __fsub_rn(l, q.x)), C, lowC));
     const float vc = __fadd_rn(
-        Ve.y, SoloExact<true>::wide(last ? 1.0f : __fmul_rn(dt, __fadd_rn(s.x.y, r)), C, lowC));
+        Ve.y, SoloExact<true>::wide(last ? 1.0f : __fmul_rn(dt, __fsub_rn(q.y, r)), C, lowC));
     if (!first) s.e.x = va;
     if (!last) s.e.y = vc;
   }
