@@ -81,10 +81,11 @@ static void launch_cnc_t(uint32_t first, uint32_t n, const ckt_wires &w, const f
   // unevenly filled when there are few, and a step then takes as long as its
   // slowest warp.  Same bits in every form (each rounds every operation
   // alike).  us per 1000 steps on a GB300, finite values:
-  //   EXACT  wires       1024  4096  8000  16000  64000  124867  200000  300000
-  //     five lanes/wire    63    76    95    139
-  //     one thread/wire    92   110   112    111    315     518     789    1136
-  //     paired, 128       207   207   209    206    391     628     874    1157
+  //   EXACT  wires       1024  4096  8000  10944  11500  64000  124867  200000  300000
+  //     five lanes/wire    57    64    89     89    108
+  //     one thread/wire    92    96   107    107    107    315     508     789    1136
+  //     paired, 128       160   163   188                   391     609     863    1123
+  //   (from the generated state at 10,944: five lanes 100, one thread 103)
   //   FAST   wires            4096  16000  48000  64000  160000  500000  4194304
   //     one thread/wire         47     48    105    135     276     760
   //     paired, 128             72     72    126    127     287     715     5525
@@ -94,7 +95,7 @@ static void launch_cnc_t(uint32_t first, uint32_t n, const ckt_wires &w, const f
   memcpy(&dt_bits, &p->dt, sizeof(dt_bits));
   if constexpr (M == CKT_MODE_EXACT) {
     if (dt_bits == kDtBits && p->steps >= kFreeSteps) {
-      if (n <= 48u * sms)  // at most two warps per scheduler
+      if (n <= 72u * sms)  // at most three warps per scheduler
         cnc_lanes_kernel<I><<<grid_for(n, kLaneWires), 32, 0, s>>>(first, n, a, v, p->steps,
                                                                   p->dt);
       else if (n <= 1440u * sms)
