@@ -1278,7 +1278,7 @@ struct LaneWire {
   bool first, last, okR, okC;  // okR, okC: eligible divisors (divisor_ok)
 
   // FR, FC, LOW: as DualExact::step_free.  The voltages at the wire's ends
-  // stay: V + a * 0.
+  // stay, V + a * 0, but for the sign of a zero (settle_zeros).
   template <QuotForm FR, QuotForm FC, bool LOW>
   __device__ __forceinline__ void step_free(LaneState &s, float &low) const {
     const float2 neg1 = make_float2(-1.0f, -1.0f);
@@ -1297,6 +1297,17 @@ struct LaneWire {
       low = min_abs(low, a3, first ? 1.0f : ae.x);
       low = fminf(low, last ? 1.0f : fabsf(ae.y));
     }
+  }
+  // After accepted free steps.  Where V0 + q cancels, so does -V0 - q, and both
+  // sums are +0: nb is +0 where minus the voltage is -0.  (V0 + q has no other
+  // zeros: V0 is not zero, or q, of a dividend of at least kCLo, is not.)  And
+  // V + a * 0 is +0 where V is -0 and a positive.  Inside the block those signs
+  // matter no more than those of the zero quotients (exact_steps): they reach a
+  // difference of voltages only where it is zero.
+  __device__ __forceinline__ void settle_zeros(LaneState &s) const {
+    if (s.nb == 0.0f) s.nb = -0.0f;
+    if (first) s.e.x = Ve.x;
+    if (last) s.e.y = Ve.y;
   }
   // As DualExact::step_wide, on the values themselves: a difference of
   // negated values has the other sign only where it is not zero.
@@ -1449,6 +1460,7 @@ __global__ void __launch_bounds__(32)
       bool right = !holds_nan();
       if (j + n == steps) right &= fminf(fabsf(s.x.x), fabsf(s.x.y)) >= 0x1p-75f;
       if (__all_sync(kAll, right || exempt)) {
+        x.settle_zeros(s);
         j += n;
         if (run == kMostRun) penalty = 1;
         run = min(2 * run, kMostRun);
@@ -1471,6 +1483,7 @@ __global__ void __launch_bounds__(32)
       } else {
         x.steps_free<kCorrected, kCorrected, true>(s, n, low);
         right = low >= kCLo && !holds_nan();
+        x.settle_zeros(s);
       }
       right = __all_sync(kAll, right || exempt);
       if (!right) {
