@@ -24,8 +24,6 @@
 // wire by wire, three expressions per wire ran on the FP64 pipe, degrees and
 // lists took a round of atomics each and zeros their own passes.
 #include <algorithm>
-#include <mutex>
-#include <vector>
 
 #include "ckt_drand.cuh"
 #include "ckt_internal.h"
@@ -39,68 +37,47 @@ constexpr int kGroup = 64;        // chunks per group
 constexpr int kNear = 1024;       // draws reached by one entry of the near table
 constexpr int kMapsBlock = 128;   // chunks per block of the decoding
 
-struct Jump {
-  uint64_t a[48], c[48];  // state after 2^i draws: a[i]*x + c[i]
+// States reached by N multiples of some number of draws: a[k]*x + c[k].  Each
+// table is written by repeated composition, x -> as (a x + c) + cs.
+template <int N>
+struct Jumps {
+  uint64_t a[N], c[N];
 };
-
-__constant__ Jump g_jump;
-
-Jump make_jump() {
-  Jump j;
+template <int N>
+constexpr Jumps<N> make_multiples(uint64_t as, uint64_t cs) {  // 0, 1, .., N - 1 times (as, cs)
+  Jumps<N> j{};
+  uint64_t a = 1, c = 0;
+  for (int k = 0; k < N; k++) {
+    j.a[k] = a;
+    j.c[k] = c;
+    c = (as * c + cs) & kMask;
+    a = (as * a) & kMask;
+  }
+  return j;
+}
+constexpr Jumps<48> make_powers() {  // 2^0, 2^1, .. draws
+  Jumps<48> j{};
   uint64_t a = kA, c = kC;
   for (int i = 0; i < 48; i++) {
     j.a[i] = a;
     j.c[i] = c;
-    // (a, c) composed with itself: x -> a(ax + c) + c
     c = (a * c + c) & kMask;
     a = (a * a) & kMask;
   }
   return j;
 }
 
-// State after k draws, k < kNear, and after k chunks, k < kMapsBlock:
-// a[k]*x + c[k], for jumps from a block's first draw (lanes index it
-// independently, so it lives in global memory, not the constant bank).
-__device__ uint64_t g_near_a[kNear], g_near_c[kNear];
-__device__ uint64_t g_chunk_a[kMapsBlock], g_chunk_c[kMapsBlock];
-
-// The jump tables never change: they are copied to each device once.  (A
-// per-call copy from pageable memory would wait for the stream's earlier
-// work.)
-constexpr int kMaxDevices = 64;
-
-int ensure_jump_table() {
-  static std::mutex mu;
-  static bool loaded[kMaxDevices] = {};
-  int dev = 0;
-  CKT_CUDA(cudaGetDevice(&dev));
-  CKT_REQUIRE(dev >= 0 && dev < kMaxDevices, "device %d out of range", dev);
-  std::lock_guard<std::mutex> lk(mu);
-  if (!loaded[dev]) {
-    const Jump jump = make_jump();
-    CKT_CUDA(cudaMemcpyToSymbol(g_jump, &jump, sizeof(Jump)));
-    std::vector<uint64_t> na(kNear), nc(kNear), ca(kMapsBlock), cc(kMapsBlock);
-    uint64_t a = 1, c = 0;
-    for (int64_t k = 0; k < (int64_t)kMapsBlock * kChunk; k++) {
-      if (k < kNear) {
-        na[k] = a;
-        nc[k] = c;
-      }
-      if (k % kChunk == 0) {
-        ca[k / kChunk] = a;
-        cc[k / kChunk] = c;
-      }
-      c = (kA * c + kC) & kMask;  // one more draw: x -> A x + C
-      a = (kA * a) & kMask;
-    }
-    CKT_CUDA(cudaMemcpyToSymbol(g_near_a, na.data(), kNear * sizeof(uint64_t)));
-    CKT_CUDA(cudaMemcpyToSymbol(g_near_c, nc.data(), kNear * sizeof(uint64_t)));
-    CKT_CUDA(cudaMemcpyToSymbol(g_chunk_a, ca.data(), kMapsBlock * sizeof(uint64_t)));
-    CKT_CUDA(cudaMemcpyToSymbol(g_chunk_c, cc.data(), kMapsBlock * sizeof(uint64_t)));
-    loaded[dev] = true;
-  }
-  return CKT_OK;
-}
+// Part of the module's image, so that they are there for whichever stream
+// generates first (copied by the first call, through the legacy stream, they
+// were not ordered before the kernels of a non-blocking one).  g_near: k
+// draws, k < kNear; g_chunk: k chunks, k < kMapsBlock: jumps from a block's
+// first draw (lanes index them independently, so they live in global memory,
+// not the constant bank).
+constexpr Jumps<48> kPowers = make_powers();
+__constant__ const Jumps<48> g_jump = kPowers;
+static_assert(kChunk == 256, "g_chunk's stride is 2^8 draws");
+__device__ const Jumps<kNear> g_near = make_multiples<kNear>(kA, kC);
+__device__ const Jumps<kMapsBlock> g_chunk = make_multiples<kMapsBlock>(kPowers.a[8], kPowers.c[8]);
 
 __device__ __forceinline__ uint64_t skip(uint64_t x, uint64_t d) {
   for (int i = 0; d; i++, d >>= 1)
@@ -116,10 +93,10 @@ __device__ __forceinline__ uint64_t next(uint64_t &x) {
 }
 
 __device__ __forceinline__ uint64_t near_jump(uint64_t x, uint32_t k) {
-  return (__ldg(g_near_a + k) * x + __ldg(g_near_c + k)) & kMask;
+  return (__ldg(g_near.a + k) * x + __ldg(g_near.c + k)) & kMask;
 }
 __device__ __forceinline__ uint64_t chunk_jump(uint64_t x, uint32_t k) {
-  return (__ldg(g_chunk_a + k) * x + __ldg(g_chunk_c + k)) & kMask;
+  return (__ldg(g_chunk.a + k) * x + __ldg(g_chunk.c + k)) & kMask;
 }
 
 // random_element of the piece's node set (its reversed order, see
@@ -611,8 +588,6 @@ extern "C" int ckt_generate_device(const ckt_gen_params *p, ckt_device_circuit *
                          o->slot_in && o->slot_out && o->gstart),
               "wire arrays are NULL");
   const cudaStream_t s = as_stream(stream);
-  int jr = ensure_jump_table();
-  if (jr) return jr;
   GenArgs g;
   g.P = P; g.npp = npp; g.wpp = wpp;
   g.crossing = P > 1 ? drand::first_crossing(drand::pct_threshold(p->pct_wire_in_piece))

@@ -1360,8 +1360,9 @@ __global__ void __launch_bounds__(32)
                      float dt) {
   constexpr uint32_t kAll = 0xffffffffu;
   const uint32_t lane = threadIdx.x, g = lane % kLanesPerWire, slot = lane / kLanesPerWire;
-  const uint32_t t = blockIdx.x * kLaneWires + slot;
-  // lanes without a wire of their own run along on another
+  const uint32_t t = blockIdx.x * kLaneWires + min(slot, kLaneWires - 1u);
+  // Lanes without a wire of their own run along on the warp's last: another
+  // warp's would be read while that warp stores it.
   const bool mine = slot < kLaneWires && t < num_wires;
   const int64_t w = (int64_t)first_wire + min(t, num_wires - 1u), S = a.S;
   const uint32_t wire_lanes = 0x1fu << (slot * kLanesPerWire);
