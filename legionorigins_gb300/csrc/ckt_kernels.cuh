@@ -172,10 +172,11 @@ __device__ __forceinline__ float min_abs(float m, float a, float b) {
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
   return __fadd2_rn(a, make_float2(-b.x, -b.y));
 }
-// i, v: the least |I0| and |V0| of a wire (NaN ones apart).  See exact_steps.
+// i, v: the least |I0| and |V0| of a wire (NaN ones apart; NaN when all are:
+// what is added to them is NaN whatever it was).  See exact_steps.
 __device__ __forceinline__ bool sound_wire(float i, float v, float L, float C, float dt) {
-  return (i >= 0x1p-50f) & (v >= 0x1p-50f) & (fabsf(L) >= 0x1p-43f) & (fabsf(C) >= 0x1p-20f) &
-         (__fmul_rn(v, fabsf(C)) >= __fmul_rn(0x1p-22f, dt));
+  return !(i < 0x1p-50f) & !(v < 0x1p-50f) & (fabsf(L) >= 0x1p-43f) & (fabsf(C) >= 0x1p-20f) &
+         !(__fmul_rn(v, fabsf(C)) < __fmul_rn(0x1p-22f, dt));
 }
 // Orders magnitudes as integers, with zero above everything: finite values
 // by magnitude, then infinity (kOrderInf), NaN, zero.
