@@ -320,14 +320,21 @@ static __device__ __noinline__ float cut_yl(float b) {
   return none;
 }
 
-// The quotient of a free step.
-enum QuotForm : uint32_t { kCorrected, kSplit, kCut };
+// The quotient of a free step.  kEither: split or cut, as `cut` says (3
+// operations), where it is not worth a loop of its own.
+enum QuotForm : uint32_t { kCorrected, kSplit, kCut, kEither };
 template <QuotForm FORM>
-__device__ __forceinline__ float free_quot(float a, const Recip &k) {
+__device__ __forceinline__ float free_quot(float a, const Recip &k, bool cut = false) {
+  if (FORM == kEither)
+    return __fmaf_rn(a, k.y, cut ? __fmul_rz(a, k.yl) : __fmul_rn(a, k.yl));
   return FORM == kCut ? cut_quot(a, k) : (FORM == kSplit ? split_quot(a, k) : recip_quot(a, k));
 }
 template <QuotForm FORM>
-__device__ __forceinline__ float2 free_quot2(float2 a, const Recip2 &k) {
+__device__ __forceinline__ float2 free_quot2(float2 a, const Recip2 &k, bool cut = false) {
+  if (FORM == kEither) {
+    const float2 n = __fmul2_rn(a, k.yl), z = __fmul2_rz(a, k.yl);
+    return __ffma2_rn(a, k.y, make_float2(cut ? z.x : n.x, cut ? z.y : n.y));
+  }
   return FORM == kCut ? cut_quot2(a, k)
                       : (FORM == kSplit ? split_quot2(a, k) : recip_quot2(a, k));
 }

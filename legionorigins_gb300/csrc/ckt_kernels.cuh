@@ -192,6 +192,11 @@ __device__ __forceinline__ uint32_t nan_bits(float2 a) {
   return (a.x != a.x ? 1u : 0u) | (a.y != a.y ? 2u : 0u);
 }
 
+__device__ __forceinline__ bool huge(float a) { return fabsf(a) > 0x1p60f; }
+__device__ __forceinline__ bool huge(float2 a) { return huge(a.x) | huge(a.y); }
+__device__ __forceinline__ bool tame(float a) { return fabsf(a) <= 0x1p60f; }  // NaN: false
+__device__ __forceinline__ bool tame(float2 a) { return tame(a.x) & tame(a.y); }
+
 // EXACT, two wires per thread: the reference's operations in the reference's
 // order, each rounded as IEEE fp32 rounds it, with the 29 divisions of a
 // wire-step done as correctly rounded quotients by precomputed reciprocals
@@ -360,24 +365,28 @@ struct DualExact {
   }
   // The same with every zero and infinite dividend's quotient as well: a * y.
   // lowR, lowC collect the least order of the nonzero dividends.
-  static __device__ __forceinline__ float2 wide(float2 a, const Recip2 &k, uint32_t &low) {
+  template <QuotForm FORM>
+  static __device__ __forceinline__ float2 wide(float2 a, const Recip2 &k, bool cut,
+                                                uint32_t &low) {
     const uint32_t tx = order(a.x), ty = order(a.y);
-    const float2 q = split_quot2(a, k), z = __fmul2_rn(a, k.y);
+    const float2 q = free_quot2<FORM>(a, k, cut), z = __fmul2_rn(a, k.y);
     low = min(low, min(tx, ty));
     return make_float2(tx >= kOrderInf ? z.x : q.x, ty >= kOrderInf ? z.y : q.y);
   }
+  template <QuotForm FORM>
   __device__ __forceinline__ void step_wide(float2 (&ni)[10], float2 (&nv)[11],
                                             const float2 (&nI0)[10], const float2 (&V0)[9],
-                                            uint32_t &lowR, uint32_t &lowC) const {
+                                            bool cutR, bool cutC, uint32_t &lowR,
+                                            uint32_t &lowC) const {
 #pragma unroll
     for (int k = 0; k < 10; k++) {
       const float2 a1 = __fmul2_rn(L, __fadd2_rn(ni[k], nI0[k]));
-      ni[k] = wide(sub2(sub2(nv[k + 1], nv[k]), dt_div(a1)), kR, lowR);
+      ni[k] = wide<FORM>(sub2(sub2(nv[k + 1], nv[k]), dt_div(a1)), kR, cutR, lowR);
     }
 #pragma unroll
     for (int k = 0; k < 9; k++)
       nv[k + 1] = __fadd2_rn(
-          V0[k], wide(__fmul2_rn(dt2, sub2(ni[k], ni[k + 1])), kC, lowC));
+          V0[k], wide<FORM>(__fmul2_rn(dt2, sub2(ni[k], ni[k + 1])), kC, cutC, lowC));
   }
   __device__ __forceinline__ bool can_wide(const float2 (&nI0)[10]) const {
     uint32_t x = ~0u, y = ~0u;
@@ -395,6 +404,22 @@ struct DualExact {
     return m;
   }
   __device__ __forceinline__ float most_C() const { return fmaxf(fabsf(kC.nb.x), fabsf(kC.nb.y)); }
+  // Dividends like those these currents come of and lead to keep LOW's bound,
+  // and nothing is about to overflow (NaN apart).
+  static __device__ __forceinline__ bool calm(const float2 (&ni)[10]) {
+    float most = 0.0f, drop = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int k = 0; k < 10; k++) most = fmaxf(most, fmaxf(fabsf(ni[k].x), fabsf(ni[k].y)));
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const float2 d = sub2(ni[k], ni[k + 1]);
+      drop = min_abs(drop, d.x, d.y);
+    }
+    return (least_current(ni) >= 0x1p-48f) & (drop >= 0x1p-20f) & (most <= 0x1p40f);
+  }
+  static __device__ __forceinline__ bool starts_zero(const float2 (&ni)[10]) {
+    return ((ni[4].x == 0.0f) & (ni[5].x == 0.0f)) | ((ni[4].y == 0.0f) & (ni[5].y == 0.0f));
+  }
   // The loop's constants keep every dividend's tininess from mattering
   // (exact_steps).
   __device__ __forceinline__ bool sound(const float2 (&nI0)[10], const float2 (&V0)[9]) const {
@@ -429,6 +454,7 @@ struct DualExact {
           V0[k], split_quot2(__fmul2_rn(dt2, sub2(ni[k], ni[k + 1])), kC));
   }
   static constexpr uint32_t kWires = 3u;  // nan_bits of both wires
+  static constexpr bool kFrontHere = true;  // exact_steps' first guarded steps not by a call
   // NaN where any of a wire's currents or voltages is NaN (or infinities
   // cancel).
   static __device__ __forceinline__ float2 state_sum(const float2 (&ni)[10],
@@ -493,16 +519,25 @@ struct DualExact {
 //        so with |L| >= 2^-43 a1 is 0 or at least 2^-118 = kDtTiny.
 //    (With LOW a1 needs no check either, see dt_outside.)
 // Where the constants are not sound, or a block failed, the next blocks are
-// careful ones: wide steps, which also divide zeros and infinities rightly (a
-// times RN(1/b)) and collect the least nonzero dividends -- by C, at least
-// 2^-77 |C| wanted, by R, 2^-66, so that a nonzero current is at least 2^-74
-// and, I0 being 0 or at least 2^-50 (wide_wire) and so the currents at the
-// block's start, a1 is 0 or at least kDtTiny -- or LOW ones, where a divisor
-// is unchecked.  A careful block that fails is done again with step(), and
-// the next 1, 2, 4 and 8 blocks are guarded outright as failures repeat.
-//
-// A failed block costs its own steps once more, so the first blocks are short
-// and after a failure sound blocks pause for 1, 2, 4 and 8 careful ones.
+// careful ones, of the form whose bounds the currents at hand let expect:
+//  * LOW ones, when those currents are calm (of ordinary size and distance);
+//    not after a free block's failure, which they would share.
+//  * Wide steps otherwise, which also divide zeros and infinities rightly (a
+//    times RN(1/b)) and collect the least nonzero dividends -- by C, at least
+//    2^-77 |C| wanted, by R, 2^-66, so that a nonzero current is at least
+//    2^-74 and, I0 being 0 or at least 2^-50 (wide_wire) and so the currents
+//    at the block's start, a1 is 0 or at least kDtTiny.  They take split or
+//    truncated products (kEither); with corrected quotients, whose overflow
+//    shows as NaN, a block must not end with a new NaN.
+//  * Guarded steps, where neither may be expected or the block failed: the next
+//    32, 64 and 128 in one call, then all the rest of the loop, as in launches
+//    of few steps.  (A warp with sound constants goes on trying.)
+// After a failure sound blocks pause for 16, 32, 64 and 128 steps; before an
+// overflow (a state whose sum is past 2^60) for one careful block, as from
+// nodes that are.  A failed block costs its own steps once more, so the first
+// blocks are short.  A careful block is a call that loads the wires' constants
+// anew and divides for their reciprocals, about as long as 5 steps, so those
+// that come out right grow to 64 steps.
 //
 // Why: the guards' 58 compares and two branches per paired step held the loop
 // at 75% of the FP32 pipe, and the corrected quotients are 76 of its 163
@@ -513,15 +548,28 @@ struct DualExact {
 // (4.80 ms with corrected quotients); the 125 operations at the pipe's full
 // rate take 3.25 ms.  From the generated state (zeros, overflow, all NaN
 // after 26 steps) 5.13 ms guarded, 3.96 ms with its first 32 steps guarded,
-// 3.73 ms with 10 guarded and 16 wide ones.
+// 3.64 ms with 10 guarded and 16 wide ones.  The careful forms, 1,048,576 /
+// 32,768 / 4096 wires, ms per 1000 steps, guarded one or two wires per thread /
+// with short careful blocks, wide first, all tried again / as here: zeros in 2%
+// of the wires' starting values 5.87 0.27 0.17 / 7.11 0.35 0.13 / 4.55 0.23
+// 0.10; loops from zeros with ordinary nodes, most segments staying below
+// 2^-66, 18.96 0.80 0.51 / 21.94 0.91 0.75 / 18.69 0.81 0.45; everything zero
+// 17.29 0.75 0.48 / 10.82 0.83 0.99 / 7.11 0.29 0.11; no inductance 5.61 0.27
+// 0.35 / 7.33 0.26 0.36 / 4.78 0.30 0.33.  Slower than guarded throughout:
+// 32 steps with such a start (5 to 25%; half a launch's warps with NaN nodes
+// 50%), and loops whose quotients are nearly all subnormal (119 / 125 / 145
+// ms), in which the divide routine is all that counts.
 constexpr int kGuardedRun = 16;  // steps between looks for all NaN (guarded loop)
-constexpr int kCarefulRun = 16;  // steps of a careful block
+constexpr int kCarefulRun = 16;  // steps of the first careful block
 // From zero currents or voltages the first steps run guarded: what the node
 // voltages start reaches one segment further per step, falling to 2^-110 on
 // its way, below what the other forms divide rightly.
 constexpr int kFrontRun = 10;
-enum CarefulForm { kGuarded, kLow, kWide };
-constexpr int kFirstRun = 8, kMostRun = 64;  // steps of a free block
+// From states with single zeros or tiny values 2 guarded steps: then the
+// dividends mostly are neither.
+constexpr int kCalmRun = 2;
+constexpr int kFirstRun = 8, kMostRun = 64;  // steps of a free or careful block
+constexpr int kMostPause = 128;  // steps before what failed is tried again
 // Values per thread in shared memory: the state at a block's start (10
 // currents, 9 voltages), the two node voltages and yl of R and C.
 constexpr int kSavedState = 23;
@@ -560,6 +608,39 @@ __device__ __forceinline__ void load_state(const F *save, F (&ni)[10], F (&nv)[1
   for (int k = 0; k < 9; k++) nv[k + 1] = save[(10 + k) * STRIDE];
 }
 
+// The loop with guarded steps only: few steps, a general dt, or states that the
+// other forms do not take.
+template <typename Stepper, typename F>
+__device__ __forceinline__ void exact_steps_guarded(const Stepper &pk, int steps, F (&ni)[10],
+                                                    F (&nv)[11], const F (&nI0)[10],
+                                                    const F (&V0)[9]) {
+  const uint32_t lanes = __activemask();
+  int j = 0;
+#pragma unroll 1
+  while (j < steps) {
+    if (__all_sync(lanes, Stepper::all_nan(ni, nv) == Stepper::kWires)) break;
+    const int n = min(kGuardedRun, steps - j);
+#pragma unroll 1
+    for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
+    j += n;
+  }
+#pragma unroll 1
+  for (; j < steps; j++) pk.step_all_nan(ni, nv, nI0, V0);
+}
+
+// The wires' constants and the state in `save`, as the steps take them.
+template <typename Stepper, int STRIDE, typename Wires, typename F>
+__device__ __forceinline__ Stepper resume(const Wires &wires, const F *save, F (&ni)[10],
+                                          F (&nv)[11], F (&nI0)[10], F (&V0)[9]) {
+  Stepper pk = wires.template stepper<Stepper>();
+  pk.kR.yl = save[21 * STRIDE];
+  pk.kC.yl = save[22 * STRIDE];
+  wires.load(nI0, V0);
+  nv[0] = save[19 * STRIDE];
+  nv[10] = save[20 * STRIDE];
+  load_state<STRIDE>(save, ni, nv);
+  return pk;
+}
 // ni, nv: the state before the first step, and after the last.  wires: the
 // thread's wires in global memory (SoloWire, DualWires), unchanged until the
 // loop is done: their constants are loaded again for each stretch of blocks
@@ -569,12 +650,12 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
                                             F (&nv)[11], F *save) {
   const uint32_t lanes = __activemask();
   QuotForm FR, FC;  // of the warp
-  bool sound;
-  CarefulForm how;
-  // careful: blocks before the next try of sound ones; skip: careful blocks
-  // before the next that is not guarded outright
-  int j = 0, run = kFirstRun, careful = 0, penalty = 1, skip = 0, again = 1;
-  save_state<STRIDE>(save, ni, nv);
+  bool sound, wide;
+  // pause: steps before the next try of free blocks; guard: steps to run
+  // guarded before the next try of the careful forms
+  int j = 0, run = kFirstRun, pause = 0, penalty = kCarefulRun;
+  int guard = 0, again = 2 * kCarefulRun, careful = kCarefulRun;
+  if (!Stepper::kFrontHere) save_state<STRIDE>(save, ni, nv);
   save[19 * STRIDE] = nv[0];
   save[20 * STRIDE] = nv[10];
   {
@@ -600,8 +681,19 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
     F nI0[10], V0[9];
     wires.load(nI0, V0);
     sound = __all_sync(lanes, pk.sound(nI0, V0));
-    skip = sound ? 0 : 1;
-    how = FR == kSplit && FC == kSplit && __all_sync(lanes, pk.can_wide(nI0)) ? kWide : kLow;
+    wide = __all_sync(lanes, pk.can_wide(nI0));
+    // NaN or overflow from a node reaches the far end within 10 steps
+    if (__any_sync(lanes, !(tame(nv[0]) & tame(nv[10])))) pause = kCarefulRun;
+    int front = 0;
+    if (__any_sync(lanes, Stepper::starts_zero(ni))) front = kFrontRun;
+    else if (!sound && !__all_sync(lanes, Stepper::calm(ni))) front = kCalmRun;
+    if (Stepper::kFrontHere) {
+#pragma unroll 1
+      for (; j < front; j++) pk.step(ni, nv, nI0, V0);
+      save_state<STRIDE>(save, ni, nv);
+    } else {
+      guard = front;
+    }
     save[21 * STRIDE] = pk.kR.yl;
     save[22 * STRIDE] = pk.kC.yl;
   }
@@ -612,7 +704,7 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
     // the switch only when every thread of the warp can take it, so that a
     // warp never runs the two loops one after the other
     if (__all_sync(lanes, nan == Stepper::kWires)) break;
-    if (sound && careful == 0) {
+    if (sound && pause <= 0) {
       Stepper pk = wires.template stepper<Stepper>();
       pk.kR.yl = save[21 * STRIDE];
       pk.kC.yl = save[22 * STRIDE];
@@ -620,15 +712,14 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
       wires.load(nI0, V0);
       nv[0] = save[19 * STRIDE];
       nv[10] = save[20 * STRIDE];
-      bool right = true, all_nan = false;
+      bool right = true, leave = false;
       float none = 0.0f;
 #pragma unroll 1
-      while (!all_nan && j < steps) {
+      while (!leave && j < steps) {
         const int n = min(run, steps - j);
-        // one loop per pair of quotient forms: a warp with one unchecked
-        // divisor (8% of paired warps) keeps the other's split quotients
-        // A loop per pair of forms, the usual one last (as a chain of ifs or
-        // with it first the loops' code differs by 1 to 4% either way).
+        // A loop per pair of quotient forms: a warp with one unchecked divisor
+        // keeps the other's split quotients.  The usual pair last (as a chain
+        // of ifs or with it first the loops' code differs by 1 to 4% either way).
         switch (FR * 3 + FC) {
           case kCut * 3 + kSplit:
 #pragma unroll 1
@@ -661,67 +752,64 @@ __device__ __forceinline__ void exact_steps(const Wires &wires, int steps, F (&n
               pk.template step_free<kSplit, kSplit, false>(ni, nv, nI0, V0, none);
             break;
         }
-        right = (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
-        if (j + n == steps) right &= Stepper::least_current(ni) >= 0x1p-75f;
-        right = __all_sync(lanes, right);
-        if (!right) break;
+        const F sum = Stepper::state_sum(ni, nv);
+        const bool done =
+            j + n < steps || Stepper::least_current(ni) >= 0x1p-75f;  // as a result
+        if (!__all_sync(lanes, tame(sum) & done)) {
+          right = __all_sync(lanes, (nan_bits(sum) & ~nan) == 0u && done);
+          if (!right) break;
+          nan = Stepper::all_nan(ni, nv);
+          leave = __all_sync(lanes, nan == Stepper::kWires);
+          // about to overflow: wide steps, which also get that right
+          if (__any_sync(lanes, huge(sum))) {
+            leave = true;
+            pause = kCarefulRun;
+          }
+        }
         j += n;
-        if (run == kMostRun) penalty = 1;
+        if (run == kMostRun) penalty = kCarefulRun;
         run = min(2 * run, kMostRun);
         save_state<STRIDE>(save, ni, nv);
-        nan = Stepper::all_nan(ni, nv);
-        all_nan = __all_sync(lanes, nan == Stepper::kWires);
       }
-      if (right) continue;
-      careful = penalty;
-      penalty = min(2 * penalty, 8);
-      run = kFirstRun;
+      if (!right) {
+        pause = penalty;
+        penalty = min(2 * penalty, kMostPause);
+        run = kFirstRun;
+      }
+      continue;
     }
-    const int n = min(j == 0 ? kFrontRun : kCarefulRun, steps - j);
-    const bool right =
-        wires.template careful<Stepper, STRIDE>(n, skip ? kGuarded : how, nan, lanes, save);
-    if (skip) {
-      skip--;
-    } else if (right) {
-      again = 1;
+    // the form whose bounds the state is likely to keep
+    const bool calm = !sound && __all_sync(lanes, Stepper::calm(ni));
+    const bool can =
+        calm || (wide && __all_sync(lanes, Stepper::least_order(ni) >= order(0x1p-74f)));
+    const int left = steps - j;
+    int n;
+    if (guard <= 0) {
+      n = min(left, sound ? min(careful, pause) : careful);
+      if (can && wires.template careful<Stepper, STRIDE>(n, calm, FR, FC, nan, lanes, save)) {
+        again = 2 * kCarefulRun;
+        careful = min(2 * careful, kMostRun);
+      } else {
+        if (!sound && (again == kMostPause || left <= kMostPause)) break;
+        guard = again;
+        again = min(2 * again, kMostPause);
+        careful = kCarefulRun;
+        continue;
+      }
     } else {
-      skip = again;
-      again = min(2 * again, 8);
+      n = wires.template guarded<Stepper, STRIDE>(min(left, guard), lanes, save);
+      guard -= n;
     }
     j += n;
-    if (careful) careful--;
+    pause -= n;
   }
   if (j < steps) {
-    const Stepper pk = wires.template stepper<Stepper>();
     F nI0[10], V0[9];
-    wires.load(nI0, V0);
-    load_state<STRIDE>(save, ni, nv);
-    nv[0] = save[19 * STRIDE];
-    nv[10] = save[20 * STRIDE];
-#pragma unroll 1
-    for (; j < steps; j++) pk.step_all_nan(ni, nv, nI0, V0);
+    const Stepper pk = resume<Stepper, STRIDE>(wires, save, ni, nv, nI0, V0);
+    exact_steps_guarded(pk, steps - j, ni, nv, nI0, V0);
   } else {
     load_state<STRIDE>(save, ni, nv);
   }
-}
-
-// The same loop with guarded steps only: few steps, or a general dt.
-template <typename Stepper, typename F>
-__device__ __forceinline__ void exact_steps_guarded(const Stepper &pk, int steps, F (&ni)[10],
-                                                    F (&nv)[11], const F (&nI0)[10],
-                                                    const F (&V0)[9]) {
-  const uint32_t lanes = __activemask();
-  int j = 0;
-#pragma unroll 1
-  while (j < steps) {
-    if (__all_sync(lanes, Stepper::all_nan(ni, nv) == Stepper::kWires)) break;
-    const int n = min(kGuardedRun, steps - j);
-#pragma unroll 1
-    for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
-    j += n;
-  }
-#pragma unroll 1
-  for (; j < steps; j++) pk.step_all_nan(ni, nv, nI0, V0);
 }
 
 // EXACT, one wire per thread: DualExact's arithmetic and guards on scalar
@@ -838,23 +926,26 @@ struct SoloExact {
       if (LOW) low = min_abs(low, a[k], a[k + 1]);
     if (LOW) low = fminf(low, fabsf(a[8]));
   }
-  static __device__ __forceinline__ float wide(float a, const Recip &k, uint32_t &low) {
+  template <QuotForm FORM>
+  static __device__ __forceinline__ float wide(float a, const Recip &k, bool cut, uint32_t &low) {
     const uint32_t t = order(a);
-    const float q = split_quot(a, k), z = __fmul_rn(a, k.y);
+    const float q = free_quot<FORM>(a, k, cut), z = __fmul_rn(a, k.y);
     low = min(low, t);
     return t >= kOrderInf ? z : q;
   }
+  template <QuotForm FORM>
   __device__ __forceinline__ void step_wide(float (&ni)[10], float (&nv)[11],
-                                            const float (&I0)[10], const float (&V0)[9],
-                                            uint32_t &lowR, uint32_t &lowC) const {
+                                            const float (&I0)[10], const float (&V0)[9], bool cutR,
+                                            bool cutC, uint32_t &lowR, uint32_t &lowC) const {
 #pragma unroll
     for (int k = 0; k < 10; k++) {
       const float a1 = __fmul_rn(L, __fsub_rn(ni[k], I0[k]));
-      ni[k] = wide(__fsub_rn(__fsub_rn(nv[k + 1], nv[k]), dt_quot(a1)), kR, lowR);
+      ni[k] = wide<FORM>(__fsub_rn(__fsub_rn(nv[k + 1], nv[k]), dt_quot(a1)), kR, cutR, lowR);
     }
 #pragma unroll
     for (int k = 0; k < 9; k++)
-      nv[k + 1] = __fadd_rn(V0[k], wide(__fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1])), kC, lowC));
+      nv[k + 1] =
+          __fadd_rn(V0[k], wide<FORM>(__fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1])), kC, cutC, lowC));
   }
   __device__ __forceinline__ bool can_wide(const float (&I0)[10]) const {
     return wide_wire(least_order(I0), L, kC.nb);
@@ -866,6 +957,17 @@ struct SoloExact {
     return m;
   }
   __device__ __forceinline__ float most_C() const { return fabsf(kC.nb); }
+  static __device__ __forceinline__ bool calm(const float (&ni)[10]) {
+    float most = 0.0f, drop = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int k = 0; k < 10; k++) most = fmaxf(most, fabsf(ni[k]));
+#pragma unroll
+    for (int k = 0; k < 9; k++) drop = fminf(drop, fabsf(__fsub_rn(ni[k], ni[k + 1])));
+    return (least_current(ni) >= 0x1p-48f) & (drop >= 0x1p-20f) & (most <= 0x1p40f);
+  }
+  static __device__ __forceinline__ bool starts_zero(const float (&ni)[10]) {
+    return (ni[4] == 0.0f) & (ni[5] == 0.0f);
+  }
   __device__ __forceinline__ bool sound(const float (&I0)[10], const float (&V0)[9]) const {
     float i = fabsf(I0[0]), v = fabsf(V0[0]);
 #pragma unroll
@@ -888,6 +990,7 @@ struct SoloExact {
       nv[k + 1] = __fadd_rn(V0[k], split_quot(__fmul_rn(dt, __fsub_rn(ni[k], ni[k + 1])), kC));
   }
   static constexpr uint32_t kWires = 1u;
+  static constexpr bool kFrontHere = false;
   static __device__ __forceinline__ float state_sum(const float (&ni)[10], const float (&nv)[11]) {
     float s = ni[9], t = nv[9];
 #pragma unroll
@@ -938,42 +1041,65 @@ struct WireSource {
   int64_t S;
   float dt;
 };
-// n steps on the state in `save`, of the given form; if those come out wrong,
-// n guarded ones.  Returns whether they were right.  Out of line: rare, and
-// the guarded steps' registers (all dividends of a phase at once) would spill
-// the free steps' loop.
+// n LOW or wide steps on the state in `save`.  FR, FC: the warp's quotient
+// forms.  Returns whether they came out right; otherwise the state there is as
+// it was.  Out of line, as guarded_steps: rare, and the registers of either
+// would spill the free steps' loop, and each other's.
 template <typename Stepper, int STRIDE, typename Wires, typename F>
-__device__ __noinline__ bool careful_steps(const Wires wires, int n, CarefulForm how, uint32_t nan,
-                                           uint32_t lanes, F *save) {
-  Stepper pk = wires.template stepper<Stepper>();
-  pk.kR.yl = save[21 * STRIDE];
-  pk.kC.yl = save[22 * STRIDE];
+__device__ __noinline__ bool careful_steps(const Wires wires, int n, bool calm, QuotForm FR,
+                                           QuotForm FC, uint32_t nan, uint32_t lanes, F *save) {
   F nI0[10], V0[9], ni[10], nv[11];
-  wires.load(nI0, V0);
-  nv[0] = save[19 * STRIDE];
-  nv[10] = save[20 * STRIDE];
-  load_state<STRIDE>(save, ni, nv);
-  bool right = false;
-  if (how == kWide) {
-    right = Stepper::least_order(ni) >= order(0x1p-74f);
-    uint32_t lowR = ~0u, lowC = ~0u;
-#pragma unroll 1
-    for (int i = 0; i < n; i++) pk.step_wide(ni, nv, nI0, V0, lowR, lowC);
-    right &= lowR >= order(0x1p-66f) && lowC >= order(__fmul_rn(0x1p-77f, pk.most_C()));
-  } else if (how == kLow) {
+  const Stepper pk = resume<Stepper, STRIDE>(wires, save, ni, nv, nI0, V0);
+  bool right;
+  if (calm) {
     float low = __int_as_float(0x7f800000);
+    if (FR == kSplit && FC == kSplit) {
 #pragma unroll 1
-    for (int i = 0; i < n; i++) pk.template step_free<kCorrected, kCorrected, true>(ni, nv, nI0, V0, low);
-    right = low >= kCLo && (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
-  }
-  right = __all_sync(lanes, right);
-  if (!right) {
-    load_state<STRIDE>(save, ni, nv);
+      for (int i = 0; i < n; i++) pk.template step_free<kSplit, kSplit, true>(ni, nv, nI0, V0, low);
+    } else {
 #pragma unroll 1
-    for (int i = 0; i < n; i++) pk.step(ni, nv, nI0, V0);
+      for (int i = 0; i < n; i++)
+        pk.template step_free<kCorrected, kCorrected, true>(ni, nv, nI0, V0, low);
+    }
+    right = low >= kCLo;
+  } else {
+    uint32_t lowR = ~0u, lowC = ~0u;
+    if (FR == kSplit && FC == kSplit) {
+#pragma unroll 1
+      for (int i = 0; i < n; i++)
+        pk.template step_wide<kSplit>(ni, nv, nI0, V0, false, false, lowR, lowC);
+    } else if (FR != kCorrected && FC != kCorrected) {
+#pragma unroll 1
+      for (int i = 0; i < n; i++)
+        pk.template step_wide<kEither>(ni, nv, nI0, V0, FR == kCut, FC == kCut, lowR, lowC);
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < n; i++)
+        pk.template step_wide<kCorrected>(ni, nv, nI0, V0, false, false, lowR, lowC);
+    }
+    right = lowR >= order(0x1p-66f) && lowC >= order(__fmul_rn(0x1p-77f, pk.most_C()));
   }
+  if (calm || FR == kCorrected || FC == kCorrected)
+    right &= (nan_bits(Stepper::state_sum(ni, nv)) & ~nan) == 0u;
+  if (!__all_sync(lanes, right)) return false;
   save_state<STRIDE>(save, ni, nv);
-  return right;
+  return true;
+}
+// n guarded steps, fewer if a look finds all of the warp's states all NaN.
+// Returns their number.
+template <typename Stepper, int STRIDE, typename Wires, typename F>
+__device__ __noinline__ int guarded_steps(const Wires wires, int n, uint32_t lanes, F *save) {
+  F nI0[10], V0[9], ni[10], nv[11];
+  const Stepper pk = resume<Stepper, STRIDE>(wires, save, ni, nv, nI0, V0);
+  int done = 0;
+  do {
+    const int m = min(kGuardedRun, n - done);
+#pragma unroll 1
+    for (int i = 0; i < m; i++) pk.step(ni, nv, nI0, V0);
+    done += m;
+  } while (done < n && !__all_sync(lanes, Stepper::all_nan(ni, nv) == Stepper::kWires));
+  save_state<STRIDE>(save, ni, nv);
+  return done;
 }
 struct SoloWire : WireSource {
   int64_t w;
@@ -988,9 +1114,13 @@ struct SoloWire : WireSource {
     for (int k = 0; k < 9; k++) V0[k] = vol[k * S + w];
   }
   template <typename Stepper, int STRIDE>
-  __device__ __forceinline__ bool careful(int n, CarefulForm how, uint32_t nan, uint32_t lanes,
-                                          float *save) const {
-    return careful_steps<Stepper, STRIDE>(*this, n, how, nan, lanes, save);
+  __device__ __forceinline__ bool careful(int n, bool calm, QuotForm FR, QuotForm FC, uint32_t nan,
+                                          uint32_t lanes, float *save) const {
+    return careful_steps<Stepper, STRIDE>(*this, n, calm, FR, FC, nan, lanes, save);
+  }
+  template <typename Stepper, int STRIDE>
+  __device__ __forceinline__ int guarded(int n, uint32_t lanes, float *save) const {
+    return guarded_steps<Stepper, STRIDE>(*this, n, lanes, save);
   }
 };
 struct DualWires : WireSource {
@@ -1007,9 +1137,13 @@ struct DualWires : WireSource {
     for (int k = 0; k < 9; k++) V0[k] = make_float2(vol[k * S + wa], vol[k * S + wb]);
   }
   template <typename Stepper, int STRIDE>
-  __device__ __forceinline__ bool careful(int n, CarefulForm how, uint32_t nan, uint32_t lanes,
-                                          float2 *save) const {
-    return careful_steps<Stepper, STRIDE>(*this, n, how, nan, lanes, save);
+  __device__ __forceinline__ bool careful(int n, bool calm, QuotForm FR, QuotForm FC, uint32_t nan,
+                                          uint32_t lanes, float2 *save) const {
+    return careful_steps<Stepper, STRIDE>(*this, n, calm, FR, FC, nan, lanes, save);
+  }
+  template <typename Stepper, int STRIDE>
+  __device__ __forceinline__ int guarded(int n, uint32_t lanes, float2 *save) const {
+    return guarded_steps<Stepper, STRIDE>(*this, n, lanes, save);
   }
 };
 
@@ -1246,7 +1380,8 @@ __global__ void __launch_bounds__(256)
 // Why: with about one warp per scheduler a step takes as long as that warp
 // needs to issue it and its chain of dependent operations.  One wire per
 // thread issues 125 operations one after another; here 13 paired ones and 5
-// single ones, and the chain of 13 operations and a shuffle shows.
+// single ones, and the chain shows: 9 dependent operations and a shuffle, from
+// a current over the neighbour's voltage to the next current.
 //
 // The arithmetic, the blocks of free steps and their checks are
 // exact_steps'; the rollback state stays in registers.
@@ -1312,20 +1447,22 @@ struct LaneWire {
   }
   // As DualExact::step_wide, on the values themselves: a difference of
   // negated values has the other sign only where it is not zero.
-  __device__ __forceinline__ void step_wide(LaneState &s, uint32_t &lowR, uint32_t &lowC) const {
+  template <QuotForm FORM>
+  __device__ __forceinline__ void step_wide(LaneState &s, bool cutR, bool cutC, uint32_t &lowR,
+                                            uint32_t &lowC) const {
     const float2 i = make_float2(-s.x.x, s.x.y), I0 = make_float2(nX0.x, -nX0.y);
     const float vb = -s.nb;
     const float2 a1 = __fmul2_rn(make_float2(L, L), sub2(i, I0));
     const float2 dv = sub2(make_float2(vb, s.e.y), make_float2(s.e.x, vb));
-    const float2 q = DualExact<true>::wide(sub2(dv, dt_quot2(a1)), R, lowR);
+    const float2 q = DualExact<true>::wide<FORM>(sub2(dv, dt_quot2(a1)), R, cutR, lowR);
     const float l = __shfl_sync(0xffffffffu, q.y, left);
     const float r = __shfl_sync(0xffffffffu, q.x, right);
     s.x = make_float2(-q.x, q.y);
-    s.nb = -__fadd_rn(-nVb, SoloExact<true>::wide(__fmul_rn(dt, __fsub_rn(q.x, q.y)), C, lowC));
+    s.nb = -__fadd_rn(-nVb, SoloExact<true>::wide<FORM>(__fmul_rn(dt, __fsub_rn(q.x, q.y)), C, cutC, lowC));
     const float va = __fadd_rn(
-        Ve.x, SoloExact<true>::wide(first ? 1.0f : __fmul_rn(dt, __fsub_rn(l, q.x)), C, lowC));
+        Ve.x, SoloExact<true>::wide<FORM>(first ? 1.0f : __fmul_rn(dt, __fsub_rn(l, q.x)), C, cutC, lowC));
     const float vc = __fadd_rn(
-        Ve.y, SoloExact<true>::wide(last ? 1.0f : __fmul_rn(dt, __fsub_rn(q.y, r)), C, lowC));
+        Ve.y, SoloExact<true>::wide<FORM>(last ? 1.0f : __fmul_rn(dt, __fsub_rn(q.y, r)), C, cutC, lowC));
     if (!first) s.e.x = va;
     if (!last) s.e.y = vc;
   }
@@ -1424,15 +1561,16 @@ __global__ void __launch_bounds__(32)
                                         min_abs(fabsf(x.nVb), x.first ? 1.0f : x.Ve.x,
                                                 x.last ? 1.0f : x.Ve.y),
                                         x.L, c, dt));
-    wide = FR == kSplit && FC == kSplit &&
-           __all_sync(kAll, wide_wire(min(order(I0), order(I1)), x.L, c));
+    wide = __all_sync(kAll, wide_wire(min(order(I0), order(I1)), x.L, c));
   }
   x.E.nb = make_float2(x.C.nb, x.C.nb);
   x.E.y = make_float2(x.first ? 0.0f : x.C.y, x.last ? 0.0f : x.C.y);
   x.E.yl = make_float2(x.first ? 0.0f : x.C.yl, x.last ? 0.0f : x.C.yl);
 
-  // as exact_steps: careful, skip count blocks
-  int j = 0, run = kFirstRun, careful = 0, penalty = 1, skip = sound ? 0 : 1, again = 1;
+  // as exact_steps
+  int j = 0, run = kFirstRun, pause = 0, penalty = kCarefulRun;
+  int again = 2 * kCarefulRun, careful = kCarefulRun;
+  int guard = sound ? 0 : (__any_sync(kAll, s.x.x == 0.0f && s.x.y == 0.0f) ? kFrontRun : kCalmRun);
 #pragma unroll 1
   while (j < steps) {
     // which lanes' state is all NaN (each answers for what it computes)
@@ -1451,7 +1589,7 @@ __global__ void __launch_bounds__(32)
       return sum != sum;
     };
     const LaneState start = s;
-    if (sound && careful == 0) {
+    if (sound && pause <= 0) {
       const int n = min(run, steps - j);
       if (FR == kSplit && FC == kSplit) x.steps_free<kSplit, kSplit, false>(s, n, low);
       else if (FR == kCut && FC == kSplit) x.steps_free<kCut, kSplit, false>(s, n, low);
@@ -1464,23 +1602,39 @@ __global__ void __launch_bounds__(32)
       if (__all_sync(kAll, right || exempt)) {
         x.settle_zeros(s);
         j += n;
-        if (run == kMostRun) penalty = 1;
+        if (run == kMostRun) penalty = kCarefulRun;
         run = min(2 * run, kMostRun);
         continue;
       }
       s = start;
       run = kFirstRun;
-      careful = penalty;
-      penalty = min(2 * penalty, 8);
+      pause = penalty;
+      penalty = min(2 * penalty, kMostPause);
     }
-    const int n = min(j == 0 ? kFrontRun : kCarefulRun, steps - j);
-    if (skip == 0 && eligible) {
-      bool right;
+    const bool guarded = guard > 0 || !eligible;
+    int n = min(guarded ? (eligible ? min(guard, kGuardedRun) : kGuardedRun) : careful, steps - j);
+    if (sound) n = min(n, pause);
+    bool right = false;
+    if (!guarded) {
+      right = wide ? min(order(s.x.x), order(s.x.y)) >= order(0x1p-74f)
+                   : min_abs(low, s.x.x, s.x.y) >= 0x1p-48f;
+      right = __all_sync(kAll, right || exempt);
+    }
+    if (right) {
       if (wide) {
-        right = min(order(s.x.x), order(s.x.y)) >= order(0x1p-74f);
         uint32_t lowR = ~0u, lowC = ~0u;
+        if (FR == kSplit && FC == kSplit) {
 #pragma unroll 1
-        for (int i = 0; i < n; i++) x.step_wide(s, lowR, lowC);
+          for (int i = 0; i < n; i++) x.step_wide<kSplit>(s, false, false, lowR, lowC);
+        } else if (FR != kCorrected && FC != kCorrected) {
+#pragma unroll 1
+          for (int i = 0; i < n; i++)
+            x.step_wide<kEither>(s, FR == kCut, FC == kCut, lowR, lowC);
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < n; i++) x.step_wide<kCorrected>(s, false, false, lowR, lowC);
+          right = !holds_nan();
+        }
         right &= lowR >= order(0x1p-66f) && lowC >= order(__fmul_rn(0x1p-77f, fabsf(c)));
       } else {
         x.steps_free<kCorrected, kCorrected, true>(s, n, low);
@@ -1488,21 +1642,24 @@ __global__ void __launch_bounds__(32)
         x.settle_zeros(s);
       }
       right = __all_sync(kAll, right || exempt);
-      if (!right) {
-        s = start;
-        skip = again + 1;  // this block and the next ones guarded
-        again = min(2 * again, 8);
-      } else {
-        again = 1;
-      }
+      if (!right) s = start;
     }
-    if (skip || !eligible) {
+    if (guarded) {
+      guard -= n;
+    } else if (right) {
+      again = 2 * kCarefulRun;
+      careful = min(2 * careful, kMostRun);
+    } else {
+      guard = again;
+      again = min(2 * again, kMostPause);
+      careful = kCarefulRun;
+    }
+    if (!right) {
 #pragma unroll 1
       for (int i = 0; i < n; i++) x.step(s);
-      if (skip) skip--;
     }
     j += n;
-    if (careful) careful--;
+    pause -= n;
   }
   if (mine) {
     a.cur[2 * g * S + w] = -s.x.x;
