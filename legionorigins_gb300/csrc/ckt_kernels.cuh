@@ -1397,11 +1397,24 @@ struct LaneState {
   float nb;  // -v_2g+1
 };
 
-// RN(a / b) for every dividend and divisor: the corrected quotient where it
-// is right, the divide routine elsewhere.
-__device__ __forceinline__ float any_quot(float a, const Recip &k, bool eligible, float lo,
-                                          float hi) {
-  return eligible && !outside(a, lo, hi) ? recip_quot(a, k) : div_rn(a, -k.nb);
+// RN(a / b) of N dividends and any divisor: corrected quotients where all are
+// in their range, wide_quot where no quotient is subnormal (zero dividends, as
+// at rest, above all), the divide routine elsewhere.
+template <int N>
+__device__ __forceinline__ void any_quot(const float (&a)[N], float (&q)[N], const Recip &k,
+                                         bool eligible, float lo, float hi) {
+  bool off = !eligible, rare = !eligible;
+#pragma unroll
+  for (int i = 0; i < N; i++) off |= outside(a[i], lo, hi);
+  if (!off) {
+#pragma unroll
+    for (int i = 0; i < N; i++) q[i] = recip_quot(a[i], k);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < N; i++) rare |= subnormal_quot(a[i], k);
+#pragma unroll
+  for (int i = 0; i < N; i++) q[i] = rare ? div_rn(a[i], -k.nb) : wide_quot(a[i], k, lo, hi);
 }
 
 struct LaneWire {
@@ -1475,15 +1488,20 @@ struct LaneWire {
     const float va = s.e.x, vb = -s.nb, vc = s.e.y;
     const float q0 = dt_div(__fmul_rn(L, __fsub_rn(-s.x.x, nX0.x)));
     const float q1 = dt_div(__fmul_rn(L, __fsub_rn(s.x.y, -nX0.y)));
-    const float i0 = any_quot(__fsub_rn(__fsub_rn(vb, va), q0), r, okR, kRLo, kRHi);
-    const float i1 = any_quot(__fsub_rn(__fsub_rn(vc, vb), q1), r, okR, kRLo, kRHi);
-    const float l = __shfl_sync(0xffffffffu, i1, left), n = __shfl_sync(0xffffffffu, i0, right);
-    const float da = __fmul_rn(dt, __fsub_rn(l, i0)), dc = __fmul_rn(dt, __fsub_rn(i1, n));
-    const float db = __fmul_rn(dt, __fsub_rn(i0, i1));
-    s.x = make_float2(-i0, i1);
-    s.nb = -__fadd_rn(-nVb, any_quot(db, C, okC, kCLo, kCHi));
-    if (!first) s.e.x = __fadd_rn(Ve.x, any_quot(da, C, okC, kCLo, kCHi));
-    if (!last) s.e.y = __fadd_rn(Ve.y, any_quot(dc, C, okC, kCLo, kCHi));
+    const float ar[2] = {__fsub_rn(__fsub_rn(vb, va), q0), __fsub_rn(__fsub_rn(vc, vb), q1)};
+    float i[2], q[3];
+    any_quot(ar, i, r, okR, kRLo, kRHi);
+    const float l = __shfl_sync(0xffffffffu, i[1], left);
+    const float n = __shfl_sync(0xffffffffu, i[0], right);
+    // a voltage at the wire's end stays: the middle one's dividend again
+    const float db = __fmul_rn(dt, __fsub_rn(i[0], i[1]));
+    const float ac[3] = {first ? db : __fmul_rn(dt, __fsub_rn(l, i[0])), db,
+                         last ? db : __fmul_rn(dt, __fsub_rn(i[1], n))};
+    any_quot(ac, q, C, okC, kCLo, kCHi);
+    s.x = make_float2(-i[0], i[1]);
+    s.nb = -__fadd_rn(-nVb, q[1]);
+    if (!first) s.e.x = __fadd_rn(Ve.x, q[0]);
+    if (!last) s.e.y = __fadd_rn(Ve.y, q[2]);
   }
   template <QuotForm FR, QuotForm FC, bool LOW>
   __device__ __forceinline__ void steps_free(LaneState &s, int n, float &low) const {
