@@ -406,21 +406,31 @@ static int make_tile_plan(uint32_t N, int64_t W, const std::vector<uint32_t> &of
 // Nodes per tile.  A tile needs every chunk of wires that its nodes' pieces
 // own, so in a graph large enough to use the tiled pass by itself (about 95
 // tiles, see tile_plan_usable) tiles divide equal pieces, or hold whole ones,
-// instead of straddling them.  Fused pass on a GB300, tiles of 8192 nodes /
-// these: 61 pieces of 16,001 nodes (95% in-piece) 56 / 46 us, 64 of 12,000
-// 52 / 39, 128 of 12,000 77 / 59, 300 of 3,000 47 / 39 us.  Multiples of 4
-// keep a tile's node data 16-byte aligned.
-static uint32_t choose_tile_nodes(const ckt_piece *pieces, int32_t num_pieces, uint32_t N) {
+// rather than straddle them at random.  (All have one size, a multiple of 4 for
+// the 16-byte alignment of their node data, so their edges drift from the
+// pieces' by up to 4 nodes a tile: over 61 pieces of 16,001 nodes, 427 of a
+// tile's 8,004.)  Fused pass on a GB300, tiles of 8192 nodes / these: 61 pieces
+// of 16,001 nodes (95% in-piece) 59 / 44 us, 64 of 12,000 50 / 36, 128 of 12,000
+// 84 / 61, 300 of 3,000 45 / 36 us.
+// But a block per tile and SM runs at a time (`sms` of them), and tiles that
+// take another wave of blocks cost more than straddling ones: 95 pieces of
+// 11,000 52 / 55 us (128 and 190 tiles), 320 of 3,000 44 / 55, 80 of 13,000 56 /
+// 57, 90 of 12,000 55 / 58: those keep 8192.
+static uint32_t choose_tile_nodes(const ckt_piece *pieces, int32_t num_pieces, uint32_t N,
+                                  uint32_t sms) {
   if (num_pieces < 1 || N / kTileNodesMax < 90) return kTileNodesMax;
   const uint32_t npp = pieces[0].num_nodes;
   for (int32_t k = 0; k < num_pieces; k++)
     if (pieces[k].num_nodes != npp) return kTileNodesMax;
-  if (npp == 0) return kTileNodesMax;
+  if (npp == 0 || sms == 0) return kTileNodesMax;
   const uint32_t parts = (npp + kTileNodesMax - 1) / kTileNodesMax;
-  const uint32_t nodes = npp <= kTileNodesMax / 2 ? kTileNodesMax / npp * npp
-                                                  : (npp + parts - 1) / parts;
+  uint32_t nodes = npp <= kTileNodesMax / 2 ? kTileNodesMax / npp * npp
+                                            : (npp + parts - 1) / parts;
   // much smaller tiles would cost more in their number than straddling does
-  return nodes < kTileNodesMax * 2 / 3 ? kTileNodesMax : (nodes + 3u) & ~3u;
+  if (nodes < kTileNodesMax * 2 / 3) return kTileNodesMax;
+  nodes = (nodes + 3u) & ~3u;
+  auto waves = [&](uint32_t tile) { return ((N + tile - 1) / tile + sms - 1) / sms; };
+  return waves(nodes) > waves(kTileNodesMax) ? kTileNodesMax : nodes;
 }
 
 // Builds and uploads the tiled distribute_charge plan.
@@ -481,6 +491,9 @@ int ckt_graph_create(const ckt_piece *pieces, int32_t num_pieces, uint32_t num_n
   for (int64_t i = 0; i < 2 * W; i++)
     if (ent[i] & 1u) gstart[i >> 5] |= 1u << (i & 31);
 
+  int dev = 0, sms = 0;
+  CKT_CUDA(cudaGetDevice(&dev));
+  CKT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   ckt_graph *g = new ckt_graph();
   g->W = W;
   g->N = num_nodes;
@@ -527,7 +540,8 @@ int ckt_graph_create(const ckt_piece *pieces, int32_t num_pieces, uint32_t num_n
       (rc = upload(&g->slot_in, slot_in, &g->device_bytes)) ||
       (rc = upload(&g->slot_out, slot_out, &g->device_bytes)) ||
       (rc = upload(&g->gstart, gstart, &g->device_bytes)) ||
-      (rc = build_tile_plan(g, off, ent, choose_tile_nodes(pieces, num_pieces, num_nodes)))) {
+      (rc = build_tile_plan(g, off, ent,
+                            choose_tile_nodes(pieces, num_pieces, num_nodes, (uint32_t)sms)))) {
     free_graph(g);
     return rc;
   }
