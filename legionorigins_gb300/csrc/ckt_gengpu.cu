@@ -485,41 +485,50 @@ __global__ void __launch_bounds__(256)
 // memory.  A lane takes an entry, not a node: its place is the number of
 // smaller entries in its run; lanes of one run read the same words, so banks
 // hardly conflict (a node per lane, insertion-sorting its run, reads words 8
-// apart).  A span larger than the stage is sorted in place in tmp instead, a
-// node per lane.
+// apart).  A span larger than the stage is counted from tmp in the same way,
+// the entry before found beside the place.  (Insertion-sorted in place, a node
+// per lane, its entries nearly in the order of their wires or not: 1024 nodes
+// of 128 entries 2.0 / 2.7 ms for the whole generator, 256 of 512 37 / 38 ms,
+// 65,536 of 32 409 / 550 us; counted 0.5 and 6.6 ms, 184 us.)
 constexpr uint32_t kFinishSpan = 384;  // entries per warp staged (256 on average)
 
 __global__ void __launch_bounds__(256)
-    csr_finish_kernel(GenArgs g, const uint32_t *__restrict__ off, uint32_t *tmp, uint32_t *ent,
-                      uint32_t *slot_in, uint32_t *slot_out, uint32_t *gstart) {
+    csr_finish_kernel(GenArgs g, const uint32_t *__restrict__ off,
+                      const uint32_t *__restrict__ tmp, uint32_t *ent, uint32_t *slot_in,
+                      uint32_t *slot_out, uint32_t *gstart) {
   __shared__ uint32_t sbuf[8][kFinishSpan], sout[8][kFinishSpan], soff[8][33];
   __shared__ uint32_t sfirst[8][kFinishSpan / 32];  // bit j: entry j opens a run
   const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
   const int64_t x0 = ((int64_t)blockIdx.x * 8 + wp) * 32;
   if (x0 >= g.N) return;
-  const int64_t xe = min(g.N, x0 + 32), x = x0 + lane;
-  const uint32_t b = off[min(x, xe)] & kOffsetMask;
+  const int64_t xe = min(g.N, x0 + 32);
+  const uint32_t b = off[min(x0 + lane, xe)] & kOffsetMask;
   const uint32_t lo = __shfl_sync(0xffffffffu, b, 0), hi = off[xe] & kOffsetMask;
   const uint32_t span = hi - lo;
   // the first wire of a wire's piece
   auto piece_first = [&g](uint32_t w) {
     return g.wpp == 1 ? w : (uint32_t)__umul64hi(g.wpp_magic, (uint64_t)w) * (uint32_t)g.wpp;
   };
+  uint32_t *run = soff[wp];
+  run[lane] = b - lo;
+  if (lane == 0) run[32] = span;
+  __syncwarp();
+  auto node_of = [run](uint32_t j) {  // the last node whose run starts at or before j
+    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t step = 16; step; step >>= 1)
+      if (run[n + step] <= j) n += step;
+    return n;
+  };
   if (span <= kFinishSpan) {
-    uint32_t *buf = sbuf[wp], *out = sout[wp], *run = soff[wp], *opens = sfirst[wp];
-    run[lane] = b - lo;
-    if (lane == 0) run[32] = span;
+    uint32_t *buf = sbuf[wp], *out = sout[wp], *opens = sfirst[wp];
     if (lane < kFinishSpan / 32) opens[lane] = 0;
 #pragma unroll 4
     for (uint32_t j = lane; j < span; j += 32) buf[j] = tmp[lo + j];
     __syncwarp();
     if (run[lane] < run[lane + 1]) atomicOr(opens + (run[lane] >> 5), 1u << (run[lane] & 31u));
     for (uint32_t j = lane; j < span; j += 32) {
-      uint32_t n = 0;  // the last node whose run starts at or before j
-#pragma unroll
-      for (uint32_t step = 16; step; step >>= 1)
-        if (run[n + step] <= j) n += step;
-      const uint32_t end = run[n + 1], v = buf[j];
+      const uint32_t n = node_of(j), end = run[n + 1], v = buf[j];
       uint32_t place = run[n];
 #pragma unroll 4
       for (uint32_t i = place; i < end; i++) place += buf[i] < v ? 1u : 0u;
@@ -546,22 +555,19 @@ __global__ void __launch_bounds__(256)
     }
     return;
   }
-  if (x >= xe) return;
-  const uint32_t e = off[x + 1] & kOffsetMask;
-  for (uint32_t i = b + 1; i < e; i++) {
-    const uint32_t v = tmp[i];
-    uint32_t j = i;
-    while (j > b && tmp[j - 1] > v) {
-      tmp[j] = tmp[j - 1];
-      j--;
+  for (uint32_t j = lane; j < span; j += 32) {
+    const uint32_t n = node_of(j), end = run[n + 1], v = tmp[lo + j], w = v >> 1;
+    uint32_t place = run[n], before = 0;  // 1 + the next smaller entry, or 0
+#pragma unroll 8
+    for (uint32_t i = place; i < end; i++) {
+      const uint32_t u = tmp[lo + i];
+      place += u < v ? 1u : 0u;
+      before = max(before, u < v ? u + 1u : 0u);
     }
-    tmp[j] = v;
-  }
-  for (uint32_t i = b; i < e; i++) {
-    const uint32_t v = tmp[i], w = v >> 1;
-    const bool start = i == b || tmp[i - 1] >> 1 < piece_first(w);
+    const uint32_t i = lo + place;
+    const bool start = before == 0u || (before - 1u) >> 1 < piece_first(w);
     ent[i] = (w << 2) | ((v & 1u) << 1) | (start ? 1u : 0u);
-    if (start) atomicOr(gstart + (i >> 5), 1u << (i & 31));
+    if (start) atomicOr(gstart + (i >> 5), 1u << (i & 31u));
     if (v & 1u) slot_out[w] = i;
     else slot_in[w] = i;
   }
