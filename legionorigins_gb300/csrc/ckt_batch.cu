@@ -276,7 +276,7 @@ int launch(ckt_batch *b, int mode, cudaStream_t s) {
     int rc = build_tables(b);
     if (rc) return rc;
   }
-  return launch_round(mode, b->cfg, b->grid, b->d_items, b->num_items, b->d_circ, (uint32_t)b->C,
+  return launch_round(mode, b->cfg, b->grid, b->d_items, b->num_items, b->d_circ, b->h_circ,
                       b->sync_mem, b->timeout_ns, s);
 }
 

@@ -191,16 +191,19 @@ __device__ __noinline__ float2 few_steps(int64_t w, const WireArrays a, const No
 // EXACT tiles of one wire too: with a third block its 80 registers spill the
 // free steps' loop (16 circuits, block 256, schedule 2: 9.29 -> 9.01 ms with
 // two blocks).
-template <uint32_t BLOCK, int WPT, int DCS, int MODE>
-__global__ void __launch_bounds__(BLOCK,
-                                  (WPT == 2 || MODE == CKT_MODE_EXACT ? 512 : 768) / BLOCK)
+// FREE: EXACT with unguarded steps, for circuits of kFreeSteps steps or more.
+// Rounds whose circuits all have fewer take EXACT without them: their CNC tiles
+// are inline and the blocks lighter (18 circuits, 101,109 wires, 1 / 8 / 31
+// steps: 53 / 63 / 130 us with, 40 / 50 / 111 us without).
+template <uint32_t BLOCK, int WPT, int DCS, int MODE, bool FREE = MODE == CKT_MODE_EXACT>
+__global__ void __launch_bounds__(BLOCK, (WPT == 2 || FREE ? 512 : 768) / BLOCK)
     round_kernel(const BatchItem *__restrict__ items, uint32_t num_items,
                  const RoundCircuit *__restrict__ circ, BatchSync sync, float dt,
                  uint64_t timeout_ns) {
   __shared__ uint32_t s_item, s_go;
   // The CNC tiles' saved states and the DC tiles' staged contributions are
   // never in use at the same time.
-  constexpr int kSave = MODE == CKT_MODE_EXACT ? kSavedState * WPT * (int)BLOCK : WPT;
+  constexpr int kSave = FREE ? kSavedState * WPT * (int)BLOCK : WPT;
   constexpr int kStage = DCS == 1 ? 1 : (int)kDcChunk;
   __shared__ __align__(8) float sbuf[kSave > kStage ? kSave : kStage];
   float *sval = sbuf;
@@ -238,15 +241,15 @@ __global__ void __launch_bounds__(BLOCK,
           const bool has_b = tb < item.count;
           const uint32_t w = item.begin + ta, wb = item.begin + (has_b ? tb : ta);
           float2 i0, i9;
-          if (MODE == CKT_MODE_EXACT && rc.steps < kFreeSteps) {
+          if (FREE && rc.steps < kFreeSteps) {
             const float4 r = few_steps_pair<MODE>((int64_t)w, (int64_t)wb, has_b, wa, volts,
                                                   rc.steps, dt);
             i0 = make_float2(r.x, r.y);
             i9 = make_float2(r.z, r.w);
           } else {
-            cnc_wire_pair<MODE, CKT_INIT_KERNEL, MODE == CKT_MODE_EXACT ? (int)BLOCK : 0>(
+            cnc_wire_pair<MODE, CKT_INIT_KERNEL, FREE ? (int)BLOCK : 0>(
                 (int64_t)w, (int64_t)wb, has_b, wa, volts, rc.steps, dt,
-                reinterpret_cast<float2 *>(sbuf) + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0),
+                reinterpret_cast<float2 *>(sbuf) + (FREE ? threadIdx.x : 0),
                 &i0, &i9);
           }
           if (DCS == 2) {
@@ -265,14 +268,14 @@ __global__ void __launch_bounds__(BLOCK,
           if (t < item.count) {
             const uint32_t w = item.begin + t;
             float i0, i9;
-            if (MODE == CKT_MODE_EXACT && rc.steps < kFreeSteps) {
+            if (FREE && rc.steps < kFreeSteps) {
               const float2 r = few_steps<MODE>((int64_t)w, wa, volts, rc.steps, dt);
               i0 = r.x;
               i9 = r.y;
             } else {
-              cnc_wire<MODE, CKT_INIT_KERNEL, MODE == CKT_MODE_EXACT ? (int)BLOCK : 0>(
+              cnc_wire<MODE, CKT_INIT_KERNEL, FREE ? (int)BLOCK : 0>(
                   (int64_t)w, wa, volts, rc.steps, dt,
-                  sbuf + (MODE == CKT_MODE_EXACT ? threadIdx.x : 0), &i0, &i9);
+                  sbuf + (FREE ? threadIdx.x : 0), &i0, &i9);
             }
             if (DCS == 2) {
               rc.contrib[rc.slot_in[w]] = __fmul_rn(-dt, i0);

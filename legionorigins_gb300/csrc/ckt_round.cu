@@ -72,33 +72,41 @@ void build_round_table(std::vector<RoundCircuit> &circuits, const ckt_batch_conf
   }
 }
 
-BatchKernelFn round_kernel_for(int mode, const ckt_batch_config &c) {
-  return mode == CKT_MODE_EXACT ? batch_kernel_exact(c.block, c.wires_per_thread, c.dc_schedule)
-                                : batch_kernel_fast(c.block, c.wires_per_thread, c.dc_schedule);
+BatchKernelFn round_kernel_for(int mode, const ckt_batch_config &c, bool few) {
+  return mode != CKT_MODE_EXACT ? batch_kernel_fast(c.block, c.wires_per_thread, c.dc_schedule)
+         : few ? batch_kernel_exact_few(c.block, c.wires_per_thread, c.dc_schedule)
+               : batch_kernel_exact(c.block, c.wires_per_thread, c.dc_schedule);
 }
 
 int round_blocks_per_sm(const ckt_batch_config &c, int *out) {
-  int a = 0, b = 0;
-  CKT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &a, reinterpret_cast<const void *>(round_kernel_for(CKT_MODE_FAST, c)), c.block, 0));
-  CKT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &b, reinterpret_cast<const void *>(round_kernel_for(CKT_MODE_EXACT, c)), c.block, 0));
-  // The modes' kernels of one configuration may differ (EXACT's one-wire tiles
-  // use more registers).  The grid is the larger: a block that is not resident
+  // The kernels of one configuration may differ (EXACT's one-wire tiles use
+  // more registers).  The grid is the largest: a block that is not resident
   // yet holds no ticket, so nothing waits for it, and it finds none left when
   // it starts.
-  *out = std::max(1, std::max(a, b));
+  *out = 1;
+  for (const BatchKernelFn fn : {round_kernel_for(CKT_MODE_FAST, c, false),
+                                 round_kernel_for(CKT_MODE_EXACT, c, false),
+                                 round_kernel_for(CKT_MODE_EXACT, c, true)}) {
+    int n = 0;
+    CKT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &n, reinterpret_cast<const void *>(fn), c.block, 0));
+    *out = std::max(*out, n);
+  }
   return CKT_OK;
 }
 
 int launch_round(int mode, const ckt_batch_config &cfg, int grid, const BatchItem *items,
-                 uint32_t num_items, const RoundCircuit *circ, uint32_t C, uint32_t *sync_mem,
+                 uint32_t num_items, const RoundCircuit *circ,
+                 const std::vector<RoundCircuit> &circuits, uint32_t *sync_mem,
                  uint64_t timeout_ns, cudaStream_t s) {
-  CKT_CUDA(cudaMemsetAsync(sync_mem, 0, (2 + 2 * (size_t)C) * sizeof(uint32_t), s));
+  const size_t C = circuits.size();
+  CKT_CUDA(cudaMemsetAsync(sync_mem, 0, (2 + 2 * C) * sizeof(uint32_t), s));
   BatchSync sync = {sync_mem, sync_mem + 1, sync_mem + 2, sync_mem + 2 + C};
   float dt = (float)1e-6;
   void *args[] = {&items, &num_items, &circ, &sync, &dt, &timeout_ns};
-  BatchKernelFn fn = round_kernel_for(mode, cfg);
+  const bool few = std::all_of(circuits.begin(), circuits.end(),
+                               [](const RoundCircuit &c) { return c.steps < kFreeSteps; });
+  BatchKernelFn fn = round_kernel_for(mode, cfg, few);
   CKT_REQUIRE(fn != nullptr, "no round kernel for this configuration");
   CKT_CUDA(cudaLaunchKernel(reinterpret_cast<const void *>(fn), dim3(grid), dim3(cfg.block), args,
                             0, s));

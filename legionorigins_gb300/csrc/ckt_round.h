@@ -30,16 +30,19 @@ inline size_t gstart_words(int64_t W) { return (size_t)((2 * W + 31) / 32); }
 void build_round_table(std::vector<RoundCircuit> &circuits, const ckt_batch_config &cfg,
                        std::vector<BatchItem> &items);
 
-// The kernel for (mode, launch shape), or null.
-BatchKernelFn round_kernel_for(int mode, const ckt_batch_config &cfg);
+// The kernel for (mode, launch shape), or null.  few: all circuits have fewer
+// than kFreeSteps steps.
+BatchKernelFn round_kernel_for(int mode, const ckt_batch_config &cfg, bool few);
 
-// Most resident blocks per SM of the round kernel for this shape, over the modes.
+// Most resident blocks per SM of the round kernels for this shape.
 int round_blocks_per_sm(const ckt_batch_config &cfg, int *out);
 
-// One round: clears the sync words (ticket, error, done counters of C
-// circuits) and launches the persistent kernel on `s`.
+// One round: clears the sync words (ticket, error, done counters of the
+// circuits) and launches the persistent kernel on `s`.  circ: the circuits'
+// descriptors on the device, circuits: on the host.
 int launch_round(int mode, const ckt_batch_config &cfg, int grid, const BatchItem *items,
-                 uint32_t num_items, const RoundCircuit *circ, uint32_t C, uint32_t *sync_mem,
+                 uint32_t num_items, const RoundCircuit *circ,
+                 const std::vector<RoundCircuit> &circuits, uint32_t *sync_mem,
                  uint64_t timeout_ns, cudaStream_t s);
 
 int check_batch_config(const ckt_batch_config *c);

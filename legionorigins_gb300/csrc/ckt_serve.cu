@@ -454,8 +454,7 @@ int launch_staged_round(ckt_server *s, int slot, const std::vector<RoundCircuit>
   CKT_CUDA(cudaMemcpyAsync(s->d_circ, st.circ, circ.size() * sizeof(RoundCircuit),
                            cudaMemcpyHostToDevice, s->compute));
   if ((rc = launch_round(s->cfg.mode, s->cfg.launch, s->grid, s->d_items, (uint32_t)items.size(),
-                         s->d_circ, (uint32_t)circ.size(), s->d_sync, s->cfg.round_timeout_ns,
-                         s->compute)))
+                         s->d_circ, circ, s->d_sync, s->cfg.round_timeout_ns, s->compute)))
     return rc;
   CKT_CUDA(cudaMemcpyAsync(st.err, s->d_sync + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                            s->compute));
