@@ -90,6 +90,8 @@ static void launch_cnc_t(uint32_t first, uint32_t n, const ckt_wires &w, const f
   //     one thread/wire         47     48    105    135     276     760
   //     paired, 128             72     72    126    127     287     715     5525
   //     paired, 256            123    123    125    125     339     763     5510
+  //   (FAST, 1,000,000 wires, 16 / 32 / 200 steps: blocks of 128 threads 41 / 61 /
+  //   284, of 256 48 / 68 / 285)
   const uint32_t sms = (uint32_t)device_sms();
   uint32_t dt_bits;
   memcpy(&dt_bits, &p->dt, sizeof(dt_bits));
@@ -112,14 +114,10 @@ static void launch_cnc_t(uint32_t first, uint32_t n, const ckt_wires &w, const f
     cnc_kernel<M, I, false><<<grid_for(n, 32), 32, 0, s>>>(first, n, a, v, p->steps, p->dt);
     return;
   }
-  if constexpr (M == CKT_MODE_FAST) {
-    if (n > 512u * sms && n <= 4096u * sms) {  // (up to one 256-thread block per SM is even)
-      cnc_pair_kernel<M, I, false, 128><<<grid_for(n, 256), 128, 0, s>>>(first, n, a, v, p->steps,
-                                                                        p->dt);
-      return;
-    }
-  }
-  if constexpr (M == CKT_MODE_FAST || M == CKT_MODE_EXACT)  // two wires per thread, paired
+  if constexpr (M == CKT_MODE_FAST)  // two wires per thread, paired
+    cnc_pair_kernel<M, I, false, 128><<<grid_for(n, 256), 128, 0, s>>>(first, n, a, v, p->steps,
+                                                                      p->dt);
+  else if constexpr (M == CKT_MODE_EXACT)
     cnc_pair_kernel<M, I, false, 256><<<grid_for(n, 512), 256, 0, s>>>(first, n, a, v, p->steps,
                                                                       p->dt);
   else
