@@ -1,7 +1,7 @@
 """The choice of the node tiles' size, on the CPU: tiles that divide equal
 pieces or hold whole ones, unless that takes another wave of blocks (one per
 SM); and the plans of such sizes -- small tiles, tiles that drift across the
-pieces' edges -- replayed as the kernel walks them (test_tile_plan's checker
+pieces' edges -- replayed as the kernel walks them (test_tile_plan's program
 with the tile size given)."""
 import os
 import shutil
